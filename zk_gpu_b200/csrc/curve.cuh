@@ -9,11 +9,9 @@
 // not recognised as zero afterwards).  Affine inputs use (0, 0) for the
 // identity (cuda/bn256.h:15-20).
 //
-// Arithmetic form: every coordinate is kept in the R' = 2^260 Montgomery
-// form of the FP64 52-bit-limb product (mul_rp: R'-form x R'-form -> R'-form),
-// lazily reduced in [0, 2q); values are made canonical only where they are
-// compared with zero.  to_rprime / from_rprime convert from / to the
-// R = 2^256 form used in memory by the API (bit-identical to halo2curves).
+// Arithmetic form: coordinates are in the R = 2^256 Montgomery form the API
+// holds in memory (bit-identical to halo2curves), lazily reduced in [0, 2q);
+// values are made canonical only where they are compared with zero.
 #pragma once
 #include "field.cuh"
 
@@ -28,32 +26,28 @@ struct aff_t {
   uint32_t x[8], y[8];
 };
 
-// ---- lazy R'-form Fq helpers --------------------------------------------
+// ---- lazy Fq helpers ------------------------------------------------------
 // ZK_MSM_CALL_PRODUCT: 0 = every product inlined; 1 = only the products of
 // the batch-affine apply pass (qmul_c / qsqr_c) are calls of one out-of-line
-// product (mul_rp_out); 2 (the default) = every qmul / qsqr is such a call.
-// Measured on B200 with bit-identical outputs, MSM of 2^22 / 2^20 / 2^18 /
-// 2^16 points: inlined 14.85 / 5.77 / 3.14 / 2.01 ms, apply pass only
-// 14.8 / 5.8 / 3.1 / 2.0 ms, every product 14.42 / 5.32 / 2.75 / 1.82 ms:
-// the XYZZ reduction and tail kernels, which inline a dozen or more products
-// per thread, lose their spills (112 B -> 0 in the window kernel at 255
-// registers) and their instruction-cache misses.
+// product (mul_out); 2 (the default) = every qmul / qsqr is such a call.
+// The XYZZ reduction and tail kernels would inline a dozen or more products
+// per thread; the call spares them instruction-cache misses.
 #ifndef ZK_MSM_CALL_PRODUCT
 #define ZK_MSM_CALL_PRODUCT 2
 #endif
 __device__ __forceinline__ void qmul(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) {
 #if ZK_MSM_CALL_PRODUCT >= 2
-  mul_rp_out<P_q>(r, a, b);
+  mul_out<P_q>(r, a, b);
 #else
-  mul_rp<P_q>(r, a, b);
+  mul_lazy<P_q>(r, a, b);
 #endif
 }
 __device__ __forceinline__ void qsqr(uint32_t r[8], const uint32_t a[8]) { qmul(r, a, a); }
 __device__ __forceinline__ void qmul_c(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) {
 #if ZK_MSM_CALL_PRODUCT >= 1
-  mul_rp_out<P_q>(r, a, b);
+  mul_out<P_q>(r, a, b);
 #else
-  mul_rp<P_q>(r, a, b);
+  mul_lazy<P_q>(r, a, b);
 #endif
 }
 __device__ __forceinline__ void qsqr_c(uint32_t r[8], const uint32_t a[8]) { qmul_c(r, a, a); }
@@ -65,21 +59,6 @@ __device__ __forceinline__ bool qzero(const uint32_t a[8]) {
   reduce_once<P_q>(c, a);
   return is_zero(c);
 }
-// x (R form, x * 2^256) -> x * 2^260, canonical: multiply by 2^264 mod q
-__device__ __forceinline__ void to_rprime(uint32_t r[8], const uint32_t a[8]) {
-  const uint32_t k[8] = {0xfaec667au, 0xfbdb0f2au, 0x9626b0ffu, 0xad825aedu,
-                         0x09e2a0fcu, 0x276f48b7u, 0xef86e357u, 0x0d791464u};
-  mul_rp<P_q>(r, a, k);
-  reduce_once<P_q>(r, r);
-}
-// x * 2^260 (lazy) -> x * 2^256, canonical: multiply by 2^256 mod q
-__device__ __forceinline__ void from_rprime(uint32_t r[8], const uint32_t a[8]) {
-  uint32_t one_r[8];
-  set_one<P_q>(one_r);  // the integer 2^256 mod q
-  mul_rp<P_q>(r, a, one_r);
-  reduce_once<P_q>(r, r);
-}
-
 __device__ __forceinline__ void xyzz_set_inf(xyzz_t& p) {
   set_zero(p.x);
   set_zero(p.y);
@@ -96,8 +75,8 @@ __device__ __forceinline__ void xyzz_from_aff(xyzz_t& r, const aff_t& q) {
   }
   cpy(r.x, q.x);
   cpy(r.y, q.y);
-  set_one_rp<P_q>(r.zz);
-  set_one_rp<P_q>(r.zzz);
+  set_one<P_q>(r.zz);
+  set_one<P_q>(r.zzz);
 }
 
 // r = 2p  (dbl-2008-s-1, a = 0).  The identity doubles to itself (ZZ stays 0).
@@ -225,41 +204,6 @@ __device__ __forceinline__ void xyzz_add(xyzz_t& p, const xyzz_t& q) {
   qmul(p.zz, p.zz, PP);
   qmul(p.zzz, p.zzz, q.zzz);
   qmul(p.zzz, p.zzz, PPP);
-}
-
-// p = k * p for a small non-negative k (double-and-add, k < 2^32)
-__device__ __forceinline__ void xyzz_mul_small(xyzz_t& p, uint32_t k) {
-  xyzz_t acc;
-  xyzz_set_inf(acc);
-  if (k == 0 || xyzz_is_inf(p)) {
-    p = acc;
-    return;
-  }
-  const int top = 31 - __clz(k);
-  acc = p;
-  for (int b = top - 1; b >= 0; b--) {
-    xyzz_dbl(acc, acc);
-    if ((k >> b) & 1) xyzz_add(acc, p);
-  }
-  p = acc;
-}
-
-// XYZZ (R' form) -> Jacobian (R form, canonical) without inversion:
-// (X ZZ^2, Y ZZ^3, ZZZ) represents the same point.
-__device__ __forceinline__ void xyzz_to_jacobian(uint32_t out[24], const xyzz_t& p) {
-  if (xyzz_is_inf(p)) {
-#pragma unroll
-    for (int i = 0; i < 24; i++) out[i] = 0;
-    return;
-  }
-  uint32_t zz2[8], zz3[8], t[8];
-  qsqr(zz2, p.zz);
-  qmul(zz3, zz2, p.zz);
-  qmul(t, p.x, zz2);
-  from_rprime(out, t);
-  qmul(t, p.y, zz3);
-  from_rprime(out + 8, t);
-  from_rprime(out + 16, p.zzz);
 }
 
 __device__ __forceinline__ void ld_aff(aff_t& q, const fe* p) {

@@ -11,8 +11,8 @@
 //
 // All of these are streaming passes: 64 or 32 B read and 32 B written per
 // element, one or zero field products.  One product per element costs about
-// 1/60 ns per element on the FP64-limb product against 96 B / 6.5 TB/s =
-// 1/68 ns of HBM time, so the kernels are balanced close to the HBM roofline.
+// 1/67 ns per element (mul_lazy) against 96 B / 6.5 TB/s = 1/68 ns of HBM
+// time, so the kernels are balanced close to the HBM roofline.
 // Grids are a multiple of the SM count; each thread walks the vector with a
 // grid stride, two elements per step so that four 16-B loads are in flight.
 #include <cstring>
@@ -27,22 +27,13 @@ namespace {
 
 using P_r = FrP;
 
-// a * b * 2^-256 for canonical R-form a, b: the FP64 product gives
-// a b 2^-260 (< 2p), four lazy doublings restore the factor 2^4.
-__device__ __forceinline__ void mont_mul_data(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) {
-  mul_rp<P_r>(r, a, b);
-#pragma unroll
-  for (int k = 0; k < 4; k++) add_lazy<P_r>(r, r, r);
-  reduce_once<P_r>(r, r);
-}
-
 template <int OP>
-__device__ __forceinline__ void ew_one(fe* out, const fe* a, const fe* b, const fe& c_rp, uint64_t i) {
+__device__ __forceinline__ void ew_one(fe* out, const fe* a, const fe* b, const fe& c, uint64_t i) {
   uint32_t x[8], y[8], r[8];
   ld_fe(x, a + i);
   if (OP == ZKGPU_EW_MUL) {
     ld_fe(y, b + i);
-    mont_mul_data(r, x, y);
+    mul<P_r>(r, x, y);
   } else if (OP == ZKGPU_EW_ADD) {
     ld_fe(y, b + i);
     add<P_r>(r, x, y);
@@ -50,31 +41,29 @@ __device__ __forceinline__ void ew_one(fe* out, const fe* a, const fe* b, const 
     ld_fe(y, b + i);
     sub<P_r>(r, x, y);
   } else if (OP == ZKGPU_EW_SCALE) {
-    mul_rp<P_r>(r, x, c_rp.w);
-    reduce_once<P_r>(r, r);
+    mul<P_r>(r, x, c.w);
   } else {  // AXPY
     ld_fe(y, b + i);
-    mul_rp<P_r>(r, x, c_rp.w);
-    reduce_once<P_r>(r, r);
+    mul<P_r>(r, x, c.w);
     add<P_r>(r, r, y);
   }
   st_fe(out + i, r);
 }
 
 template <int OP>
-__global__ void __launch_bounds__(256) ew_kernel(fe* out, const fe* a, const fe* b, const fe c_rp, uint64_t n) {
+__global__ void __launch_bounds__(256) ew_kernel(fe* out, const fe* a, const fe* b, const fe c_fe, uint64_t n) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   for (; i + stride < n; i += 2 * stride) {
-    ew_one<OP>(out, a, b, c_rp, i);
-    ew_one<OP>(out, a, b, c_rp, i + stride);
+    ew_one<OP>(out, a, b, c_fe, i);
+    ew_one<OP>(out, a, b, c_fe, i + stride);
   }
-  if (i < n) ew_one<OP>(out, a, b, c_rp, i);
+  if (i < n) ew_one<OP>(out, a, b, c_fe, i);
 }
 
 constexpr int kMaxVanish = 64;  // distinct values of X^n - 1 on the coset (extension factor <= 64)
 struct VanishInv {
-  fe v[kMaxVanish];  // 1 / t_j in R' form
+  fe v[kMaxVanish];  // 1 / t_j
 };
 
 __global__ void __launch_bounds__(256) vanish_kernel(fe* d, const VanishInv tinv, uint32_t mask, uint64_t n) {
@@ -82,16 +71,14 @@ __global__ void __launch_bounds__(256) vanish_kernel(fe* d, const VanishInv tinv
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
     uint32_t x[8];
     ld_fe(x, d + i);
-    mul_rp<P_r>(x, x, tinv.v[i & mask].w);
-    reduce_once<P_r>(x, x);
+    mul<P_r>(x, x, tinv.v[i & mask].w);
     st_fe(d + i, x);
   }
 }
 
-fe to_fe_rp(const host::Fr& a) {
-  const host::Fr r = host::mul(a, host::from_u64(16));
+fe to_fe(const host::Fr& a) {
   fe out;
-  std::memcpy(out.w, r.v, 32);
+  std::memcpy(out.w, a.v, 32);
   return out;
 }
 
@@ -116,12 +103,12 @@ extern "C" int zkgpu_ew_dev(int device, uint32_t op, uint64_t* d_out, const uint
   const bool needs_b = op != ZKGPU_EW_SCALE;
   const bool needs_c = op == ZKGPU_EW_SCALE || op == ZKGPU_EW_AXPY;
   if (!d_out || !d_a || (needs_b && !d_b) || (needs_c && !c)) return ZKGPU_EINVAL;
-  fe c_rp{};
+  fe c_fe{};
   if (needs_c) {
     zk::host::Fr cc;
     std::memcpy(cc.v, c, 32);
     if (!zk::host::is_canonical(cc)) return ZKGPU_EINVAL;
-    c_rp = zk::to_fe_rp(cc);
+    c_fe = zk::to_fe(cc);
   }
   cudaStream_t own;
   int st = zk::bind_device(device, &own);
@@ -136,11 +123,11 @@ extern "C" int zkgpu_ew_dev(int device, uint32_t op, uint64_t* d_out, const uint
   {
     zk::ProfScope ps(names[op], s, products, (double)n * (needs_b ? 96.0 : 64.0));
     switch (op) {
-      case ZKGPU_EW_MUL: zk::ew_kernel<ZKGPU_EW_MUL><<<grid, 256, 0, s>>>(out, a, b, c_rp, n); break;
-      case ZKGPU_EW_ADD: zk::ew_kernel<ZKGPU_EW_ADD><<<grid, 256, 0, s>>>(out, a, b, c_rp, n); break;
-      case ZKGPU_EW_SUB: zk::ew_kernel<ZKGPU_EW_SUB><<<grid, 256, 0, s>>>(out, a, b, c_rp, n); break;
-      case ZKGPU_EW_SCALE: zk::ew_kernel<ZKGPU_EW_SCALE><<<grid, 256, 0, s>>>(out, a, b, c_rp, n); break;
-      default: zk::ew_kernel<ZKGPU_EW_AXPY><<<grid, 256, 0, s>>>(out, a, b, c_rp, n); break;
+      case ZKGPU_EW_MUL: zk::ew_kernel<ZKGPU_EW_MUL><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
+      case ZKGPU_EW_ADD: zk::ew_kernel<ZKGPU_EW_ADD><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
+      case ZKGPU_EW_SUB: zk::ew_kernel<ZKGPU_EW_SUB><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
+      case ZKGPU_EW_SCALE: zk::ew_kernel<ZKGPU_EW_SCALE><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
+      default: zk::ew_kernel<ZKGPU_EW_AXPY><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
     }
   }
   zk::count_launches(1);
@@ -164,7 +151,7 @@ extern "C" int zkgpu_divide_by_vanishing_dev(int device, uint64_t* d_ext, uint32
   for (uint32_t j = 0; j < J; j++) {
     const hf::Fr t = hf::sub(cur, hf::one());
     if (hf::eq(t, hf::zero())) return ZKGPU_EINVAL;  // X^n - 1 vanishes on this coset
-    tinv.v[j] = zk::to_fe_rp(hf::inv(t));
+    tinv.v[j] = zk::to_fe(hf::inv(t));
     cur = hf::mul(cur, step);
   }
   cudaStream_t own;

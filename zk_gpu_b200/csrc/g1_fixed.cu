@@ -8,8 +8,7 @@
 // Method: fixed 4-bit windows.  A table T[w][d] = d * 16^w * B (w < 64,
 // 1 <= d < 16) is built once per call by 64 threads, normalised to affine;
 // each scalar then costs at most 64 mixed additions (XYZZ madd) and one field
-// inversion (Fermat, a^(q-2)) to return to affine.  All arithmetic is the
-// R'-form product (mul_rp) of field.cuh; outputs are canonical R-form
+// inversion (Fermat, a^(q-2)) to return to affine.  Outputs are canonical
 // (Montgomery, 2^256) affine points, (0, 0) for the identity.
 #include <cuda_runtime.h>
 
@@ -19,11 +18,11 @@
 namespace zk {
 namespace {
 
-// a^(q-2) = a^-1 for a != 0, R' form in and out (lazy in, canonical out)
-__device__ void fq_inv_rp(uint32_t r[8], const uint32_t a[8]) {
+// a^(q-2) = a^-1 for a != 0 (lazy in, canonical out)
+__device__ void fq_inv_fermat(uint32_t r[8], const uint32_t a[8]) {
   const uint32_t e[8] = {FqP::P0 - 2u, FqP::P1, FqP::P2, FqP::P3, FqP::P4, FqP::P5, FqP::P6, FqP::P7};
   uint32_t acc[8];
-  set_one_rp<FqP>(acc);
+  set_one<FqP>(acc);
   for (int w = 7; w >= 0; w--) {
     for (int b = 31; b >= 0; b--) {
       qsqr(acc, acc);
@@ -33,8 +32,8 @@ __device__ void fq_inv_rp(uint32_t r[8], const uint32_t a[8]) {
   reduce_once<FqP>(r, acc);
 }
 
-// XYZZ -> affine (R' form, canonical); identity -> (0, 0)
-__device__ void xyzz_to_affine_rp(aff_t& o, const xyzz_t& p) {
+// XYZZ -> affine (canonical); identity -> (0, 0)
+__device__ void xyzz_to_affine(aff_t& o, const xyzz_t& p) {
   if (xyzz_is_inf(p)) {
     set_zero(o.x);
     set_zero(o.y);
@@ -42,7 +41,7 @@ __device__ void xyzz_to_affine_rp(aff_t& o, const xyzz_t& p) {
   }
   uint32_t t[8], inv[8], izz[8], izzz[8];
   qmul(t, p.zz, p.zzz);
-  fq_inv_rp(inv, t);       // 1 / (ZZ ZZZ)
+  fq_inv_fermat(inv, t);       // 1 / (ZZ ZZZ)
   qmul(izz, inv, p.zzz);    // 1 / ZZ
   qmul(izzz, inv, p.zz);    // 1 / ZZZ
   qmul(o.x, p.x, izz);
@@ -51,16 +50,12 @@ __device__ void xyzz_to_affine_rp(aff_t& o, const xyzz_t& p) {
   reduce_once<FqP>(o.y, o.y);
 }
 
-// T[w * 16 + d] = d * 16^w * B (affine, R' form); T[w * 16] = (0, 0)
+// T[w * 16 + d] = d * 16^w * B (affine); T[w * 16] = (0, 0)
 __global__ void g1_fixed_table_kernel(const fe* base, fe* table) {
   const int w = threadIdx.x;
   if (w >= 64) return;
   aff_t b;
   ld_aff(b, base);
-  if (!aff_is_inf(b)) {
-    to_rprime(b.x, b.x);
-    to_rprime(b.y, b.y);
-  }
   xyzz_t p, acc;
   xyzz_from_aff(p, b);
   for (int i = 0; i < 4 * w; i++) xyzz_dbl(p, p);
@@ -71,7 +66,7 @@ __global__ void g1_fixed_table_kernel(const fe* base, fe* table) {
   st_fe(table + 2 * (w * 16) + 1, o.y);
   acc = p;
   for (int d = 1; d < 16; d++) {
-    xyzz_to_affine_rp(o, acc);
+    xyzz_to_affine(o, acc);
     st_fe(table + 2 * (w * 16 + d), o.x);
     st_fe(table + 2 * (w * 16 + d) + 1, o.y);
     xyzz_add(acc, p);
@@ -99,11 +94,7 @@ __global__ void __launch_bounds__(128) g1_fixed_mul_kernel(const fe* scalars, ui
     }
   }
   aff_t o;
-  xyzz_to_affine_rp(o, acc);
-  if (!aff_is_inf(o)) {
-    from_rprime(o.x, o.x);
-    from_rprime(o.y, o.y);
-  }
+  xyzz_to_affine(o, acc);
   st_fe(out + 2 * i, o.x);
   st_fe(out + 2 * i + 1, o.y);
 }

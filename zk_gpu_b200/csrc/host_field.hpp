@@ -297,20 +297,18 @@ inline void xyzz_add(Xyzz& p, const Xyzz& q) {
 
 // The last step of a windowed MSM on the host: Horner over the per-window
 // sums, sum_w 2^(c w) S_w, then normalisation.  winsum holds `windows` XYZZ
-// points (16 words each: X, Y, ZZ, ZZZ) in the device's R' = 2^260 form,
-// lazily reduced (< 2q).  out: normalised Jacobian (x, y, one), zeros for the
+// points (16 words each: X, Y, ZZ, ZZZ), lazily reduced (< 2q).  out: normalised Jacobian (x, y, one), zeros for the
 // identity.  A single GPU thread needs ~1.5 ms for the ~250 dependent
 // doublings; the host takes well under 0.1 ms.
 inline void msm_combine_windows(const uint64_t* winsum, uint32_t windows, uint32_t c, uint64_t out[12]) {
-  // R' -> R: times 2^252 mod q (mul divides by 2^256)
-  static constexpr E K252 = {{0, 0, 0, 0x1000000000000000ULL}};  // 2^252 < q
   auto load = [&](uint32_t w) {
     Xyzz p;
     E* co[4] = {&p.x, &p.y, &p.zz, &p.zzz};
     for (int k = 0; k < 4; k++) {
       E v;
       std::memcpy(v.v, winsum + 16 * (size_t)w + 4 * k, 32);
-      *co[k] = mul(v, K252);
+      if (geq_p(v.v)) subp(v.v);
+      *co[k] = v;
     }
     return p;
   };

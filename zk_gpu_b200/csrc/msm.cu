@@ -185,18 +185,15 @@ __global__ void scan_add_kernel(uint32_t* out, uint32_t* cursor, const uint32_t*
 constexpr uint32_t BA_K = 16;  // pair sums per task (one chain of products)
 constexpr uint32_t BA_G = 32;  // task products per inversion
 
-__device__ __forceinline__ void fq_one_rp(uint32_t r[8]) { set_one_rp<FqP>(r); }
-
-// a^-1 for a != 0 in R' form (x 2^260), lazy in, canonical out: the divstep
-// inversion (fq_inv.cuh) of the representative a 2^260 gives a^-1 2^-260,
-// and one product with 2^780 mod q returns it to R' form.
-__device__ __forceinline__ void fq_inv_rp_bin(uint32_t r[8], const uint32_t a[8]) {
-  const uint32_t k780[8] = {0x3fe3a1a8u, 0x13e32478u, 0x6ad256c5u, 0xc59c2897u,
-                            0x3603f972u, 0xc5387239u, 0x8d1987f5u, 0x10f16dedu};
+// a^-1 for a != 0 in Montgomery form, lazy in, canonical out: the divstep
+// inversion (fq_inv.cuh) of the representative a 2^256 gives a^-1 2^-256,
+// and one product with 2^768 mod q returns it to Montgomery form.
+__device__ __forceinline__ void fq_inv_mont(uint32_t r[8], const uint32_t a[8]) {
+  const uint32_t k768[8] = {0xda1530dfu, 0xb1cd6dafu, 0xa7283db6u, 0x62f210e6u, 0x0ada0afbu, 0xef7f0b0cu, 0x2d592544u, 0x20fd6e90u};
   uint32_t c[8], t[8];
   reduce_once<FqP>(c, a);
   fq_inv_divsteps(t, c);
-  qmul(r, t, k780);
+  qmul(r, t, k768);
   reduce_once<FqP>(r, r);
 }
 
@@ -323,7 +320,7 @@ __device__ __forceinline__ void ba_stage_pq(uint4* st, uint32_t bd, const fe* sr
   if (p) cp_fe(st, bd, 8, p);
 }
 
-// denominator of one pair sum (R' one when no inversion is needed: a carried
+// denominator of one pair sum (one when no inversion is needed: a carried
 // point, an identity operand, or P = -Q), from the staged x coordinates;
 // equal x (doubling or P = -Q, rare) reads both points again for y
 template <bool FIRST>
@@ -349,7 +346,7 @@ __device__ __forceinline__ void ba_denominator(uint32_t d[8], const uint4* st, u
       }
     }
   }
-  fq_one_rp(d);
+  set_one<FqP>(d);
 }
 
 // buckets with at most one entry are final before any round; every count
@@ -462,7 +459,7 @@ __global__ void __launch_bounds__(128) ba_invert_kernel(fe* tot, fe* tpre, const
       st_fe(tpre + i, acc);
     }
     uint32_t inv[8];
-    fq_inv_rp_bin(inv, acc);
+    fq_inv_mont(inv, acc);
     for (uint32_t i = i1 - 1; i > i0; i--) {
       uint32_t p[8], it[8];
       ld_fe(p, tpre + i - 1);
@@ -538,7 +535,7 @@ __global__ void __launch_bounds__(256, 2) ba_apply_kernel(const fe* __restrict__
           kind = 2;
         }
       }
-      if (kind == 0) fq_one_rp(d);
+      if (kind == 0) set_one<FqP>(d);
       uint32_t inv_d[8];
       if (q > q0) {
         uint32_t p[8];
@@ -781,19 +778,6 @@ __global__ void __launch_bounds__(256) msm_window_kernel(const fe* seg_t, const 
   }
 }
 
-// bases (R form, as the API holds them) -> R' form for the curve arithmetic
-__global__ void msm_convert_bases_kernel(const fe* in, fe* out, uint64_t n) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t x[8], y[8];
-  ld_fe(x, in + 2 * i);
-  ld_fe(y, in + 2 * i + 1);
-  to_rprime(x, x);
-  to_rprime(y, y);
-  st_fe(out + 2 * i, x);
-  st_fe(out + 2 * i + 1, y);
-}
-
 __global__ void zero_out_kernel(fe* out) {
   if (threadIdx.x < 3) {
     uint32_t z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -886,7 +870,7 @@ struct MsmLayout {
   uint64_t tasks0 = 0;
   uint64_t chunks = 0;           // tail chunks, upper bound
   bool ok = false;
-  uint64_t bytes(bool own_winsum, uint64_t nbases_convert) const {
+  uint64_t bytes(bool own_winsum) const {
     const uint64_t T1 = T + 1ull;
     uint64_t b = 0;
     b += T * 4ull * 2 + T1 * 4 + (nblk + 1ull) * 4 + E * 4;        // counts, cursor, offsets, bsums, list
@@ -895,7 +879,6 @@ struct MsmLayout {
     b += tasks0 * 32 * 2;                                         // task products, their prefixes
     b += T * 4ull * 2 + chunks * 128 + 4;                         // tail: chunk counts, heavy list, chunk sums
     b += T * 128ull + segs * 256ull + (own_winsum ? W * 128ull : 0);  // buckets, segment T_s and S_s
-    b += nbases_convert * 64;
     return b + 24 * 256;  // pool granularity per allocation
   }
 };
@@ -943,11 +926,10 @@ int sm_count() {
 
 // n: scalars (all jobs); jobs > 1: job_off (device, jobs + 1 entries) splits
 // them and every job reads bases [0, nbases); the window sums of job j are
-// windows [j W, (j + 1) W) of wout.  bases_rp_given: the bases are already in
-// the R' form of the curve arithmetic (resident bases converted once).
+// windows [j W, (j + 1) W) of wout.
 cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe* d_out, cudaStream_t s,
                          int c_override, uint64_t* launches, MsmWindowsOut* wout, const uint32_t* job_off,
-                         uint32_t jobs, uint64_t nbases, bool bases_rp_given) {
+                         uint32_t jobs) {
   uint64_t nl = 0;
   if (n == 0) {
     if (wout) {
@@ -973,7 +955,7 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
   uint32_t *counts = nullptr, *offsets = nullptr, *cursor = nullptr, *bsums = nullptr, *list = nullptr;
   uint32_t *cnt = nullptr, *cprev = nullptr, *np = nullptr, *joff[2] = {nullptr, nullptr};
   fe *fin = nullptr, *buf[2] = {nullptr, nullptr}, *pre = nullptr, *tot = nullptr, *tpre = nullptr;
-  fe *buckets = nullptr, *segres = nullptr, *segsum = nullptr, *winsum = nullptr, *bases_rp = nullptr;
+  fe *buckets = nullptr, *segres = nullptr, *segsum = nullptr, *winsum = nullptr;
   fe* chunk_res = nullptr;
   uint32_t *nch = nullptr, *heavy = nullptr, *heavy_count = nullptr;
   cudaError_t e = cudaSuccess;
@@ -1007,7 +989,6 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
     winsum = wout->d_winsum;  // caller's buffer, left for the host's Horner step
   else
     alloc((void**)&winsum, W * 128ull);
-  if (!bases_rp_given) alloc((void**)&bases_rp, nbases * 64ull);
   if (e == cudaSuccess) {
     int dev = 0;
     e = cudaGetDevice(&dev);
@@ -1020,12 +1001,6 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
     cudaMemsetAsync(counts, 0, T * 4ull, s);
     const unsigned g = (unsigned)((n + 255) / 256);
     const unsigned gb = (T + 255) / 256;
-    const fe* bases = d_bases;
-    if (!bases_rp_given) {
-      msm_convert_bases_kernel<<<(unsigned)((nbases + 255) / 256), 256, 0, s>>>(d_bases, bases_rp, nbases);
-      bases = bases_rp;
-      nl++;
-    }
     {
       ProfScope ps("msm_count", s, nd, nd * 32);
       msm_count_kernel<<<g, 256, 0, s>>>(d_scalars, n, (uint32_t)p.c, Wj, counts, job_off, jobs);
@@ -1042,14 +1017,14 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
       // convention: 6 Fq products per point-window (the batch-affine cost);
       // algorithmic bytes: each entry's index and signed base read once
       ProfScope ps("msm_bucket", s, (double)entries * 6, (double)entries * 68);
-      ba_setup_kernel<<<gb, 256, 0, s>>>(counts, offsets, list, bases, cnt, fin, T);
+      ba_setup_kernel<<<gb, 256, 0, s>>>(counts, offsets, list, d_bases, cnt, fin, T);
       nl++;
       uint64_t jb = l.jb[0];
       for (uint32_t r = 0; r < l.rounds; r++) {
         const bool first = r == 0;
         uint32_t* jo = joff[r & 1];
         const uint32_t* in_off = first ? offsets : joff[(r + 1) & 1];
-        const fe* src = first ? bases : buf[(r + 1) & 1];
+        const fe* src = first ? d_bases : buf[(r + 1) & 1];
         fe* dst = buf[r & 1];
         ba_jobs_kernel<<<gb, 256, 0, s>>>(cnt, cprev, np, T);
         scan_block_kernel<<<nblk, 1024, 0, s>>>(np, jo, bsums, T);
@@ -1105,37 +1080,29 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
                     (void*)cprev, (void*)np, (void*)joff[0], (void*)joff[1], (void*)fin, (void*)buf[0],
                     (void*)buf[1], (void*)pre, (void*)tot, (void*)tpre, (void*)buckets, (void*)segres, (void*)segsum,
                     (void*)nch, (void*)heavy, (void*)heavy_count, (void*)chunk_res,
-                    (void*)(wout ? nullptr : winsum), (void*)bases_rp})
+                    (void*)(wout ? nullptr : winsum)})
     if (ptr) cudaFreeAsync(ptr, s);
   if (launches) *launches = nl;
   return e;
 }
 }  // namespace
 
-uint64_t msm_scratch_bytes(uint64_t n_total, uint32_t jobs, uint64_t nbases, bool bases_rp_given, bool own_winsum,
-                           int device) {
+uint64_t msm_scratch_bytes(uint64_t n_total, uint32_t jobs, bool own_winsum, int device) {
   if (n_total == 0) return 256;
   const MsmLayout l = msm_layout(n_total, jobs, 0, device);
   if (!l.ok) return ~0ull >> 2;
-  return l.bytes(own_winsum, bases_rp_given ? 0 : nbases);
-}
-
-cudaError_t msm_convert_bases(const fe* d_in, fe* d_out, uint64_t n, cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  msm_convert_bases_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_in, d_out, n);
-  return cudaGetLastError();
+  return l.bytes(own_winsum);
 }
 
 cudaError_t msm_run(const fe* d_scalars, const fe* d_bases, uint64_t n, fe* d_out, cudaStream_t s, int c_override,
-                    uint64_t* launches, MsmWindowsOut* wout, bool bases_rp) {
-  return msm_run_impl(d_scalars, d_bases, n, d_out, s, c_override, launches, wout, nullptr, 1, n, bases_rp);
+                    uint64_t* launches, MsmWindowsOut* wout) {
+  return msm_run_impl(d_scalars, d_bases, n, d_out, s, c_override, launches, wout, nullptr, 1);
 }
 
 cudaError_t msm_run_multi(const fe* d_scalars, const fe* d_bases, const uint32_t* d_job_off, uint32_t jobs,
-                          uint64_t n_total, uint64_t max_n, cudaStream_t s, uint64_t* launches, MsmWindowsOut* wout,
-                          bool bases_rp) {
+                          uint64_t n_total, cudaStream_t s, uint64_t* launches, MsmWindowsOut* wout) {
   if (!wout || !wout->d_winsum || jobs == 0 || !d_job_off || n_total >= (1ull << 32)) return cudaErrorInvalidValue;
-  return msm_run_impl(d_scalars, d_bases, n_total, nullptr, s, 0, launches, wout, d_job_off, jobs, max_n, bases_rp);
+  return msm_run_impl(d_scalars, d_bases, n_total, nullptr, s, 0, launches, wout, d_job_off, jobs);
 }
 
 }  // namespace zk

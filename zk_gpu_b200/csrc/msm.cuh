@@ -44,33 +44,24 @@ int tuned_msm_window(int device, int log_n);
 // host (host::fq::msm_combine_windows), which does the ~250 dependent
 // doublings of the Horner step far faster than one GPU thread.
 struct MsmWindowsOut {
-  fe* d_winsum = nullptr;  // >= plan.windows * 4 elements (XYZZ, R' form)
+  fe* d_winsum = nullptr;  // >= plan.windows * 4 elements (XYZZ)
   uint32_t windows = 0;    // set by msm_run (0 for n = 0)
   uint32_t c = 0;
 };
 constexpr uint32_t MSM_MAX_WINDOWS = 64;  // c >= 4
-// bases_rp: d_bases_xy is already in the R' = 2^260 form of the curve
-// arithmetic (msm_convert_bases; resident bases are converted once)
 cudaError_t msm_run(const fe* d_scalars, const fe* d_bases_xy, uint64_t n, fe* d_out, cudaStream_t s,
-                    int c_override = 0, uint64_t* launches = nullptr, MsmWindowsOut* wout = nullptr,
-                    bool bases_rp = false);
+                    int c_override = 0, uint64_t* launches = nullptr, MsmWindowsOut* wout = nullptr);
 // Several MSMs over one base array (the serving loop's jobs against resident
 // bases) in one pass: job j's scalars are [off[j], off[j+1]) of d_scalars
 // (d_job_off: jobs + 1 offsets in device memory, off[0] = 0), each against
-// bases [0, n_j); max_n = the largest n_j.  One window size (the plan of the
+// bases [0, n_j).  One window size (the plan of the
 // mean job size); job j's window sums land in windows [j W, (j + 1) W) of
 // wout->d_winsum (>= jobs * W * 4 elements), W = wout->windows on return.
 cudaError_t msm_run_multi(const fe* d_scalars, const fe* d_bases_xy, const uint32_t* d_job_off, uint32_t jobs,
-                          uint64_t n_total, uint64_t max_n, cudaStream_t s, uint64_t* launches,
-                          MsmWindowsOut* wout, bool bases_rp = false);
+                          uint64_t n_total, cudaStream_t s, uint64_t* launches, MsmWindowsOut* wout);
 // Device scratch one msm_run / msm_run_multi call allocates from the stream
-// pool (n_total scalars over `jobs` MSMs; nbases converted unless bases_rp;
-// own_winsum: the window sums are not the caller's buffer; the window size of
+// pool (n_total scalars over `jobs` MSMs; own_winsum: the window sums are not the caller's buffer; the window size of
 // `device`, -1 = the current device).
-uint64_t msm_scratch_bytes(uint64_t n_total, uint32_t jobs, uint64_t nbases, bool bases_rp, bool own_winsum,
-                           int device = -1);
-// Affine bases from the API's R form (x 2^256) to the curve arithmetic's
-// R' form (x 2^260), canonical; (0, 0) stays (0, 0).  In place is allowed.
-cudaError_t msm_convert_bases(const fe* d_in, fe* d_out, uint64_t n, cudaStream_t s);
+uint64_t msm_scratch_bytes(uint64_t n_total, uint32_t jobs, bool own_winsum, int device = -1);
 
 }  // namespace zk

@@ -132,9 +132,8 @@ __global__ void ntt_tiny_kernel(fe* a, uint32_t log_n, fe w, const fe* pre_lo, c
       uint32_t c0[8], c1[8];
       ld_fe_nc(c0, pre_lo + (i & ((1u << pre_shift) - 1)));
       ld_fe_nc(c1, pre_hi + (i >> pre_shift));
-      mul_rp<P_r>(c0, c0, c1);
-      mul_rp<P_r>(in[i], in[i], c0);
-      reduce_once<P_r>(in[i], in[i]);
+      mul_lazy<P_r>(c0, c0, c1);
+      mul<P_r>(in[i], in[i], c0);
     }
   }
   uint32_t acc[8];
@@ -150,8 +149,7 @@ __global__ void ntt_tiny_kernel(fe* a, uint32_t log_n, fe w, const fe* pre_lo, c
       mul<P_r>(wik, wik, wk);
     }
     if (has_post) {
-      mul_rp<P_r>(acc, acc, post.w);
-      reduce_once<P_r>(acc, acc);
+      mul<P_r>(acc, acc, post.w);
     }
   }
   __syncthreads();
@@ -163,7 +161,7 @@ __global__ void pow_seq_kernel(fe* out, fe base, uint64_t count, uint64_t step) 
   const uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (e >= count) return;
   uint32_t r[8];
-  pow_u64_rp<P_r>(r, base.w, e * step);
+  pow_u64<P_r>(r, base.w, e * step);
   st_fe(out + e, r);
 }
 
@@ -176,8 +174,7 @@ __global__ void twist_table_kernel(fe* out, const fe* lo, const fe* hi, uint32_t
   uint32_t a[8], b[8];
   ld_fe_nc(a, lo + (e & ((1ull << shift) - 1)));
   ld_fe_nc(b, hi + (e >> shift));
-  mul_rp<P_r>(a, a, b);
-  reduce_once<P_r>(a, a);
+  mul<P_r>(a, a, b);
   st_fe(out + idx, a);
 }
 
@@ -192,9 +189,8 @@ __global__ void scale_copy_kernel(fe* dst, const fe* src, uint64_t n, uint64_t d
     uint32_t a[8], b[8];
     ld_fe_nc(a, lo + (i & ((1ull << shift) - 1)));
     ld_fe_nc(b, hi + (i >> shift));
-    mul_rp<P_r>(a, a, b);
-    mul_rp<P_r>(v, v, a);
-    reduce_once<P_r>(v, v);
+    mul_lazy<P_r>(a, a, b);
+    mul<P_r>(v, v, a);
   }
   st_fe(dst + i * dst_stride, v);
 }
@@ -207,9 +203,6 @@ static fe to_fe(const host::Fr& a) {
   std::memcpy(r.w, a.v, 32);
   return r;
 }
-// R-form (x 2^256) -> R'-form (x 2^260): every constant the kernels multiply
-// data by (roots, twists, coset powers, scales) is kept in R' form for mul_rp.
-static fe to_fe_rp(const host::Fr& a) { return to_fe(host::mul(a, host::from_u64(16))); }
 
 static cudaError_t pow_two_level(fe** lo, fe** hi, uint32_t* shift, const host::Fr& base, int log_count,
                                  cudaStream_t s, bool pooled) {
@@ -229,20 +222,19 @@ static cudaError_t pow_two_level(fe** lo, fe** hi, uint32_t* shift, const host::
     if (e != cudaSuccess) return e;
   }
   const host::Fr bstep = host::pow_2k(base, sh);
-  pow_seq_kernel<<<(unsigned)((nlo + 255) / 256), 256, 0, s>>>(*lo, to_fe_rp(base), nlo, 1);
-  pow_seq_kernel<<<(unsigned)((nhi + 255) / 256), 256, 0, s>>>(*hi, to_fe_rp(bstep), nhi, 1);
+  pow_seq_kernel<<<(unsigned)((nlo + 255) / 256), 256, 0, s>>>(*lo, to_fe(base), nlo, 1);
+  pow_seq_kernel<<<(unsigned)((nhi + 255) / 256), 256, 0, s>>>(*hi, to_fe(bstep), nhi, 1);
   *shift = sh;
   return cudaGetLastError();
 }
 
-// t[i] *= scale (R' form)
+// t[i] *= scale
 __global__ void scale_table_kernel(fe* t, fe scale, uint64_t count) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= count) return;
   uint32_t v[8];
   ld_fe(v, t + i);
-  mul_rp<P_r>(v, v, scale.w);
-  reduce_once<P_r>(v, v);
+  mul<P_r>(v, v, scale.w);
   st_fe(t + i, v);
 }
 
@@ -251,7 +243,7 @@ cudaError_t pow_tables_make(PowTables* t, const host::Fr& c, int log_n, cudaStre
   cudaError_t e = pow_two_level(&t->lo, &t->hi, &t->shift, c, log_n, s, pooled);
   if (e == cudaSuccess && scale) {
     const uint64_t nlo = 1ull << t->shift;
-    scale_table_kernel<<<(unsigned)((nlo + 255) / 256), 256, 0, s>>>(t->lo, to_fe_rp(*scale), nlo);
+    scale_table_kernel<<<(unsigned)((nlo + 255) / 256), 256, 0, s>>>(t->lo, to_fe(*scale), nlo);
     e = cudaGetLastError();
   }
   return e;
@@ -276,7 +268,7 @@ static cudaError_t build_tables(NttTables* t, cudaStream_t s) {
     e = cudaMalloc((void**)&t->inner[k], half * sizeof(fe));
     if (e != cudaSuccess) return e;
     t->bytes += half * sizeof(fe);
-    pow_seq_kernel<<<(unsigned)((half + 255) / 256), 256, 0, s>>>(t->inner[k], to_fe_rp(wm), half, 1);
+    pow_seq_kernel<<<(unsigned)((half + 255) / 256), 256, 0, s>>>(t->inner[k], to_fe(wm), half, 1);
     if (k + 1 < p.npass) {
       const uint64_t total = 1ull << (b + log_J);
       e = cudaMalloc((void**)&t->twist[k], total * sizeof(fe));
@@ -331,7 +323,7 @@ cudaError_t ntt_tables_fill(NttTables* t, const host::Fr& omega, int log_n, fe* 
     const uint64_t half = b >= 1 ? (1ull << (b - 1)) : 1;
     t->inner[k] = cur;
     cur += half;
-    pow_seq_kernel<<<(unsigned)((half + 255) / 256), 256, 0, s>>>(t->inner[k], to_fe_rp(wm), half, 1);
+    pow_seq_kernel<<<(unsigned)((half + 255) / 256), 256, 0, s>>>(t->inner[k], to_fe(wm), half, 1);
     if (k + 1 < p.npass) {
       const int lc = b + log_J;
       const uint32_t sh = (uint32_t)((lc + 1) / 2);
@@ -340,8 +332,8 @@ cudaError_t ntt_tables_fill(NttTables* t, const host::Fr& omega, int log_n, fe* 
       fe* hi = cur + nlo;
       t->twist[k] = cur + nlo + nhi;
       cur += nlo + nhi + total;
-      pow_seq_kernel<<<(unsigned)((nlo + 255) / 256), 256, 0, s>>>(lo, to_fe_rp(wMJ), nlo, 1);
-      pow_seq_kernel<<<(unsigned)((nhi + 255) / 256), 256, 0, s>>>(hi, to_fe_rp(host::pow_2k(wMJ, sh)), nhi, 1);
+      pow_seq_kernel<<<(unsigned)((nlo + 255) / 256), 256, 0, s>>>(lo, to_fe(wMJ), nlo, 1);
+      pow_seq_kernel<<<(unsigned)((nhi + 255) / 256), 256, 0, s>>>(hi, to_fe(host::pow_2k(wMJ, sh)), nhi, 1);
       twist_table_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(t->twist[k], lo, hi, sh, (uint32_t)log_J,
                                                                           total);
     } else {
@@ -432,7 +424,7 @@ uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const Nt
   }
   if (final_pass && post) {
     pp.has_post = 1;
-    pp.post = to_fe_rp(*post);
+    pp.post = to_fe(*post);
   }
   if (final_pass && f.post_tab) {
     pp.post_lo = f.post_tab->lo;
@@ -488,7 +480,7 @@ cudaError_t ntt_run(const NttTables& t, fe* d_a, fe* d_tmp, const NttFuse& f, cu
   if (L <= 2) {
     if (f.post_tab) return cudaErrorInvalidValue;  // the direct kernel takes constant scales only
     fe po{};
-    if (post) po = to_fe_rp(*post);
+    if (post) po = to_fe(*post);
     ntt_tiny_kernel<<<1, 32, 0, s>>>(d_a, (uint32_t)L, to_fe(t.omega), pre ? pre->lo : nullptr, pre ? pre->hi : nullptr,
                                      pre ? pre->shift : 0u, post ? 1u : 0u, po);
     return cudaGetLastError();
@@ -508,7 +500,7 @@ cudaError_t ntt_run(const NttTables& t, fe* d_a, fe* d_tmp, const NttFuse& f, cu
   return cudaSuccess;
 }
 
-static size_t batch_smem_bytes() { return (size_t)8 * 2048 * 4 + (size_t)1024 * 40; }  // B <= 11
+static size_t batch_smem_bytes() { return (size_t)8 * 2048 * 4 + (size_t)1024 * 32; }  // B <= 11
 
 int ntt_batch_grid(int device) {
   static int cached[64] = {0};

@@ -96,8 +96,8 @@ void table_cache_clear(int device);
 struct PassParams {
   const fe* in;
   fe* out;
-  const fe* inner;   // w_m^e, e < m/2 (R' form)
-  const fe* twist;   // [k * J + j], non-final passes (R' form)
+  const fe* inner;   // w_m^e, e < m/2
+  const fe* twist;   // [k * J + j], non-final passes
   const fe* pre_lo;  // coset powers (first pass), or null
   const fe* pre_hi;
   uint32_t pre_shift;
@@ -109,7 +109,7 @@ struct PassParams {
   uint32_t G;
   uint32_t is_final;
   uint32_t has_post;
-  fe post;  // R' form
+  fe post;
   // final pass: output k multiplied by post_lo[k & mask] * post_hi[k >> shift]
   const fe* post_lo;
   const fe* post_hi;

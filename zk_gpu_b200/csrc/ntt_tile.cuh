@@ -33,10 +33,11 @@ __device__ __forceinline__ void ld_smem_fe(uint32_t r[8], const uint32_t* plane0
 #pragma unroll
   for (int k = 0; k < 8; k++) r[k] = plane0[k * plane_stride + a];
 }
-// a twiddle stored pre-split as 5 planes of 52-bit limbs (doubles)
-__device__ __forceinline__ void ld_smem_tw(double r[5], const double* plane0, uint32_t plane_stride, uint32_t a) {
-#pragma unroll
-  for (int k = 0; k < 5; k++) r[k] = plane0[k * plane_stride + a];
+// a twiddle: its low and high 16 bytes in two planes
+__device__ __forceinline__ void ld_smem_tw(uint32_t r[8], const uint4* plane0, uint32_t plane_stride, uint32_t a) {
+  const uint4 x = plane0[a], y = plane0[plane_stride + a];
+  r[0] = x.x; r[1] = x.y; r[2] = x.z; r[3] = x.w;
+  r[4] = y.x; r[5] = y.y; r[6] = y.z; r[7] = y.w;
 }
 __device__ __forceinline__ void st_smem_fe(uint32_t* plane0, uint32_t plane_stride, uint32_t a, const uint32_t r[8]) {
 #pragma unroll
@@ -52,56 +53,29 @@ __device__ __forceinline__ void st_smem_fe(uint32_t* plane0, uint32_t plane_stri
 // pre-multiply, the output scale) are calls only in passes of width
 // B >= ZK_NTT_CALL_EDGE_MIN_B: inlined they overlap their loads and run
 // faster in the narrow passes, while in the wide ones the shorter code and
-// lower register pressure win.  Measured on B200 with bit-identical
-// results, against the build that inlined every product (bench, autotuned
-// plans): forward NTT 2^24 4.72 -> 4.45 ms, LDE 2^24 -> 2^26 25.9 -> 24.7 ms,
-// 512 batched jobs of 2^10..2^20 31.8 -> 28.2 ms, the same jobs one call
-// each 94 -> 71 ms.
+// lower register pressure win.
 #ifndef ZK_NTT_CALL_PRODUCT
 #define ZK_NTT_CALL_PRODUCT 1
 #endif
 #ifndef ZK_NTT_CALL_EDGE_MIN_B
 #define ZK_NTT_CALL_EDGE_MIN_B 7
 #endif
-struct Tw5 { double d[5]; };
-template <class P>
-__device__ __noinline__ Fe8 mul_rp_pre_call(const Fe8 a, const Tw5 b) {
-  Fe8 r;
-  mul_rp_pre<P>(r.w, a.w, b.d);
-  return r;
-}
 template <bool CALL = (ZK_NTT_CALL_PRODUCT != 0)>
 __device__ __forceinline__ void ntt_mul(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) {
 #if ZK_NTT_CALL_PRODUCT
   if constexpr (!CALL) {
-    mul_rp<P_r>(r, a, b);
+    mul_lazy<P_r>(r, a, b);
     return;
   }
-  mul_rp_out<P_r>(r, a, b);
+  mul_out<P_r>(r, a, b);
 #else
-  mul_rp<P_r>(r, a, b);
+  mul_lazy<P_r>(r, a, b);
 #endif
 }
-__device__ __forceinline__ void ntt_mul_pre(uint32_t r[8], const uint32_t a[8], const double w[5]) {
-#if ZK_NTT_CALL_PRODUCT
-  Fe8 av;
-  Tw5 wv;
-#pragma unroll
-  for (int k = 0; k < 8; k++) av.w[k] = a[k];
-#pragma unroll
-  for (int k = 0; k < 5; k++) wv.d[k] = w[k];
-  const Fe8 rv = mul_rp_pre_call<P_r>(av, wv);
-#pragma unroll
-  for (int k = 0; k < 8; k++) r[k] = rv.w[k];
-#else
-  mul_rp_pre<P_r>(r, a, w);
-#endif
-}
-
 // One round: registers hold i(r) = ins3<LO>(q, r); perform the DIF stages
-// with butterfly bits HI-1 .. LO.  tws: inner roots w_m^e (e < m/2), 5 planes.
+// with butterfly bits HI-1 .. LO.  tws: inner roots w_m^e (e < m/2), 2 planes.
 template <int B, int LO, int HI>
-__device__ __forceinline__ void ntt_round(uint32_t x[8][8], uint32_t q, const double* tws) {
+__device__ __forceinline__ void ntt_round(uint32_t x[8][8], uint32_t q, const uint4* tws) {
   constexpr uint32_t HALF = 1u << (B - 1);
 #pragma unroll
   for (int b = HI - 1; b >= LO; b--) {
@@ -120,15 +94,15 @@ __device__ __forceinline__ void ntt_round(uint32_t x[8][8], uint32_t q, const do
 #pragma unroll
           for (int k = 0; k < 8; k++) x[r2][k] = t[k];
         } else {
-          double w[5];
+          uint32_t w[8];
           ld_smem_tw(w, tws, HALF, e);
-          ntt_mul_pre(x[r2], t, w);
+          ntt_mul<true>(x[r2], t, w);
         }
       } else {
         const uint32_t e = ((q & ((1u << LO) - 1u)) | ((uint32_t)(r & ((1 << rb) - 1)) << LO)) << (B - 1 - b);
-        double w[5];
+        uint32_t w[8];
         ld_smem_tw(w, tws, HALF, e);
-        ntt_mul_pre(x[r2], t, w);
+        ntt_mul<true>(x[r2], t, w);
       }
     }
   }
@@ -151,7 +125,7 @@ __device__ __forceinline__ void ntt_exchange(uint32_t x[8][8], uint32_t q, uint3
 
 template <int B, int HI>
 __device__ __forceinline__ void ntt_rounds(uint32_t x[8][8], uint32_t q, uint32_t gbase, uint32_t* sm,
-                                           uint32_t plane_stride, const double* tws, bool active) {
+                                           uint32_t plane_stride, const uint4* tws, bool active) {
   constexpr int LO = HI - 3 > 0 ? HI - 3 : 0;
   ntt_round<B, LO, HI>(x, q, tws);
   if constexpr (LO > 0) {
@@ -176,7 +150,7 @@ __device__ __forceinline__ void ntt_pass_tile(const PassParams& p, uint64_t tile
   constexpr uint32_t T = M / 8;  // threads per column
   const uint32_t G = p.G;
   const uint32_t plane_stride = G * M;
-  double* tws = reinterpret_cast<double*>(smem + 8 * plane_stride);  // 8-byte aligned: 32 G M bytes in
+  uint4* tws = reinterpret_cast<uint4*>(smem + 8 * plane_stride);  // 32 G M bytes in
 
   const uint32_t tid = threadIdx.x;
   const uint32_t g = tid / T, q = tid % T;
@@ -184,11 +158,9 @@ __device__ __forceinline__ void ntt_pass_tile(const PassParams& p, uint64_t tile
 
   for (uint32_t e = tid; e < M / 2; e += blockDim.x) {
     uint32_t w[8];
-    double wl[5];
     ld_fe_nc(w, p.inner + e);
-    split52(wl, w);  // stored pre-split: 5 limb planes
-#pragma unroll
-    for (int k = 0; k < 5; k++) tws[k * (M / 2) + e] = wl[k];
+    tws[e] = make_uint4(w[0], w[1], w[2], w[3]);
+    tws[M / 2 + e] = make_uint4(w[4], w[5], w[6], w[7]);
   }
 
   // element indices are < 2^28: 32-bit arithmetic, powers of two as shifts
@@ -307,7 +279,7 @@ template <int B>
 inline cudaError_t launch_pass(const PassParams& pp, uint64_t ncta, cudaStream_t s) {
   constexpr uint32_t M = 1u << B;
   const uint32_t threads = pp.G * (M / 8);
-  const size_t smem = (size_t)8 * pp.G * M * 4 + (size_t)(M / 2) * 40;
+  const size_t smem = (size_t)8 * pp.G * M * 4 + (size_t)(M / 2) * 32;
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);

@@ -38,7 +38,7 @@ using clk = std::chrono::steady_clock;
 // its scalars, its window sums and the pass's scratch (resident bases are
 // already in the curve arithmetic's form, so nothing is converted).
 uint64_t msm_job_bytes(uint64_t n, int device) {
-  return n * 32 + MSM_MAX_WINDOWS * 128ull + msm_scratch_bytes(n, 1, n, true, false, device);
+  return n * 32 + MSM_MAX_WINDOWS * 128ull + msm_scratch_bytes(n, 1, false, device);
 }
 
 host::Fr fr_of(const uint64_t v[4]) {
@@ -152,13 +152,9 @@ class Server {
     }
     BaseSet b;
     b.n = n;
-    // resident bases are kept in the curve arithmetic's R' form: converted
-    // once here (in place) instead of on every MSM over them
     cudaError_t e = cudaSetDevice(device_);
     if (e == cudaSuccess) e = cudaMalloc((void**)&b.d, std::max<uint64_t>(bytes, 64));
     if (e == cudaSuccess) e = cudaMemcpy(b.d, xy, bytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = msm_convert_bases(b.d, b.d, n, s_msm_[0]);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s_msm_[0]);
     if (e != cudaSuccess) {
       if (b.d) cudaFree(b.d);
       std::lock_guard<std::mutex> lk(mu_);
@@ -348,16 +344,15 @@ class Server {
     std::map<uint32_t, bool> merge_ok;
     for (auto& g : msm_groups) {
       const std::vector<JobRec*>& grp = g.second;
-      uint64_t tot = 0, max_n = 0, admitted = 0;
+      uint64_t tot = 0, admitted = 0;
       for (const JobRec* r : grp) {
         tot += r->job.n;
-        max_n = std::max<uint64_t>(max_n, r->job.n);
         admitted += r->bytes;
       }
       bool ok_merge = grp.size() >= 2 && tot <= (1ull << 25);
       if (ok_merge) {
         const uint64_t need = tot * 32 + grp.size() * (MSM_MAX_WINDOWS * 128ull + 4) +
-                              msm_scratch_bytes(tot, (uint32_t)grp.size(), max_n, true, false, device_);
+                              msm_scratch_bytes(tot, (uint32_t)grp.size(), false, device_);
         if (need > admitted) {  // borrow the difference from the free budget until the wave retires
           std::lock_guard<std::mutex> lk(mu_);
           ok_merge = adm_.take(need - admitted);
@@ -375,10 +370,8 @@ class Server {
       if (!merged(g.first)) continue;
       const BaseSet& bs = bases_[g.first];
       std::vector<uint32_t> off(grp.size() + 1, 0);
-      uint64_t max_n = 0;
       for (size_t k = 0; k < grp.size(); k++) {
         off[k + 1] = off[k] + (uint32_t)grp[k]->job.n;
-        max_n = std::max<uint64_t>(max_n, grp[k]->job.n);
       }
       const uint64_t n_total = off.back();
       fe *ds = nullptr, *dwin = nullptr;
@@ -398,7 +391,7 @@ class Server {
         uint64_t nl = 0;
         MsmWindowsOut wo;
         wo.d_winsum = dwin;
-        if (ok(msm_run_multi(ds, bs.d, doff, (uint32_t)grp.size(), n_total, max_n, w.s_msm, &nl, &wo, true))) {
+        if (ok(msm_run_multi(ds, bs.d, doff, (uint32_t)grp.size(), n_total, w.s_msm, &nl, &wo))) {
           merged_passes_++;
           merged_jobs_ += grp.size();
           for (size_t k = 0; k < grp.size(); k++) {
@@ -431,7 +424,7 @@ class Server {
           uint64_t nl = 0;
           MsmWindowsOut wo;
           wo.d_winsum = dwin;
-          if (ok(msm_run(ds, bs.d, j.n, nullptr, w.s_msm, 0, &nl, &wo, true))) {
+          if (ok(msm_run(ds, bs.d, j.n, nullptr, w.s_msm, 0, &nl, &wo))) {
             r->msm_out = next_msm_slot;
             next_msm_slot += kMsmSlotWords;
             r->msm_out[0] = wo.windows;
