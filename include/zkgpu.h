@@ -130,7 +130,7 @@ int zkgpu_extended_to_coeff_dev(int device, const uint64_t *d_ext, uint32_t log_
  * running under stream capture, or inside a runtime that owns every device
  * allocation.  It calls no allocator: its scratch (ping-pong buffer and root
  * tables) is a static device array in the library sized for log_n <=
- * ZKGPU_STATIC_NTT_MAX_LOG (about 16.8 MB per GPU, held until process exit);
+ * ZKGPU_STATIC_NTT_MAX_LOG (about 25.5 MB per GPU, held until process exit);
  * larger log_n returns ZKGPU_EINVAL.  It always runs the built-in pass plan
  * for log_n (the autotuner's choices are not consulted; results are the same,
  * only the speed can differ).  The first call on a device resolves the

@@ -199,3 +199,21 @@ def test_device_api_matches_host_api(zk, oracle):
     ref = oracle.best_fft(oracle.distribute_powers(a, oracle.to_mont(5)), w, log_n)
     ref = oracle.mul_vec(ref, np.tile(oracle.to_mont(3), (1 << log_n, 1)))
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("log_n", [3, 4, 5, 6, 7, 8, 9, 13, 14, 17, 19])
+def test_extreme_values(zk, oracle, log_n):
+    """Inputs of 0, 1, (p - 1) / 2 and p - 1 only: sums and differences inside
+    a pass reach the ends of the ranges its unreduced butterflies rely on, in
+    every narrow pass width, forward, inverse and on a coset."""
+    n = 1 << log_n
+    vals = np.stack([oracle.from_int(v) for v in (0, 1, (B.R_MOD - 1) // 2, B.R_MOD - 1)])
+    rng = np.random.default_rng(log_n)
+    w = oracle.omega(log_n)
+    for weights in ((0.5, 0.0, 0.0, 0.5), (0.25, 0.25, 0.25, 0.25), (0.02, 0.0, 0.0, 0.98)):
+        a = np.ascontiguousarray(vals[rng.choice(4, n, p=weights)])
+        assert np.array_equal(zk.fft(a, w, log_n), oracle.best_fft(a, w, log_n))
+        wi, d = oracle.inv(w), inv_n(oracle, log_n)
+        assert np.array_equal(zk.ifft(a, wi, log_n, d), oracle.ifft(a, wi, log_n, d))
+        c = oracle.from_int(B.R_MOD - 1)
+        assert np.array_equal(zk.coset_fft(a, w, log_n, c), oracle.best_fft(oracle.distribute_powers(a, c), w, log_n))

@@ -175,6 +175,210 @@ __device__ __forceinline__ void mul_out(uint32_t r[8], const uint32_t a[8], cons
   for (int k = 0; k < 8; k++) r[k] = rv.w[k];
 }
 
+// ---- products by tabulated multiplicands -----------------------------------
+// Half of a Montgomery product's 128 multiply-add pairs go into its reduction.
+// For a multiplicand w that is known beforehand (a root of unity, a twist),
+// tables of w 2^(32 s) mod p let rows of a that lie 32 s bits apart share one
+// reduction, so that only a few words are left to reduce:
+//   mul_w4: w^(k) = w 2^(64 k + 96) mod p, k < 4 (128 B): a = sum_k A_k 2^(64 k),
+//     V = sum_k A_k w^(k) < 4 2^64 p, three words reduced: 64 + 24 pairs;
+//   mul_w2: w^(k) = w 2^(128 k + 160) mod p, k < 2 (64 B): four words and one
+//     more reduced: 64 + 40 pairs.
+// Both take any a < 2^256 (5.29 p) and return a w mod p below p (1 + 2^-29),
+// in the form (Montgomery or not) a has; the last reduced word is there for
+// that bound, which lets a radix-8 butterfly add eight such values without
+// conditional subtractions in between.  Cycles per warp on one scheduler
+// (B200): 555 mul_lazy, about 460 mul_w2, about 390 mul_w4.
+
+// A += x b over the four pairs of A[0..7], the carry into the two words above
+__device__ __forceinline__ void row_mad_cc(uint32_t A[10], uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3,
+                                           uint32_t b) {
+  asm("mad.lo.cc.u32  %0, %10, %14, %0;\n\t"
+      "madc.hi.cc.u32 %1, %10, %14, %1;\n\t"
+      "madc.lo.cc.u32 %2, %11, %14, %2;\n\t"
+      "madc.hi.cc.u32 %3, %11, %14, %3;\n\t"
+      "madc.lo.cc.u32 %4, %12, %14, %4;\n\t"
+      "madc.hi.cc.u32 %5, %12, %14, %5;\n\t"
+      "madc.lo.cc.u32 %6, %13, %14, %6;\n\t"
+      "madc.hi.cc.u32 %7, %13, %14, %7;\n\t"
+      "addc.cc.u32    %8, %8, 0;\n\t"
+      "addc.u32       %9, %9, 0;"
+      : ZK_A8(A), "+r"(A[8]), "+r"(A[9])
+      : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(b));
+}
+// One reduced word on the chains E (E[0] = 0 already dropped into E[1..7] and
+// E89 = words 8, 9 of E) and O: afterwards E is the old O plus m p's even
+// words, O the old E >> 64 plus its odd ones.
+template <class P>
+__device__ __forceinline__ void reduce_word(uint32_t E[8], uint32_t O[8], uint32_t e8, uint32_t e9) {
+  uint32_t N[8], m;
+  asm("add.cc.u32     %8, %8, %10;\n\t"
+      "mul.lo.u32     %9, %8, %19;\n\t"
+      "madc.lo.cc.u32 %0, %9, %20, %11;\n\t"
+      "madc.hi.cc.u32 %1, %9, %20, %12;\n\t"
+      "madc.lo.cc.u32 %2, %9, %21, %13;\n\t"
+      "madc.hi.cc.u32 %3, %9, %21, %14;\n\t"
+      "madc.lo.cc.u32 %4, %9, %22, %15;\n\t"
+      "madc.hi.cc.u32 %5, %9, %22, %16;\n\t"
+      "madc.lo.cc.u32 %6, %9, %23, %17;\n\t"
+      "madc.hi.u32    %7, %9, %23, %18;"
+      : "=&r"(N[0]), "=&r"(N[1]), "=&r"(N[2]), "=&r"(N[3]), "=&r"(N[4]), "=&r"(N[5]), "=&r"(N[6]), "=&r"(N[7]),
+        "+r"(O[0]), "=&r"(m)
+      : "r"(E[1]), "r"(E[2]), "r"(E[3]), "r"(E[4]), "r"(E[5]), "r"(E[6]), "r"(E[7]), "r"(e8), "r"(e9), "n"(P::INV),
+        "n"(P::P1), "n"(P::P3), "n"(P::P5), "n"(P::P7));
+  row_mad_c(O, N[7], P::P0, P::P2, P::P4, P::P6, m);
+#pragma unroll
+  for (int j = 0; j < 8; j++) E[j] = O[j], O[j] = N[j];
+}
+
+// Table words through a loader: w(k, v) puts the eight words of w^(k) in v.
+template <class P, class W>
+__device__ __forceinline__ void mul_w4(uint32_t r[8], const uint32_t a[8], W w) {
+  uint32_t E[10], O[8], o8 = 0, v[8];
+  w(0, v);
+  row_mul(E, v[0], v[2], v[4], v[6], a[0]);
+  E[8] = E[9] = 0;
+  row_mul(O, v[1], v[3], v[5], v[7], a[0]);
+  row_mad_c(O, o8, v[0], v[2], v[4], v[6], a[1]);
+  row_mad(E + 2, v[1], v[3], v[5], v[7], a[1]);
+#pragma unroll
+  for (int k = 1; k < 4; k++) {
+    w(k, v);
+    row_mad_cc(E, v[0], v[2], v[4], v[6], a[2 * k]);
+    row_mad_c(O, o8, v[1], v[3], v[5], v[7], a[2 * k]);
+    row_mad_c(O, o8, v[0], v[2], v[4], v[6], a[2 * k + 1]);
+    row_mad(E + 2, v[1], v[3], v[5], v[7], a[2 * k + 1]);
+  }
+  const uint32_t m = E[0] * P::INV;
+  row_mad_cc(E, P::P0, P::P2, P::P4, P::P6, m);
+  row_mad_c(O, o8, P::P1, P::P3, P::P5, P::P7, m);
+  reduce_word<P>(E, O, E[8], E[9] + o8);
+  reduce_word<P>(E, O, 0u, 0u);
+  merge_chains(r, E, O);
+}
+template <class P>
+__device__ __forceinline__ void mul_w2(uint32_t r[8], const uint32_t a[8], const uint32_t v[8], const uint32_t w[8]) {
+  uint32_t E[8], O[8];
+  row_mul(E, v[0], v[2], v[4], v[6], a[0]);
+  row_mul(O, v[1], v[3], v[5], v[7], a[0]);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    if (i > 0) {
+      uint32_t N[8];
+      row_mad_shift(N, E, O[0], v[1], v[3], v[5], v[7], a[i]);
+#pragma unroll
+      for (int j = 0; j < 8; j++) E[j] = O[j], O[j] = N[j];
+      row_mad_c(E, O[7], v[0], v[2], v[4], v[6], a[i]);
+    }
+    row_mad(O, w[1], w[3], w[5], w[7], a[i + 4]);
+    row_mad_c(E, O[7], w[0], w[2], w[4], w[6], a[i + 4]);
+    const uint32_t m = E[0] * P::INV;
+    row_mad(O, P::P1, P::P3, P::P5, P::P7, m);
+    row_mad_c(E, O[7], P::P0, P::P2, P::P4, P::P6, m);
+  }
+  reduce_word<P>(E, O, 0u, 0u);
+  merge_chains(r, E, O);
+}
+
+// mul_w8: w^(k) = w 2^(32 k + 64) mod p, k < 8 (256 B), V < 8 2^32 p, two words
+// reduced: 64 + 16 pairs; the result is below p (1 + 2^-28).
+template <class P, class W>
+__device__ __forceinline__ void mul_w8(uint32_t r[8], const uint32_t a[8], W w) {
+  uint32_t E[8], O[8], e8 = 0, o8 = 0, v[8];
+  w(0, v);
+  row_mul(E, v[0], v[2], v[4], v[6], a[0]);
+  row_mul(O, v[1], v[3], v[5], v[7], a[0]);
+#pragma unroll
+  for (int k = 1; k < 8; k++) {
+    w(k, v);
+    row_mad_c(E, e8, v[0], v[2], v[4], v[6], a[k]);
+    row_mad_c(O, o8, v[1], v[3], v[5], v[7], a[k]);
+  }
+  const uint32_t m = E[0] * P::INV;
+  row_mad_c(E, e8, P::P0, P::P2, P::P4, P::P6, m);
+  row_mad_c(O, o8, P::P1, P::P3, P::P5, P::P7, m);
+  reduce_word<P>(E, O, e8, o8);
+  merge_chains(r, E, O);
+}
+
+// word j of K p (K p < 2^256: K <= 5)
+template <class P, uint32_t K>
+__host__ __device__ constexpr uint32_t kp(int j) {
+  uint64_t c = 0;
+  for (int i = 0; i <= j; i++) {
+    const uint32_t w = i == 0   ? P::P0
+                       : i == 1 ? P::P1
+                       : i == 2 ? P::P2
+                       : i == 3 ? P::P3
+                       : i == 4 ? P::P4
+                       : i == 5 ? P::P5
+                       : i == 6 ? P::P6
+                                : P::P7;
+    c = (c >> 32) + (uint64_t)w * K;
+  }
+  return (uint32_t)c;
+}
+#define ZK_KP_OPS(P, K)                                                                                      \
+  "n"(kp<P, K>(0)), "n"(kp<P, K>(1)), "n"(kp<P, K>(2)), "n"(kp<P, K>(3)), "n"(kp<P, K>(4)), "n"(kp<P, K>(5)), \
+      "n"(kp<P, K>(6)), "n"(kp<P, K>(7))
+
+// r = a + b (no reduction)
+__device__ __forceinline__ void add_raw(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) {
+  asm("add.cc.u32  %0, %8, %16;\n\t"
+      "addc.cc.u32 %1, %9, %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : ZK_A_OPS(a), ZK_A_OPS(b));
+}
+// r = a + K p - b (the caller keeps it within [0, 2^256))
+template <class P, uint32_t K>
+__device__ __forceinline__ void sub_off(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) {
+  uint32_t t[8];
+  asm("add.cc.u32  %0, %8, %16;\n\t"
+      "addc.cc.u32 %1, %9, %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
+      : ZK_A_OPS(a), ZK_KP_OPS(P, K));
+  asm("sub.cc.u32  %0, %8, %16;\n\t"
+      "subc.cc.u32 %1, %9, %17;\n\t"
+      "subc.cc.u32 %2, %10, %18;\n\t"
+      "subc.cc.u32 %3, %11, %19;\n\t"
+      "subc.cc.u32 %4, %12, %20;\n\t"
+      "subc.cc.u32 %5, %13, %21;\n\t"
+      "subc.cc.u32 %6, %14, %22;\n\t"
+      "subc.u32    %7, %15, %23;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : ZK_A_OPS(t), ZK_A_OPS(b));
+}
+// x -= K p if x >= K p
+template <class P, uint32_t K>
+__device__ __forceinline__ void cond_sub(uint32_t x[8]) {
+  uint32_t t[8], borrow;
+  asm("sub.cc.u32  %0, %9, %17;\n\t"
+      "subc.cc.u32 %1, %10, %18;\n\t"
+      "subc.cc.u32 %2, %11, %19;\n\t"
+      "subc.cc.u32 %3, %12, %20;\n\t"
+      "subc.cc.u32 %4, %13, %21;\n\t"
+      "subc.cc.u32 %5, %14, %22;\n\t"
+      "subc.cc.u32 %6, %15, %23;\n\t"
+      "subc.cc.u32 %7, %16, %24;\n\t"
+      "subc.u32    %8, 0, 0;"
+      : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]), "=r"(borrow)
+      : ZK_A_OPS(x), ZK_KP_OPS(P, K));
+#pragma unroll
+  for (int j = 0; j < 8; j++) x[j] = borrow ? x[j] : t[j];
+}
+
 // r = a + b - 2p if that does not borrow, else a + b.  Inputs < 2p.
 template <class P>
 __device__ __forceinline__ void add_lazy(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) {

@@ -2,15 +2,10 @@
 //
 // Per pass, one CTA owns G columns of one outer block (or, in the last pass,
 // G groups whose outputs are adjacent).  Each thread holds 8 elements of one
-// column and runs the m-point DIF DFT as "rounds": a round covers three
-// index bits [lo, lo+3) that the thread holds in registers and performs the
-// radix-2 stages whose butterfly bit falls in that range.  Between rounds the
-// column is exchanged through shared memory, stored as 8 u32 planes with the
-// XOR swizzle  addr = e ^ ((e >> 3) & 31),  which keeps every round's
-// 32-lane access pattern on 32 distinct banks for all b in [3, 12].
-// Twiddles of the last round are the 8th roots of unity (compile-time
-// indices, broadcast reads); the w == 1 butterflies skip the product.
-// Values stay in [0, 2p) between stages (lazy reduction, 4p < 2^256) and
+// column and runs the m-point DIF DFT as "rounds" (ntt_tile.cuh): a round
+// covers three index bits [lo, lo+3) that the thread holds in registers.
+// Between rounds the columns are exchanged through shared memory, stored as
+// 8 u32 planes.  Values stay below 2^256 between rounds (lazy reduction) and
 // are made canonical on the final store.
 #include <algorithm>
 #include <cstring>
@@ -27,6 +22,12 @@
 
 namespace zk {
 
+static fe to_fe(const host::Fr& a) {
+  fe r;
+  std::memcpy(r.w, a.v, 32);
+  return r;
+}
+
 NttPlan make_ntt_plan(int log_n) {
   NttPlan p;
   p.log_n = log_n;
@@ -34,15 +35,20 @@ NttPlan make_ntt_plan(int log_n) {
     p.npass = 0;
     return p;
   }
-  if (log_n <= 11) {
-    p.npass = 1;
-    p.bits[0] = log_n;
+  // Balanced passes of at most kNarrowMax bits; from 2^25, where four are
+  // needed, passes of 6 bits (the fewest products per bit) with what is left
+  // over in the last pass, which has no twists, and then the first: 2^26 as
+  // 6+6+6+8 takes 10.7 ms, as 7+7+6+6 12.2 ms (B200).
+  const int np = (log_n + kNarrowMax - 1) / kNarrowMax;
+  p.npass = np;
+  if (np == NTT_MAX_PASS) {
+    const int last = std::min(log_n - 18, kNarrowMax);
+    p.bits[0] = log_n - 12 - last;
+    p.bits[1] = p.bits[2] = 6;
+    p.bits[3] = last;
     return p;
   }
-  int np = (log_n + 8) / 9;  // passes of at most 9 bits
-  if (np < 2) np = 2;
-  p.npass = np;
-  int base = log_n / np, extra = log_n % np;
+  const int base = log_n / np, extra = log_n % np;
   for (int t = 0; t < np; t++) p.bits[t] = base + (t < extra ? 1 : 0);
   return p;
 }
@@ -100,15 +106,15 @@ __global__ void __launch_bounds__(256, 2) ntt_batch_kernel(const BatchPass* pass
     const BatchPass& bp = passes[s_k];
     const uint64_t tile = s_w - bp.tile_base;
     switch (bp.B) {
-      case 3: ntt_pass_tile<3, true>(bp.p, tile, smem); break;
-      case 4: ntt_pass_tile<4, true>(bp.p, tile, smem); break;
-      case 5: ntt_pass_tile<5, true>(bp.p, tile, smem); break;
-      case 6: ntt_pass_tile<6, true>(bp.p, tile, smem); break;
-      case 7: ntt_pass_tile<7, true>(bp.p, tile, smem); break;
-      case 8: ntt_pass_tile<8, true>(bp.p, tile, smem); break;
-      case 9: ntt_pass_tile<9, true>(bp.p, tile, smem); break;
-      case 10: ntt_pass_tile<10, true>(bp.p, tile, smem); break;
-      case 11: ntt_pass_tile<11, true>(bp.p, tile, smem); break;
+      case 3: ntt_pass_tile<3, true>(bp.p, nullptr, tile, smem); break;
+      case 4: ntt_pass_tile<4, true>(bp.p, nullptr, tile, smem); break;
+      case 5: ntt_pass_tile<5, true>(bp.p, nullptr, tile, smem); break;
+      case 6: ntt_pass_tile<6, true>(bp.p, nullptr, tile, smem); break;
+      case 7: ntt_pass_tile<7, true>(bp.p, nullptr, tile, smem); break;
+      case 8: ntt_pass_tile<8, true>(bp.p, nullptr, tile, smem); break;
+      case 9: ntt_pass_tile<9, true>(bp.p, nullptr, tile, smem); break;
+      case 10: ntt_pass_tile<10, true>(bp.p, nullptr, tile, smem); break;
+      case 11: ntt_pass_tile<11, true>(bp.p, nullptr, tile, smem); break;
       default: break;
     }
     __threadfence();  // every thread publishes its own stores before the tile is counted
@@ -165,8 +171,47 @@ __global__ void pow_seq_kernel(fe* out, fe base, uint64_t count, uint64_t step) 
   st_fe(out + e, r);
 }
 
-// twist[k * J + j] = lo[(k j) & mask] * hi[(k j) >> shift]
-__global__ void twist_table_kernel(fe* out, const fe* lo, const fe* hi, uint32_t shift, uint32_t log_J, uint64_t total) {
+// 2^e mod r for the table forms of mul_w4 (2^(64 k + 96)) and mul_w2
+// (2^(128 k + 160)): the product of a Montgomery w 2^256 with it is w 2^e
+struct TableScale {
+  fe w4[4], w2[2];
+};
+static host::Fr pow2(int e) {  // the integer 2^e mod r, e < 512
+  host::Fr x{{1, 0, 0, 0}};
+  for (int i = 0; i < e; i++) x = host::add(x, x);
+  return x;
+}
+static TableScale table_scale() {
+  static const TableScale s = {{to_fe(pow2(96)), to_fe(pow2(160)), to_fe(pow2(224)), to_fe(pow2(288))},
+                               {to_fe(pow2(160)), to_fe(pow2(288))}};
+  return s;
+}
+
+// Roots of a narrow pass: entry e, form k (layout in ntt_tile.cuh); special:
+// the three constants of the 8-point DFT
+struct Special {
+  fe v[3];
+};
+__global__ void roots_w4_kernel(fe* out, fe wm, const Special special, const TableScale sc, int B) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int e = (int)(i >> 2);
+  if (e >= tw_entries(B)) return;
+  uint32_t v[8];
+  if (e < 3) {
+    cpy(v, special.v[e].w);
+  } else {
+    int lo = B - 3, at = 3;
+    while (e >= at + (7 << lo)) at += 7 << lo, lo -= 3;
+    const uint32_t f = (uint32_t)((e - at) >> lo) + 1, low = (uint32_t)(e - at) & ((1u << lo) - 1u);
+    pow_u64<P_r>(v, wm.w, (uint64_t)(f * low) << (B - 3 - lo));
+  }
+  mul<P_r>(v, v, sc.w4[i & 3].w);
+  st_fe(out + i, v);
+}
+
+// twist[k * J + j] = lo[(k j) & mask] * hi[(k j) >> shift], both forms of mul_w2
+__global__ void twist_table_kernel(fe* out, const fe* lo, const fe* hi, uint32_t shift, uint32_t log_J, uint64_t total,
+                                   const TableScale sc) {
   const uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const uint64_t k = idx >> log_J, j = idx & ((1ull << log_J) - 1);
@@ -174,8 +219,12 @@ __global__ void twist_table_kernel(fe* out, const fe* lo, const fe* hi, uint32_t
   uint32_t a[8], b[8];
   ld_fe_nc(a, lo + (e & ((1ull << shift) - 1)));
   ld_fe_nc(b, hi + (e >> shift));
-  mul<P_r>(a, a, b);
-  st_fe(out + idx, a);
+  mul_lazy<P_r>(a, a, b);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    mul<P_r>(b, a, sc.w2[k].w);
+    st_fe(out + 2 * idx + k, b);
+  }
 }
 
 // dst[i * dst_stride] = src[i] * c^i (powc may be null: plain strided copy)
@@ -198,11 +247,6 @@ __global__ void scale_copy_kernel(fe* dst, const fe* src, uint64_t n, uint64_t d
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-static fe to_fe(const host::Fr& a) {
-  fe r;
-  std::memcpy(r.w, a.v, 32);
-  return r;
-}
 
 static cudaError_t pow_two_level(fe** lo, fe** hi, uint32_t* shift, const host::Fr& base, int log_count,
                                  cudaStream_t s, bool pooled) {
@@ -254,6 +298,25 @@ void pow_tables_free(PowTables* t, cudaStream_t s) {
   t->lo = t->hi = nullptr;
 }
 
+// elements of a pass's root table, and its launch
+static uint64_t inner_elems(int B) { return B <= kNarrowMax ? 4ull * tw_entries(B) : 1ull << (B - 1); }
+static void fill_inner(fe* out, DftConsts* dft, const host::Fr& wm, int B, cudaStream_t s) {
+  const unsigned count = (unsigned)inner_elems(B), grid = (count + 255) / 256;
+  if (B > kNarrowMax) {
+    pow_seq_kernel<<<grid, 256, 0, s>>>(out, to_fe(wm), count, 1);
+    return;
+  }
+  const host::Fr w8 = host::pow_2k(wm, (unsigned)(B - 3)), w4 = host::mul(w8, w8), w83 = host::mul(w4, w8);
+  static const host::Fr half = host::inv(host::from_u64(2));
+  Special sp;
+  const host::Fr c[3] = {w4, host::mul(half, host::add(w8, w83)), host::mul(half, host::sub(w8, w83))};
+  for (int k = 0; k < 3; k++) {
+    sp.v[k] = to_fe(c[k]);
+    for (int j = 0; j < 8; j++) std::memcpy(dft->w[k] + 8 * j, host::mul(c[k], pow2(32 * j + 64)).v, 32);
+  }
+  roots_w4_kernel<<<grid, 256, 0, s>>>(out, to_fe(wm), sp, table_scale(), B);
+}
+
 static cudaError_t build_tables(NttTables* t, cudaStream_t s) {
   const NttPlan& p = t->plan;
   int done_bits = 0;
@@ -264,21 +327,21 @@ static cudaError_t build_tables(NttTables* t, cudaStream_t s) {
     // this pass works on the sub-problem of size m*J whose root is w^(n / (m J))
     const host::Fr wMJ = host::pow_2k(t->omega, (unsigned)done_bits);
     const host::Fr wm = host::pow_2k(wMJ, (unsigned)log_J);
-    const uint64_t half = b >= 1 ? (1ull << (b - 1)) : 1;
-    e = cudaMalloc((void**)&t->inner[k], half * sizeof(fe));
+    e = cudaMalloc((void**)&t->inner[k], inner_elems(b) * sizeof(fe));
     if (e != cudaSuccess) return e;
-    t->bytes += half * sizeof(fe);
-    pow_seq_kernel<<<(unsigned)((half + 255) / 256), 256, 0, s>>>(t->inner[k], to_fe(wm), half, 1);
+    t->bytes += inner_elems(b) * sizeof(fe);
+    fill_inner(t->inner[k], &t->dft[k], wm, b, s);
     if (k + 1 < p.npass) {
       const uint64_t total = 1ull << (b + log_J);
-      e = cudaMalloc((void**)&t->twist[k], total * sizeof(fe));
+      e = cudaMalloc((void**)&t->twist[k], 2 * total * sizeof(fe));
       if (e != cudaSuccess) return e;
-      t->bytes += total * sizeof(fe);
+      t->bytes += 2 * total * sizeof(fe);
       fe *lo = nullptr, *hi = nullptr;
       uint32_t sh = 0;
       e = pow_two_level(&lo, &hi, &sh, wMJ, b + log_J, s, true);
       if (e != cudaSuccess) return e;
-      twist_table_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(t->twist[k], lo, hi, sh, (uint32_t)log_J, total);
+      twist_table_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(t->twist[k], lo, hi, sh, (uint32_t)log_J, total,
+                                                                          table_scale());
       cudaFreeAsync(lo, s);
       cudaFreeAsync(hi, s);
     }
@@ -296,11 +359,11 @@ size_t ntt_tables_elems(int log_n) {
   for (int k = 0; k < p.npass; k++) {
     const int b = p.bits[k];
     const int log_J = p.log_n - done - b;
-    total += b >= 1 ? (1ull << (b - 1)) : 1;
+    total += inner_elems(b);
     if (k + 1 < p.npass) {
       const int lc = b + log_J;
       const int sh = (lc + 1) / 2;
-      total += (1ull << lc) + (1ull << sh) + (1ull << (lc > sh ? lc - sh : 0));
+      total += (2ull << lc) + (1ull << sh) + (1ull << (lc > sh ? lc - sh : 0));
     }
     done += b;
   }
@@ -320,10 +383,9 @@ cudaError_t ntt_tables_fill(NttTables* t, const host::Fr& omega, int log_n, fe* 
     const int log_J = p.log_n - done - b;
     const host::Fr wMJ = host::pow_2k(omega, (unsigned)done);
     const host::Fr wm = host::pow_2k(wMJ, (unsigned)log_J);
-    const uint64_t half = b >= 1 ? (1ull << (b - 1)) : 1;
     t->inner[k] = cur;
-    cur += half;
-    pow_seq_kernel<<<(unsigned)((half + 255) / 256), 256, 0, s>>>(t->inner[k], to_fe(wm), half, 1);
+    cur += inner_elems(b);
+    fill_inner(t->inner[k], &t->dft[k], wm, b, s);
     if (k + 1 < p.npass) {
       const int lc = b + log_J;
       const uint32_t sh = (uint32_t)((lc + 1) / 2);
@@ -331,11 +393,11 @@ cudaError_t ntt_tables_fill(NttTables* t, const host::Fr& omega, int log_n, fe* 
       fe* lo = cur;
       fe* hi = cur + nlo;
       t->twist[k] = cur + nlo + nhi;
-      cur += nlo + nhi + total;
+      cur += nlo + nhi + 2 * total;
       pow_seq_kernel<<<(unsigned)((nlo + 255) / 256), 256, 0, s>>>(lo, to_fe(wMJ), nlo, 1);
       pow_seq_kernel<<<(unsigned)((nhi + 255) / 256), 256, 0, s>>>(hi, to_fe(host::pow_2k(wMJ, sh)), nhi, 1);
       twist_table_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(t->twist[k], lo, hi, sh, (uint32_t)log_J,
-                                                                          total);
+                                                                          total, table_scale());
     } else {
       t->twist[k] = nullptr;
     }
@@ -378,26 +440,26 @@ void ntt_tables_release(NttTables* t) {
   t->bytes = 0;
 }
 
-static cudaError_t dispatch_pass(int B, const PassParams& pp, uint64_t ncta, cudaStream_t s) {
+static uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* out,
+                                bool batch);
+
+static cudaError_t dispatch_pass(int B, const PassParams& pp, const DftConsts& dft, uint64_t ncta, cudaStream_t s) {
   switch (B) {
-    case 3: return launch_pass<3>(pp, ncta, s);
-    case 4: return launch_pass<4>(pp, ncta, s);
-    case 5: return launch_pass<5>(pp, ncta, s);
-    case 6: return launch_pass<6>(pp, ncta, s);
-    case 7: case 8: case 9: case 10: case 11: return launch_pass_wide(B, pp, ncta, s);
+    case 3: return launch_pass<3>(pp, dft, ncta, s);
+    case 4: return launch_pass<4>(pp, dft, ncta, s);
+    case 5: return launch_pass<5>(pp, dft, ncta, s);
+    case 6: return launch_pass<6>(pp, dft, ncta, s);
+    case 7: case 8: case 9: case 10: case 11: return launch_pass_wide(B, pp, dft, ncta, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
-uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const PowTables* pre, const host::Fr* post,
-                         PassParams* out) {
-  NttFuse f;
-  f.pre = pre;
-  f.post = post;
-  return ntt_pass_params(t, k, d_a, d_tmp, f, out);
+uint64_t ntt_batch_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* out) {
+  return ntt_pass_params(t, k, d_a, d_tmp, f, out, true);
 }
 
-uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* out) {
+static uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* out,
+                                bool batch) {
   const PowTables* pre = f.pre;
   const host::Fr* post = f.post;
   const NttPlan& p = t.plan;
@@ -416,6 +478,7 @@ uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const Nt
   pp.log_m1 = p.npass > 1 ? (uint32_t)p.bits[0] : 0u;
   pp.nprev = final_pass ? (uint32_t)k : 0u;
   for (int j = 0; j < k && j < NTT_MAX_PASS; j++) pp.prev_bits[j] = (uint32_t)p.bits[j];
+  pp.is_first = k == 0 ? 1u : 0u;
   pp.is_final = final_pass ? 1u : 0u;
   if (k == 0 && pre) {
     pp.pre_lo = pre->lo;
@@ -451,7 +514,12 @@ uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const Nt
     pp.out = d_a;
   }
   if (k == 0 && f.src) pp.in = f.src;  // out of place: the first pass reads the source
-  const uint32_t Gmax = b >= 11 ? 1u : (1u << (11 - b));
+  // Tiles of 2^10 elements (128 threads), two to a block (2^24 as 8+8+8: 2780
+  // us with one tile of 2^11, 2685 with two of 2^10); a pass with too few of
+  // them to give every SM a block takes one to a block (2^16: 47 -> 35 us).
+  // Passes wider than kNarrowMax keep tiles of 2^11.
+  const int tile_log = b > kNarrowMax ? 11 : 10;
+  const uint32_t Gmax = b >= tile_log ? 1u : (1u << (tile_log - b));
   uint64_t groups_dim;
   if (!final_pass) {
     groups_dim = 1ull << pp.log_J;  // columns per outer block
@@ -461,8 +529,10 @@ uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const Nt
     groups_dim = 1ull << p.bits[0];  // consecutive k_1 digits
   }
   pp.G = (uint32_t)std::min<uint64_t>(Gmax, groups_dim);
+  const uint64_t tiles = (1ull << (L - b)) / pp.G;
+  pp.ntile = b <= kNarrowMax && pp.G << (b - 3) == 128 && tiles >= (batch ? 2 : 256) ? 2u : 1u;
   *out = pp;
-  return (1ull << (L - b)) / pp.G;
+  return tiles / pp.ntile;
 }
 
 cudaError_t ntt_run(const NttTables& t, fe* d_a, fe* d_tmp, const PowTables* pre, const host::Fr* post, cudaStream_t s) {
@@ -490,17 +560,19 @@ cudaError_t ntt_run(const NttTables& t, fe* d_a, fe* d_tmp, const NttFuse& f, cu
   for (int k = 0; k < p.npass; k++) {
     const int b = p.bits[k];
     PassParams pp;
-    const uint64_t ncta = ntt_pass_params(t, k, d_a, d_tmp, f, &pp);
+    const uint64_t ncta = ntt_pass_params(t, k, d_a, d_tmp, f, &pp, false);
     const double nel = (double)(1ull << L);
     // algorithmic work: radix-2 convention (n/2) * b products; bytes: read + write (+ twist table)
-    ProfScope prof(names[b], s, nel / 2 * b, nel * 32.0 * (pp.is_final ? 2 : 3));
-    cudaError_t e = dispatch_pass(b, pp, ncta, s);
+    ProfScope prof(names[b], s, nel / 2 * b, nel * 32.0 * (pp.is_final ? 2 : 4));
+    cudaError_t e = dispatch_pass(b, pp, t.dft[k], ncta, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
-static size_t batch_smem_bytes() { return (size_t)8 * 2048 * 4 + (size_t)1024 * 32; }  // B <= 11
+static size_t batch_smem_bytes() {
+  return (size_t)8 * 2048 * 4 + std::max(tw_smem_bytes(kNarrowMax), tw_smem_bytes(11));
+}
 
 int ntt_batch_grid(int device) {
   static int cached[64] = {0};

@@ -40,13 +40,20 @@ bool ntt_plan_valid(const NttPlan& p);
 // The plan the autotuner chose for (device, log_n), else make_ntt_plan.
 NttPlan tuned_ntt_plan(int device, int log_n);
 
-// Device tables for one (omega, log_n): per pass the inner roots
-// w_m^e (e < m/2) and, for non-final passes, the twist table [k * J + j].
+// The three constants of the 8-point DFT, each in the form of mul_w8: a kernel
+// parameter of the narrow passes, so that the products read them as operands.
+struct DftConsts {
+  uint32_t w[3][64];
+};
+
+// Device tables for one (omega, log_n): per pass the roots its rounds use and,
+// for non-final passes, the twist table [k * J + j] (two entries of mul_w2).
 struct NttTables {
   NttPlan plan;
   host::Fr omega;
   fe* inner[NTT_MAX_PASS] = {nullptr, nullptr, nullptr, nullptr};
   fe* twist[NTT_MAX_PASS] = {nullptr, nullptr, nullptr, nullptr};
+  DftConsts dft[NTT_MAX_PASS];  // narrow passes
   size_t bytes = 0;
 };
 
@@ -96,8 +103,8 @@ void table_cache_clear(int device);
 struct PassParams {
   const fe* in;
   fe* out;
-  const fe* inner;   // w_m^e, e < m/2
-  const fe* twist;   // [k * J + j], non-final passes
+  const fe* inner;   // the pass's roots (ntt_tile.cuh)
+  const fe* twist;   // w^(k j) at [k * J + j] as the two entries of mul_w2, non-final passes
   const fe* pre_lo;  // coset powers (first pass), or null
   const fe* pre_hi;
   uint32_t pre_shift;
@@ -106,7 +113,9 @@ struct PassParams {
   uint32_t log_m1;
   uint32_t nprev;
   uint32_t prev_bits[NTT_MAX_PASS];
-  uint32_t G;
+  uint32_t G;      // columns per tile
+  uint32_t ntile;  // tiles per block: 1 or 2
+  uint32_t is_first;
   uint32_t is_final;
   uint32_t has_post;
   fe post;
@@ -127,10 +136,9 @@ struct NttFuse {
   const fe* src = nullptr;              // read the input from here instead of d_a (d_a gets the result)
 };
 
-// Pass k of the plan in `t` over d_a / d_tmp; returns its CTA count.
-uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const PowTables* pre, const host::Fr* post,
-                         PassParams* pp);
-uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* pp);
+// Pass k of the plan in `t` over d_a / d_tmp as the batch kernel runs it;
+// returns its tile count.
+uint64_t ntt_batch_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* pp);
 
 // One pass of one transform inside a batch launch.
 struct BatchPass {

@@ -7,7 +7,7 @@
 // data (device memory, transformed in place); the scratch the multi-pass NTT
 // needs — the ping-pong buffer and the root / twist tables — lives in the
 // file-scope device array below, sized for transforms of up to
-// 2^ZKGPU_STATIC_NTT_MAX_LOG elements (about 16.8 MB, held by every GPU that
+// 2^ZKGPU_STATIC_NTT_MAX_LOG elements (about 25.5 MB, held by every GPU that
 // loads the library until the process exits).
 //
 // Sharing rules: every call on a device uses the same array and leaves its
@@ -30,7 +30,7 @@ namespace {
 
 constexpr int kMaxLog = ZKGPU_STATIC_NTT_MAX_LOG;
 constexpr size_t kBuf = (size_t)1 << kMaxLog;                        // ping-pong buffer
-constexpr size_t kTables = ((size_t)1 << kMaxLog) + (1u << 10) + (1u << 12);  // twist + pow + inner tables
+constexpr size_t kTables = ((size_t)2 << kMaxLog) + (2u << 12) + (1u << 12);  // twist + pow + inner tables
 constexpr size_t kScratchElems = kBuf + kTables;
 
 static __device__ __align__(256) zk::fe g_static_ntt_scratch[kScratchElems];

@@ -2,13 +2,8 @@
 // DIF columns with the twist or the final digit-reversed store), shared by
 // the per-pass kernels, the persistent batch kernel and their launchers.
 //
-// The launchers of the wide passes (B = 7..11) live in their own translation
-// unit, ntt_pass_wide.cu, which compiles in parallel with ntt.cu and can take
-// its own ptxas options.  With inlined products, the three register rounds of
-// a wide pass made ptxas -O3 spill about 1.3 KB per thread at 128 registers
-// and -O1 was faster; with the out-of-line products below, -O3 spills
-// 200-380 B and runs the radix-2^8 and 2^9 plans as fast as or faster than
-// -O1, so every pass is built at -O3.
+// The launchers of the passes B = 7..11 live in their own translation unit,
+// ntt_pass_wide.cu, which compiles in parallel with ntt.cu.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -22,7 +17,15 @@ using P_r = FrP;
 // ---------------------------------------------------------------------------
 // device helpers
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t swz(uint32_t e) { return e ^ ((e >> 3) & 31u); }
+// Shared-memory word of element i of column g.  Columns are adjacent, so a
+// warp whose lanes hold 32 columns reads and writes 32 consecutive words (and
+// reads one twiddle for all lanes).  With fewer columns the lanes differ in
+// low bits of the thread's column position q, which are element bits 0.. in
+// all rounds but the last and bits 3.. there; the XOR puts both on distinct
+// banks.
+__device__ __forceinline__ uint32_t word_of(uint32_t i, uint32_t g, uint32_t log_G) {
+  return ((i << log_G) + g) ^ (((i >> 3) << log_G) & 31u);
+}
 
 template <int LO>
 __device__ __forceinline__ uint32_t ins3(uint32_t q, uint32_t r) {
@@ -33,44 +36,205 @@ __device__ __forceinline__ void ld_smem_fe(uint32_t r[8], const uint32_t* plane0
 #pragma unroll
   for (int k = 0; k < 8; k++) r[k] = plane0[k * plane_stride + a];
 }
-// a twiddle: its low and high 16 bytes in two planes
-__device__ __forceinline__ void ld_smem_tw(uint32_t r[8], const uint4* plane0, uint32_t plane_stride, uint32_t a) {
-  const uint4 x = plane0[a], y = plane0[plane_stride + a];
-  r[0] = x.x; r[1] = x.y; r[2] = x.z; r[3] = x.w;
-  r[4] = y.x; r[5] = y.y; r[6] = y.z; r[7] = y.w;
-}
 __device__ __forceinline__ void st_smem_fe(uint32_t* plane0, uint32_t plane_stride, uint32_t a, const uint32_t r[8]) {
 #pragma unroll
   for (int k = 0; k < 8; k++) plane0[k * plane_stride + a] = r[k];
 }
 
-// The products of a pass.  With ZK_NTT_CALL_PRODUCT (the default) the
-// butterfly products are calls of one out-of-line product, its operands and
-// result passed by value so that they stay in registers: a radix-8 round then
-// runs one product's code from the instruction cache instead of a fresh
-// inlined copy per butterfly, whose cache misses held the fully unrolled
-// rounds back.  The products outside the rounds (the twist, the coset
-// pre-multiply, the output scale) are calls only in passes of width
-// B >= ZK_NTT_CALL_EDGE_MIN_B: inlined they overlap their loads and run
-// faster in the narrow passes, while in the wide ones the shorter code and
-// lower register pressure win.
-#ifndef ZK_NTT_CALL_PRODUCT
-#define ZK_NTT_CALL_PRODUCT 1
-#endif
-#ifndef ZK_NTT_CALL_EDGE_MIN_B
-#define ZK_NTT_CALL_EDGE_MIN_B 7
-#endif
-template <bool CALL = (ZK_NTT_CALL_PRODUCT != 0)>
-__device__ __forceinline__ void ntt_mul(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) {
-#if ZK_NTT_CALL_PRODUCT
-  if constexpr (!CALL) {
-    mul_lazy<P_r>(r, a, b);
+// ---------------------------------------------------------------------------
+// Rounds of the passes of up to 2^8 points.
+//
+// A round runs 8-point DFTs on the elements a thread holds, then multiplies
+// output f of the DFT by the round's twiddle w^(f low).  What bounds a pass is
+// its field products, so the round is arranged for few and cheap ones:
+//  * the DFT takes four products instead of five.  With t_i = x_i - x_(i+4)
+//    and w = w_8, the odd outputs need w t_1 + w^3 t_3 and
+//    i (w t_1 - w^3 t_3) = w^3 t_1 + w t_3, which are E_1 + E_2 and E_1 - E_2
+//    for E_1 = (w + w^3) / 2 (t_1 + t_3), E_2 = (w - w^3) / 2 (t_1 - t_3);
+//  * eight twiddle-free stages and seven products by f, low instead of twelve
+//    butterflies with a product each: 11 products per 8 elements and 3 bits;
+//  * every multiplicand is known beforehand, so each product is a mul_w4 over
+//    a table in shared memory (about 390 cycles against mul_lazy's 555).
+//  * the DFT's three constants are the same for the whole pass: the per-pass
+//    kernels take them as kernel parameters in the form of mul_w8 (350 cycles,
+//    no loads).
+// Forward NTT of 2^24 (8+8+8) on B200: 4320 us with a mul_lazy in each radix-2
+// butterfly, 2685 us in this form; the multiply pipe is then busy for 73 % of a
+// pass (ncu, sm__pipe_fmaheavy_cycles_active).  The per-pass kernels inline every
+// product; the batch kernel, which holds all pass widths, calls one out of
+// line, as its dozens of copies would miss the instruction cache.
+//
+// Ranges, with 1 for p (1 + 2^-29), the bound of a mul_w4 result: inputs <= 1;
+// a difference gets the multiple of p that keeps it positive, and a sum that
+// would leave [0, 5.29] (2^256 = 5.29 p) loses 2p first if it is at least 2p.
+// ---------------------------------------------------------------------------
+constexpr int kNarrowMax = 8;  // widest pass of this form: its tables take 32 KiB of shared memory
+
+// twiddle table of a pass: I = w_4, (w_8 + w_8^3) / 2, (w_8 - w_8^3) / 2, then
+// per round with LO > 0 the roots w_(8 2^LO)^(f low) at [(f - 1) 2^LO + low]
+__host__ __device__ constexpr int tw_entries(int B) {
+  int n = 3;
+  for (int lo = B - 3; lo > 0; lo -= 3) n += 7 << lo;
+  return n;
+}
+__host__ __device__ constexpr int tw_offset(int B, int LO) {
+  int n = 3;
+  for (int lo = B - 3; lo > LO; lo -= 3) n += 7 << lo;
+  return n;
+}
+
+// shared memory of a pass's root table
+__host__ __device__ constexpr size_t tw_smem_bytes(int B) {
+  return B <= kNarrowMax ? (size_t)tw_entries(B) * 128 : (size_t)16 << B;
+}
+
+__device__ __forceinline__ void lds_v4(uint32_t v[4], uint32_t addr) {
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
+}
+struct SmemW4 {  // entry at `addr` of a table stored as eight planes of 16 bytes
+  uint32_t addr, plane;
+  __device__ __forceinline__ void operator()(int k, uint32_t v[8]) const {
+    lds_v4(v, addr + 2 * k * plane);
+    lds_v4(v + 4, addr + (2 * k + 1) * plane);
+  }
+};
+template <class P>
+__device__ __noinline__ Fe8 mul_w4_call(const Fe8 a, uint32_t addr, uint32_t plane) {
+  Fe8 r;
+  mul_w4<P>(r.w, a.w, SmemW4{addr, plane});
+  return r;
+}
+// r = a times table entry e
+template <int B, bool INLINE = false>
+__device__ __forceinline__ void tw_mul(uint32_t r[8], const uint32_t a[8], uint32_t tab, uint32_t e) {
+  if constexpr (INLINE) {
+    mul_w4<P_r>(r, a, SmemW4{tab + 16 * e, 16 * tw_entries(B)});
     return;
   }
-  mul_out<P_r>(r, a, b);
-#else
-  mul_lazy<P_r>(r, a, b);
-#endif
+  Fe8 av;
+#pragma unroll
+  for (int k = 0; k < 8; k++) av.w[k] = a[k];
+  const Fe8 rv = mul_w4_call<P_r>(av, tab + 16 * e, 16 * tw_entries(B));
+#pragma unroll
+  for (int k = 0; k < 8; k++) r[k] = rv.w[k];
+}
+
+struct ParamC8 {
+  const DftConsts& d;
+  __device__ __forceinline__ void mul(uint32_t r[8], const uint32_t a[8], int e) const {
+    const uint32_t* t = d.w[e];
+    mul_w8<P_r>(r, a, [t](int k, uint32_t v[8]) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) v[j] = t[8 * k + j];
+    });
+  }
+};
+template <int B>
+struct SmemC4 {
+  uint32_t tab;
+  __device__ __forceinline__ void mul(uint32_t r[8], const uint32_t a[8], int e) const { tw_mul<B>(r, a, tab, e); }
+};
+// 8-point DFT in place, position r <- output rev3(r); inputs <= 1, outputs <= 5
+template <class C>
+__device__ __forceinline__ void dft8(uint32_t x[8][8], const C& c) {
+  uint32_t s0[8], s1[8], s2[8], s3[8], u[8], v[8], e[8], f[8];
+  // products first: their operands die here
+  add_raw(s1, x[1], x[5]);
+  add_raw(s3, x[3], x[7]);
+  add_raw(u, x[1], x[3]);
+  add_raw(e, x[5], x[7]);
+  sub_off<P_r, 3>(u, u, e);       // t1 + t3, 1 .. 5
+  add_raw(v, x[1], x[7]);
+  add_raw(e, x[3], x[5]);
+  sub_off<P_r, 3>(v, v, e);       // t1 - t3, 1 .. 5
+  c.mul(u, u, 1);        // E1
+  c.mul(v, v, 2);        // E2
+  sub_off<P_r, 2>(e, x[2], x[6]);
+  c.mul(e, e, 0);        // i t2
+  add_raw(s0, x[0], x[4]);
+  add_raw(s2, x[2], x[6]);
+  // odd outputs
+  add_raw(x[5], x[4], e);
+  sub_off<P_r, 3>(x[7], x[0], x[5]);  // t0 - i t2, 1 .. 4
+  cond_sub<P_r, 2>(x[7]);
+  sub_off<P_r, 2>(x[0], x[0], x[4]);
+  add_raw(x[0], x[0], e);             // t0 + i t2, 1 .. 4
+  cond_sub<P_r, 2>(x[0]);
+  add_raw(e, u, v);
+  sub_off<P_r, 2>(u, u, v);           // E1 - E2 + 2, 1 .. 3
+  add_raw(x[4], x[0], e);             // 0 .. 4
+  sub_off<P_r, 3>(x[5], x[0], e);     // 1 .. 5
+  add_raw(x[6], x[7], u);             // 1 .. 5
+  sub_off<P_r, 4>(x[7], x[7], u);     // 1 .. 5: E2 - E1 + 2 added
+  // even outputs
+  add_raw(e, s0, s2);
+  cond_sub<P_r, 2>(e);
+  add_raw(f, s1, s3);
+  cond_sub<P_r, 2>(f);
+  add_raw(x[0], e, f);                // 0 .. 4
+  sub_off<P_r, 3>(x[1], e, f);        // 1 .. 5
+  sub_off<P_r, 3>(s0, s0, s2);        // 1 .. 5
+  cond_sub<P_r, 2>(s0);               // 0 .. 3
+  sub_off<P_r, 3>(s1, s1, s3);        // 1 .. 5
+  c.mul(s1, s1, 0);
+  add_raw(x[2], s0, s1);              // 0 .. 4
+  sub_off<P_r, 2>(x[3], s0, s1);      // 1 .. 5
+}
+// 4-point DFT of x[0..3], position r <- output rev2(r); outputs <= 5
+template <class C>
+__device__ __forceinline__ void dft4(uint32_t x[4][8], const C& c) {
+  uint32_t s0[8], s1[8], d[8];
+  sub_off<P_r, 2>(d, x[1], x[3]);
+  c.mul(d, d, 0);
+  add_raw(s0, x[0], x[2]);
+  add_raw(s1, x[1], x[3]);
+  sub_off<P_r, 2>(x[0], x[0], x[2]);
+  add_raw(x[2], x[0], d);             // 1 .. 4
+  sub_off<P_r, 2>(x[3], x[0], d);     // 2 .. 5
+  add_raw(x[0], s0, s1);
+  sub_off<P_r, 3>(x[1], s0, s1);      // 1 .. 5
+}
+
+template <int B, int LO, int HI, bool INLINE, class C>
+__device__ __forceinline__ void narrow_round(uint32_t x[8][8], uint32_t q, uint32_t tab, const C& c) {
+  if constexpr (HI - LO == 3) {
+    dft8(x, c);
+  } else if constexpr (HI - LO == 2) {
+    dft4(x, c);
+    dft4(x + 4, c);
+  } else {
+#pragma unroll
+    for (int r = 0; r < 8; r += 2) {
+      uint32_t t[8];
+      sub_off<P_r, 2>(t, x[r], x[r + 1]);
+      add_raw(x[r], x[r], x[r + 1]);
+      cpy(x[r + 1], t);
+    }
+  }
+  if constexpr (LO > 0) {
+    static_assert(HI - LO == 3, "only the last round has fewer than three bits");
+    const uint32_t low = q & ((1u << LO) - 1u);
+    cond_sub<P_r, 2>(x[0]);
+    cond_sub<P_r, 1>(x[0]);
+#pragma unroll
+    for (int r = 1; r < 8; r++) {
+      const uint32_t f = (uint32_t)((r & 1) << 2 | (r & 2) | r >> 2);
+      tw_mul<B, INLINE>(x[r], x[r], tab, tw_offset(B, LO) + ((f - 1) << LO) + low);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Rounds of the wider passes (B = 9..11), which only plans asked for by name
+// or by the autotuner use: their root tables would not leave room for two
+// blocks per SM in the form above.  Radix-2 butterflies on values below 2p,
+// each with a Montgomery product by a root w_m^e, e < m / 2.
+// ---------------------------------------------------------------------------
+// a twiddle: its low and high 16 bytes in two planes
+__device__ __forceinline__ void ld_smem_tw(uint32_t r[8], const uint4* plane0, uint32_t plane_stride, uint32_t a) {
+  const uint4 x = plane0[a], y = plane0[plane_stride + a];
+  r[0] = x.x; r[1] = x.y; r[2] = x.z; r[3] = x.w;
+  r[4] = y.x; r[5] = y.y; r[6] = y.z; r[7] = y.w;
 }
 // One round: registers hold i(r) = ins3<LO>(q, r); perform the DIF stages
 // with butterfly bits HI-1 .. LO.  tws: inner roots w_m^e (e < m/2), 2 planes.
@@ -96,76 +260,144 @@ __device__ __forceinline__ void ntt_round(uint32_t x[8][8], uint32_t q, const ui
         } else {
           uint32_t w[8];
           ld_smem_tw(w, tws, HALF, e);
-          ntt_mul<true>(x[r2], t, w);
+          mul_out<P_r>(x[r2], t, w);
         }
       } else {
         const uint32_t e = ((q & ((1u << LO) - 1u)) | ((uint32_t)(r & ((1 << rb) - 1)) << LO)) << (B - 1 - b);
         uint32_t w[8];
         ld_smem_tw(w, tws, HALF, e);
-        ntt_mul<true>(x[r2], t, w);
+        mul_out<P_r>(x[r2], t, w);
       }
     }
   }
 }
 
-template <int B, int LO_CUR, int LO_NEXT>
-__device__ __forceinline__ void ntt_exchange(uint32_t x[8][8], uint32_t q, uint32_t gbase, uint32_t* sm,
-                                             uint32_t plane_stride, bool active) {
-  if (active) {
-#pragma unroll
-    for (int r = 0; r < 8; r++) st_smem_fe(sm, plane_stride, swz(gbase + ins3<LO_CUR>(q, r)), x[r]);
-  }
-  __syncthreads();
-  if (active) {
-#pragma unroll
-    for (int r = 0; r < 8; r++) ld_smem_fe(x[r], sm, plane_stride, swz(gbase + ins3<LO_NEXT>(q, r)));
-  }
-  __syncthreads();
+// A block runs up to two tiles that share its root table and nothing else, so
+// that each waits at its own barriers: with 256 threads at one barrier the
+// pass is in the same phase (loads, products, exchange) in half of an SM's
+// warps at a time, and its products overlap less with the rest.
+struct TilePos {
+  uint32_t q, g;  // position in the column, column
+  uint32_t log_G;
+  uint32_t t, nt;   // thread of the tile, its threads
+  uint32_t barrier, barrier_threads;
+  bool active;
+};
+// Barriers 1 and 2; barrier 0 stays with __syncthreads, which one tile's threads
+// may already wait at (the batch kernel's end of a work item) while the other's
+// still meet here: one barrier must not be met with two thread counts at once.
+__device__ __forceinline__ void tile_sync(const TilePos& pos) {
+  asm volatile("bar.sync %0, %1;" ::"r"(pos.barrier), "r"(pos.barrier_threads) : "memory");
 }
 
-template <int B, int HI>
-__device__ __forceinline__ void ntt_rounds(uint32_t x[8][8], uint32_t q, uint32_t gbase, uint32_t* sm,
-                                           uint32_t plane_stride, const uint4* tws, bool active) {
+template <int B, int LO_CUR, int LO_NEXT>
+__device__ __forceinline__ void ntt_exchange(uint32_t x[8][8], const TilePos& pos, uint32_t* sm,
+                                             uint32_t plane_stride) {
+  // q is made opaque so that the eight addresses are computed here again and
+  // not kept in registers through the round before (spills at 128 registers)
+  uint32_t q = pos.q;
+  asm volatile("" : "+r"(q));
+  if (pos.active) {
+#pragma unroll
+    for (int r = 0; r < 8; r++) st_smem_fe(sm, plane_stride, word_of(ins3<LO_CUR>(q, r), pos.g, pos.log_G), x[r]);
+  }
+  tile_sync(pos);
+  asm volatile("" : "+r"(q));
+  if (pos.active) {
+#pragma unroll
+    for (int r = 0; r < 8; r++) ld_smem_fe(x[r], sm, plane_stride, word_of(ins3<LO_NEXT>(q, r), pos.g, pos.log_G));
+  }
+  tile_sync(pos);
+}
+
+// The twists of a thread's eight outputs (64 B each) come through four slots
+// of the data area, free once the last exchange is over: cp.async fills them
+// while the last round computes, and refills each after its product, so the
+// products do not wait for the table (measured without: 2.6-3.3 stalled warps
+// per issue on it).  A thread reads only what it copied itself.
+__device__ __forceinline__ uint32_t twist_index(const PassParams& p, int B, uint32_t q, uint32_t col, int r) {
+  return (__brev(8 * q + r) >> (32 - B) << p.log_J) + col;
+}
+__device__ __forceinline__ void twist_fetch(const PassParams& p, int B, const TilePos& pos, uint32_t col, uint32_t sm,
+                                            int r) {
+  if (pos.active) {
+    const char* src = reinterpret_cast<const char*>(p.twist + 2 * (size_t)twist_index(p, B, pos.q, col, r));
+    const uint32_t dst = sm + 16 * (4 * (r & 3) * pos.nt + pos.t);
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * c * pos.nt), "l"(src + 16 * c)
+                   : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int B, int HI, bool BATCH>
+__device__ __forceinline__ void ntt_rounds(const PassParams& p, const DftConsts* dft, uint32_t x[8][8],
+                                           TilePos pos, uint32_t col,
+                                           uint32_t* sm, uint32_t plane_stride, const uint4* tws) {
   constexpr int LO = HI - 3 > 0 ? HI - 3 : 0;
-  ntt_round<B, LO, HI>(x, q, tws);
+  if constexpr (LO == 0) {
+    if (!p.is_final) {
+#pragma unroll
+      for (int r = 0; r < 4; r++) twist_fetch(p, B, pos, col, (uint32_t)__cvta_generic_to_shared(sm), r);
+    }
+  }
+  if constexpr (B <= kNarrowMax) {
+    const uint32_t tab = (uint32_t)__cvta_generic_to_shared(tws);
+    if constexpr (BATCH)
+      narrow_round<B, LO, HI, false>(x, pos.q, tab, SmemC4<B>{tab});
+    else
+      narrow_round<B, LO, HI, true>(x, pos.q, tab, ParamC8{*dft});
+  } else
+    ntt_round<B, LO, HI>(x, pos.q, tws);
   if constexpr (LO > 0) {
     constexpr int LO_N = LO - 3 > 0 ? LO - 3 : 0;
-    ntt_exchange<B, LO, LO_N>(x, q, gbase, sm, plane_stride, active);
-    ntt_rounds<B, LO>(x, q, gbase, sm, plane_stride, tws, active);
+    ntt_exchange<B, LO, LO_N>(x, pos, sm, plane_stride);
+    // what follows depends on the thread's position through this copy: the
+    // addresses of later phases are not computed ahead and kept (spills)
+    asm volatile("" : "+r"(pos.q), "+r"(col));
+    ntt_rounds<B, LO, BATCH>(p, dft, x, pos, col, sm, plane_stride, tws);
   }
 }
 
-
-#ifndef ZK_NTT_MIN_BLOCKS
-#define ZK_NTT_MIN_BLOCKS 2
-#endif
 
 // One CTA tile of one pass.  `tile` plays the role of the block index.  In
 // BATCH mode the CTA may be wider than the tile (G * T threads are active,
 // the rest only join the barriers) and data is read through L2 only, since
 // other CTAs of the same launch produced it.
 template <int B, bool BATCH>
-__device__ __forceinline__ void ntt_pass_tile(const PassParams& p, uint64_t tile, uint32_t* smem) {
+__device__ __forceinline__ void ntt_pass_tile(const PassParams& p, const DftConsts* dft, uint64_t tile,
+                                              uint32_t* smem) {
   constexpr uint32_t M = 1u << B;
   constexpr uint32_t T = M / 8;  // threads per column
   const uint32_t G = p.G;
   const uint32_t plane_stride = G * M;
-  uint4* tws = reinterpret_cast<uint4*>(smem + 8 * plane_stride);  // 32 G M bytes in
+  uint4* tws = reinterpret_cast<uint4*>(smem + 8 * plane_stride * p.ntile);  // 32 G M bytes per tile in
 
   const uint32_t tid = threadIdx.x;
-  const uint32_t g = tid / T, q = tid % T;
-  const bool active = !BATCH || g < G;
+  const uint32_t log_G = __ffs(G) - 1, log_nt = log_G + (B - 3);
+  const uint32_t sub = p.ntile > 1 ? tid >> log_nt : 0u;
+  const uint32_t t = tid - (sub << log_nt);
+  const uint32_t g = t & (G - 1), q = t >> log_G;
+  const bool active = !BATCH || (sub < p.ntile && q < T);
+  const TilePos pos{q, g, log_G, t, G * T, 1 + sub, p.ntile > 1 ? G * T : (blockDim.x + 31u) & ~31u, active};
 
-  for (uint32_t e = tid; e < M / 2; e += blockDim.x) {
-    uint32_t w[8];
-    ld_fe_nc(w, p.inner + e);
-    tws[e] = make_uint4(w[0], w[1], w[2], w[3]);
-    tws[M / 2 + e] = make_uint4(w[4], w[5], w[6], w[7]);
+  if constexpr (B <= kNarrowMax) {
+    constexpr uint32_t N = tw_entries(B);
+    const uint4* src = reinterpret_cast<const uint4*>(p.inner);
+    for (uint32_t e = tid; e < 8 * N; e += blockDim.x) tws[(e & 7) * N + (e >> 3)] = __ldg(src + e);
+  } else {
+    for (uint32_t e = tid; e < M / 2; e += blockDim.x) {
+      uint32_t w[8];
+      ld_fe_nc(w, p.inner + e);
+      tws[e] = make_uint4(w[0], w[1], w[2], w[3]);
+      tws[M / 2 + e] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
   }
 
   // element indices are < 2^28: 32-bit arithmetic, powers of two as shifts
-  const uint32_t t32 = (uint32_t)tile;
-  const uint32_t log_G = __ffs(G) - 1;
+  const uint32_t t32 = (uint32_t)tile * p.ntile + sub;
+  smem += 8 * plane_stride * sub;
   const uint32_t J = 1u << p.log_J;
   uint32_t o, col = 0, base, stride;
   if (!p.is_final) {
@@ -208,25 +440,38 @@ __device__ __forceinline__ void ntt_pass_tile(const PassParams& p, uint64_t tile
       uint32_t a[8], b[8];
       ld_fe_nc(a, p.pre_lo + (xi & mask));
       ld_fe_nc(b, p.pre_hi + (xi >> p.pre_shift));
-      ntt_mul<(B >= ZK_NTT_CALL_EDGE_MIN_B)>(a, a, b);
-      ntt_mul<(B >= ZK_NTT_CALL_EDGE_MIN_B)>(x[r], x[r], a);
+      mul_out<P_r>(a, a, b);
+      mul_out<P_r>(x[r], a, x[r]);  // < 3p for any input
+      cond_sub<P_r, 2>(x[r]);
+      cond_sub<P_r, 1>(x[r]);
     }
+  } else if (p.is_first) {  // the caller's values, taken up to 2p
+#pragma unroll
+    for (int r = 0; r < 8; r++) cond_sub<P_r, 1>(x[r]);
   }
   __syncthreads();
 
-  ntt_rounds<B, B>(x, q, g * M, smem, plane_stride, tws, active);
+  ntt_rounds<B, B, BATCH>(p, dft, x, pos, col, smem, plane_stride, tws);
   if (!active) return;
 
   // element r now holds output k = bitrev_B(8q + r)
   if (!p.is_final) {
+    const uint32_t sm = (uint32_t)__cvta_generic_to_shared(smem);
 #pragma unroll
     for (int r = 0; r < 8; r++) {
-      const uint32_t k = __brev(8 * q + r) >> (32 - B);
-      uint32_t w[8];
-      const uint32_t kj = (k << p.log_J) + col;
-      ld_fe_nc(w, p.twist + kj);
-      ntt_mul<(B >= ZK_NTT_CALL_EDGE_MIN_B)>(x[r], x[r], w);
-      st_fe(p.out + (((o << B) << p.log_J) + kj), x[r]);
+      asm volatile("cp.async.wait_group 3;" ::: "memory");
+      uint32_t v[8], w[8];
+      const uint32_t slot = sm + 16 * (4 * (r & 3) * pos.nt + t);
+      lds_v4(v, slot);
+      lds_v4(v + 4, slot + 16 * pos.nt);
+      lds_v4(w, slot + 32 * pos.nt);
+      lds_v4(w + 4, slot + 48 * pos.nt);
+      mul_w2<P_r>(x[r], x[r], v, w);
+      if (r < 4)
+        twist_fetch(p, B, pos, col, sm, r + 4);
+      else
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      st_fe(p.out + ((o << B << p.log_J) + twist_index(p, B, q, col, r)), x[r]);
     }
   } else {
     // rev(o): o = k_1 * 2^(b_2+..) + ... + k_(p-1);  rev = k_1 + 2^b_1 k_2 + ...
@@ -255,14 +500,20 @@ __device__ __forceinline__ void ntt_pass_tile(const PassParams& p, uint64_t tile
         uint32_t a[8], b[8];
         ld_fe_nc(a, p.post_lo + (kout & ((1u << p.post_shift) - 1u)));
         ld_fe_nc(b, p.post_hi + (kout >> p.post_shift));
-        ntt_mul<(B >= ZK_NTT_CALL_EDGE_MIN_B)>(a, a, b);
-        ntt_mul<(B >= ZK_NTT_CALL_EDGE_MIN_B)>(v, x[r], a);
-        reduce_once<P_r>(v, v);
+        mul_out<P_r>(a, a, b);
+        mul_out<P_r>(v, a, x[r]);  // < 3p
+        cond_sub<P_r, 2>(v);
+        cond_sub<P_r, 1>(v);
       } else if (p.has_post) {
-        ntt_mul<(B >= ZK_NTT_CALL_EDGE_MIN_B)>(v, x[r], p.post.w);
-        reduce_once<P_r>(v, v);
-      } else {
-        reduce_once<P_r>(v, x[r]);
+        mul_out<P_r>(v, p.post.w, x[r]);  // < 2p
+        cond_sub<P_r, 1>(v);
+      } else {  // the rounds leave up to 5 p
+        cpy(v, x[r]);
+        if constexpr (B <= kNarrowMax) {
+          cond_sub<P_r, 4>(v);
+          cond_sub<P_r, 2>(v);
+        }
+        cond_sub<P_r, 1>(v);
       }
       st_fe(p.out + kout, v);
     }
@@ -270,16 +521,16 @@ __device__ __forceinline__ void ntt_pass_tile(const PassParams& p, uint64_t tile
 }
 
 template <int B>
-__global__ void __launch_bounds__(256, ZK_NTT_MIN_BLOCKS) ntt_pass_kernel(const PassParams p) {
+__global__ void __launch_bounds__(256, 2) ntt_pass_kernel(const PassParams p, const DftConsts dft) {
   extern __shared__ __align__(16) uint32_t smem[];
-  ntt_pass_tile<B, false>(p, blockIdx.x, smem);
+  ntt_pass_tile<B, false>(p, &dft, blockIdx.x, smem);
 }
 
 template <int B>
-inline cudaError_t launch_pass(const PassParams& pp, uint64_t ncta, cudaStream_t s) {
+inline cudaError_t launch_pass(const PassParams& pp, const DftConsts& dft, uint64_t ncta, cudaStream_t s) {
   constexpr uint32_t M = 1u << B;
-  const uint32_t threads = pp.G * (M / 8);
-  const size_t smem = (size_t)8 * pp.G * M * 4 + (size_t)(M / 2) * 32;
+  const uint32_t threads = pp.ntile * pp.G * (M / 8);
+  const size_t smem = (size_t)8 * pp.ntile * pp.G * M * 4 + tw_smem_bytes(B);
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -287,11 +538,11 @@ inline cudaError_t launch_pass(const PassParams& pp, uint64_t ncta, cudaStream_t
     cudaFuncSetAttribute(ntt_pass_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     attr_set[dev & 63] = true;
   }
-  ntt_pass_kernel<B><<<(unsigned)ncta, threads, smem, s>>>(pp);
+  ntt_pass_kernel<B><<<(unsigned)ncta, threads, smem, s>>>(pp, dft);
   return cudaGetLastError();
 }
 
 // B = 7..11 (ntt_pass_wide.cu)
-cudaError_t launch_pass_wide(int B, const PassParams& pp, uint64_t ncta, cudaStream_t s);
+cudaError_t launch_pass_wide(int B, const PassParams& pp, const DftConsts& dft, uint64_t ncta, cudaStream_t s);
 
 }  // namespace zk
