@@ -174,3 +174,34 @@ def test_msm_in_bucket_doubling_and_cancellation(zk, oracle, n_pos, n_neg):
     kk = oracle.mul(oracle.to_mont((n_pos - n_neg) % B.R_MOD), k[0])
     want = oracle.msm_by_dlog(s[:1], kk.reshape(1, 4))
     assert np.array_equal(affine_of(zk.msm(s, bases)), want)
+
+
+@pytest.mark.parametrize("n_pos,n_neg", [(1 << 19, 5), (300_000, 300_000), (1 << 20, 0)])
+def test_msm_rounds_doubling_and_cancellation(zk, oracle, n_pos, n_neg):
+    """enough entries for the batch-affine rounds, in one bucket per window:
+    copies of P and -P in random order"""
+    pts, k = oracle.rand_bases(1, 79, with_dlog=True)
+    q = zk.FQ_MODULUS
+    neg = pts[0].copy()
+    neg[4:] = oracle.to_mont((q - oracle.from_mont(neg[4:], oracle.FQ)) % q, oracle.FQ)
+    n = n_pos + n_neg
+    order = np.random.default_rng(n).permutation(n)
+    bases = np.empty((n, 8), np.uint64)
+    bases[order[:n_pos]] = pts[0]
+    bases[order[n_pos:]] = neg
+    v = B.R_MOD - 0xBEEF12345
+    s = np.tile(oracle.to_mont(v), (n, 1))
+    kk = oracle.mul(oracle.to_mont((n_pos - n_neg) % B.R_MOD), k[0])
+    assert np.array_equal(affine_of(zk.msm(s, bases)), oracle.msm_by_dlog(s[:1], kk.reshape(1, 4)))
+
+
+@pytest.mark.parametrize("n", [257, 40_000, (1 << 19) + 77])
+def test_msm_few_buckets_and_identities(zk, oracle, n):
+    """Scalars from a handful of values (buckets of very different sizes, heavy
+    ones among them), a third of the bases the identity."""
+    pts, k = oracle.rand_bases(n, 83, with_dlog=True)
+    pts[::3] = 0
+    k[::3] = 0
+    vals = np.stack([oracle.to_mont(v) for v in (0, 1, 2, 2**15, 2**200 + 1, B.R_MOD - 1)])
+    s = np.ascontiguousarray(vals[np.random.default_rng(n).choice(6, n, p=[0.1, 0.5, 0.2, 0.1, 0.05, 0.05])])
+    assert np.array_equal(affine_of(zk.msm(s, pts)), oracle.msm_by_dlog(s, k))

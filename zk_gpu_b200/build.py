@@ -21,11 +21,10 @@ LIB = os.path.join(HERE, "libzkgpu.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
+FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
          "--expt-relaxed-constexpr", "-I", INCLUDE, "-I", CSRC]
-# extra nvcc flags, e.g. ZKGPU_NVCC_EXTRA="-DZK_MSM_CALL_PRODUCT=0"; BUILD_DIR /
-# LIB may be redirected with ZKGPU_BUILD_DIR / ZKGPU_LIB_OUT to keep such a
-# variant apart
+# extra nvcc flags; BUILD_DIR / LIB may be redirected with ZKGPU_BUILD_DIR /
+# ZKGPU_LIB_OUT to keep a variant apart
 FLAGS += os.environ.get("ZKGPU_NVCC_EXTRA", "").split()
 BUILD = os.environ.get("ZKGPU_BUILD_DIR", BUILD)
 LIB = os.environ.get("ZKGPU_LIB_OUT", LIB)

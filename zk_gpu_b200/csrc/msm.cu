@@ -8,6 +8,7 @@
 #include "fq_inv.cuh"
 #include "host_field.hpp"
 #include "msm.cuh"
+#include "quad.cuh"
 #include "prof.cuh"
 #include "runtime.cuh"
 
@@ -184,6 +185,9 @@ __global__ void scan_add_kernel(uint32_t* out, uint32_t* cursor, const uint32_t*
 // ---------------------------------------------------------------------------
 constexpr uint32_t BA_K = 16;  // pair sums per task (one chain of products)
 constexpr uint32_t BA_G = 32;  // task products per inversion
+// Apply blocks: five of 128 threads per SM fit at the 96 registers the kernel
+// needs (MSM of 2^22: 11.95 ms with two of 256, 11.73 ms so).
+constexpr uint32_t BA_APPLY = 128;
 
 // a^-1 for a != 0 in Montgomery form, lazy in, canonical out: the divstep
 // inversion (fq_inv.cuh) of the representative a 2^256 gives a^-1 2^-256,
@@ -232,32 +236,15 @@ __device__ __forceinline__ void sm_fe(uint32_t r[8], const uint4* my, uint32_t b
 
 // one pair sum of a round: its two points in the round's source (round 0:
 // entry-list words, base index plus sign bit; later rounds: positions in the
-// previous round's output), its bucket, and whether the second point exists
+// previous round's output), its bucket, whether the second point exists,
+// whether it is its bucket's first, and the bucket's points after the round
 constexpr uint32_t BA_CP = 4;   // chunks per prefix stage: x of both points
 constexpr uint32_t BA_CA = 10;  // chunks per apply stage: both points, one prefix product
 struct BaJob {
-  uint32_t pa, pb, b;
-  bool has2;
+  uint32_t pa, pb, b, nb;
+  bool has2, first;
 };
 
-template <bool FIRST>
-__device__ __forceinline__ BaJob ba_job(uint32_t q, uint32_t b, const uint32_t* __restrict__ joff,
-                                        const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ cprev,
-                                        const uint32_t* __restrict__ list) {
-  BaJob d;
-  const uint32_t j = q - joff[b];
-  const uint32_t i0 = in_off[b] + 2 * j;
-  d.b = b;
-  d.has2 = 2 * j + 1 < cprev[b];
-  if (FIRST) {
-    d.pa = list[i0];
-    d.pb = d.has2 ? list[i0 + 1] : 0u;
-  } else {
-    d.pa = i0;
-    d.pb = i0 + 1;
-  }
-  return d;
-}
 // point p of a round's source ((x, y) adjacent): round 0 reads the bases
 // (the entry's index, sign bit cleared), later rounds their own buffer of
 // affine pair sums.  (Bases kept as an x array and a y array instead were
@@ -268,12 +255,15 @@ template <bool FIRST>
 __device__ __forceinline__ const fe* ba_pt(const fe* src, uint32_t p) {
   return src + 2 * (uint64_t)(FIRST ? (p & 0x7fffffffu) : p);
 }
-// y of a round-0 point read out of its slot: negated for a negative digit
+// y of a round-0 point read out of its slot: q - y for a negative digit
 template <bool FIRST>
 __device__ __forceinline__ void ba_sign(aff_t& p, uint32_t e) {
-  if (FIRST && (e & 0x80000000u) && !is_zero(p.x)) {
-    uint32_t z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    sub<FqP>(p.y, z, p.y);
+  if (FIRST) {
+    uint32_t z[8] = {0, 0, 0, 0, 0, 0, 0, 0}, n[8];
+    sub_off<FqP, 1>(n, z, p.y);
+    const bool neg = (e & 0x80000000u) && !is_zero(p.y);
+#pragma unroll
+    for (int k = 0; k < 8; k++) p.y[k] = neg ? n[k] : p.y[k];
   }
 }
 
@@ -287,17 +277,59 @@ __device__ __forceinline__ uint32_t ba_search(const uint32_t* __restrict__ joff,
   }
   return lo;
 }
-__device__ __forceinline__ uint32_t ba_bucket_fwd(const uint32_t* __restrict__ joff, uint32_t T, uint32_t b,
-                                                  uint32_t q) {
-  if (joff[b + 1] > q) return b;
-  if (b + 2 <= T && joff[b + 2] > q) return b + 1;
-  return ba_search(joff, b + 1, T, q);
-}
-__device__ __forceinline__ uint32_t ba_bucket_bwd(const uint32_t* __restrict__ joff, uint32_t b, uint32_t q) {
-  if (joff[b] <= q) return b;
-  if (joff[b - 1] <= q) return b - 1;
-  return ba_search(joff, 0, b - 1, q);
-}
+// The bucket a thread's chain is in, kept in registers while the chain stays
+// in it: a job then costs no load but its entry-list words (three dependent
+// loads per job left 2.2 stalled warps per issue in the apply pass).
+struct BaCursor {
+  const uint32_t *joff, *in_off, *cprev;
+  uint32_t T, b, j0, j1, in0, c;  // bucket, its jobs [j0, j1), its first point, its points
+  __device__ __forceinline__ void load() {
+    j0 = joff[b];
+    j1 = joff[b + 1];
+    in0 = in_off[b];
+    c = cprev[b];
+  }
+  __device__ __forceinline__ BaCursor(const uint32_t* joff_, const uint32_t* in_off_, const uint32_t* cprev_,
+                                      uint32_t T_, uint32_t q)
+      : joff(joff_), in_off(in_off_), cprev(cprev_), T(T_) {
+    b = ba_search(joff, 0, T, q);
+    load();
+  }
+  // job q in the cursor's bucket or after (before) it
+  __device__ __forceinline__ void forward(uint32_t q) {
+    if (q < j1) return;
+    b++;
+    load();
+    if (q < j1) return;
+    b = ba_search(joff, b + 1, T, q);
+    load();
+  }
+  __device__ __forceinline__ void backward(uint32_t q) {
+    if (q >= j0) return;
+    b--;
+    load();
+    if (q >= j0) return;
+    b = ba_search(joff, 0, b, q);
+    load();
+  }
+  template <bool FIRST>
+  __device__ __forceinline__ BaJob job(uint32_t q, const uint32_t* __restrict__ list) const {
+    BaJob d;
+    const uint32_t j = q - j0, i0 = in0 + 2 * j;
+    d.b = b;
+    d.nb = (c + 1) / 2;
+    d.first = j == 0;
+    d.has2 = 2 * j + 1 < c;
+    if (FIRST) {
+      d.pa = list[i0];
+      d.pb = d.has2 ? list[i0 + 1] : 0u;
+    } else {
+      d.pa = i0;
+      d.pb = i0 + 1;
+    }
+    return d;
+  }
+};
 
 // stage the x coordinates of a job's points (prefix pass)
 template <bool FIRST>
@@ -332,7 +364,7 @@ __device__ __forceinline__ void ba_denominator(uint32_t d[8], const uint4* st, u
     sm_fe(x2, st, bd, 2);
     if (!is_zero(x1) && !is_zero(x2)) {
       if (!eq(x1, x2)) {
-        sub<FqP>(d, x2, x1);
+        sub_off<FqP, 1>(d, x2, x1);
         return;
       }
       aff_t p, q;
@@ -403,13 +435,13 @@ __global__ void __launch_bounds__(256) ba_prefix_kernel(const fe* __restrict__ s
   const uint32_t tasks = (J + K - 1) / K;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < tasks; t += gridDim.x * blockDim.x) {
     const uint32_t q0 = t * K, q1 = min(q0 + K, J);
-    uint32_t b = ba_search(joff, 0, T, q0);
-    BaJob d0 = ba_job<FIRST>(q0, b, joff, in_off, cprev, list), d1 = d0;
+    BaCursor at(joff, in_off, cprev, T, q0);
+    BaJob d0 = at.job<FIRST>(q0, list), d1 = d0;
     ba_stage_x<FIRST>(my, bd, src, d0);
     cp_commit();
     if (q0 + 1 < q1) {
-      b = ba_bucket_fwd(joff, T, b, q0 + 1);
-      d1 = ba_job<FIRST>(q0 + 1, b, joff, in_off, cprev, list);
+      at.forward(q0 + 1);
+      d1 = at.job<FIRST>(q0 + 1, list);
     }
     uint32_t acc[8];
     for (uint32_t q = q0; q < q1; q++) {
@@ -418,8 +450,8 @@ __global__ void __launch_bounds__(256) ba_prefix_kernel(const fe* __restrict__ s
       cp_commit();
       BaJob d2 = d1;
       if (q + 2 < q1) {
-        b = ba_bucket_fwd(joff, T, b, q + 2);
-        d2 = ba_job<FIRST>(q + 2, b, joff, in_off, cprev, list);
+        at.forward(q + 2);
+        d2 = at.job<FIRST>(q + 2, list);
       }
       cp_wait<1>();
       uint32_t d[8];
@@ -427,7 +459,7 @@ __global__ void __launch_bounds__(256) ba_prefix_kernel(const fe* __restrict__ s
       if (q == q0)
         cpy(acc, d);
       else
-        qmul(acc, acc, d);
+        mul_lazy<FqP>(acc, acc, d);
       st_fe(pre + q, acc);
       d0 = d1;
       d1 = d2;
@@ -475,12 +507,11 @@ __global__ void __launch_bounds__(128) ba_invert_kernel(fe* tot, fe* tpre, const
 // apply: walk each task's chain back and finish its pair sums; dynamic
 // shared memory: 2 stages x BA_CA chunks x 16 B per thread
 template <bool FIRST>
-__global__ void __launch_bounds__(256, 2) ba_apply_kernel(const fe* __restrict__ src,
+__global__ void __launch_bounds__(BA_APPLY, 5) ba_apply_kernel(const fe* __restrict__ src,
                                                           const uint32_t* __restrict__ list,
                                                           const uint32_t* __restrict__ in_off,
                                                           const uint32_t* __restrict__ cprev,
-                                                          const uint32_t* __restrict__ joff,
-                                                          const uint32_t* __restrict__ np, uint32_t T,
+                                                          const uint32_t* __restrict__ joff, uint32_t T,
                                                           const fe* __restrict__ pre, const fe* __restrict__ tot,
                                                           fe* __restrict__ dst, fe* __restrict__ fin,
                                                           uint32_t* __restrict__ cnt, uint32_t fill_k) {
@@ -494,13 +525,13 @@ __global__ void __launch_bounds__(256, 2) ba_apply_kernel(const fe* __restrict__
     const uint32_t q0 = t * K, q1 = min(q0 + K, J);
     uint32_t inv_run[8];
     ld_fe(inv_run, tot + t);
-    uint32_t b = ba_search(joff, 0, T, q1 - 1);
-    BaJob d0 = ba_job<FIRST>(q1 - 1, b, joff, in_off, cprev, list), d1 = d0;
+    BaCursor at(joff, in_off, cprev, T, q1 - 1);
+    BaJob d0 = at.job<FIRST>(q1 - 1, list), d1 = d0;
     ba_stage_pq<FIRST>(my, bd, src, d0, q1 - 1 > q0 ? pre + q1 - 2 : nullptr);
     cp_commit();
     if (q1 - 1 > q0) {
-      b = ba_bucket_bwd(joff, b, q1 - 2);
-      d1 = ba_job<FIRST>(q1 - 2, b, joff, in_off, cprev, list);
+      at.backward(q1 - 2);
+      d1 = at.job<FIRST>(q1 - 2, list);
     }
     for (uint32_t q = q1, i = 0; q-- > q0; i++) {
       const uint32_t s = i & 1;
@@ -508,8 +539,8 @@ __global__ void __launch_bounds__(256, 2) ba_apply_kernel(const fe* __restrict__
       cp_commit();
       BaJob d2 = d1;
       if (q > q0 + 1) {
-        b = ba_bucket_bwd(joff, b, q - 2);
-        d2 = ba_job<FIRST>(q - 2, b, joff, in_off, cprev, list);
+        at.backward(q - 2);
+        d2 = at.job<FIRST>(q - 2, list);
       }
       cp_wait<1>();
       const uint4* st = my + s * BA_CA * bd;
@@ -528,7 +559,7 @@ __global__ void __launch_bounds__(256, 2) ba_apply_kernel(const fe* __restrict__
       int kind = 0;  // 0: no inversion, 1: addition, 2: doubling
       if (has2 && !is_zero(P.x) && !is_zero(Q.x)) {
         if (!eq(P.x, Q.x)) {
-          sub<FqP>(d, Q.x, P.x);
+          sub_off<FqP, 1>(d, Q.x, P.x);
           kind = 1;
         } else if (eq(P.y, Q.y)) {
           add<FqP>(d, P.y, P.y);
@@ -540,8 +571,8 @@ __global__ void __launch_bounds__(256, 2) ba_apply_kernel(const fe* __restrict__
       if (q > q0) {
         uint32_t p[8];
         sm_fe(p, st, bd, 8);
-        qmul_c(inv_d, inv_run, p);
-        qmul_c(inv_run, inv_run, d);
+        mul_lazy<FqP>(inv_d, inv_run, p);
+        mul_lazy<FqP>(inv_run, inv_run, d);
       } else {
         cpy(inv_d, inv_run);
       }
@@ -553,30 +584,33 @@ __global__ void __launch_bounds__(256, 2) ba_apply_kernel(const fe* __restrict__
         set_zero(out.x);
         set_zero(out.y);
       } else {
+        // coordinates are canonical, products below 2q; each difference gets
+        // the multiple of q that keeps it positive
         uint32_t lam[8], t1[8];
         if (kind == 1) {
-          sub<FqP>(t1, Q.y, P.y);
+          sub_off<FqP, 1>(t1, Q.y, P.y);
         } else {  // doubling: 3 x^2 / (2 y)
-          qsqr_c(t1, P.x);
+          mul_out<FqP>(t1, P.x, P.x);
           uint32_t t2[8];
           add_lazy<FqP>(t2, t1, t1);
           add_lazy<FqP>(t1, t2, t1);
         }
-        qmul_c(lam, t1, inv_d);
-        qsqr_c(t1, lam);
-        qsub(t1, t1, P.x);
-        qsub(out.x, t1, Q.x);  // Q.x = P.x when doubling
-        reduce_once<FqP>(out.x, out.x);
-        qsub(t1, P.x, out.x);
-        qmul_c(t1, lam, t1);
-        qsub(out.y, t1, P.y);
-        reduce_once<FqP>(out.y, out.y);
+        mul_lazy<FqP>(lam, t1, inv_d);
+        mul_lazy<FqP>(t1, lam, lam);
+        add_raw(d, P.x, Q.x);  // Q.x = P.x when doubling
+        sub_off<FqP, 2>(out.x, t1, d);
+        cond_sub<FqP, 2>(out.x);
+        cond_sub<FqP, 1>(out.x);
+        sub_off<FqP, 1>(t1, P.x, out.x);
+        mul_lazy<FqP>(t1, lam, t1);
+        sub_off<FqP, 1>(out.y, t1, P.y);
+        cond_sub<FqP, 2>(out.y);
+        cond_sub<FqP, 1>(out.y);
       }
-      const uint32_t bq = d0.b, nb = np[bq];
-      fe* o = nb == 1 ? fin + 2 * (uint64_t)bq : dst + 2 * (uint64_t)q;
+      fe* o = d0.nb == 1 ? fin + 2 * (uint64_t)d0.b : dst + 2 * (uint64_t)q;
       st_fe(o, out.x);
       st_fe(o + 1, out.y);
-      if (q == joff[bq]) cnt[bq] = nb;
+      if (d0.first) cnt[d0.b] = d0.nb;
       d0 = d1;
       d1 = d2;
     }
@@ -585,89 +619,156 @@ __global__ void __launch_bounds__(256, 2) ba_apply_kernel(const fe* __restrict__
 }
 
 // Tail: what the rounds left (a few points per bucket, or many in a skewed
-// bucket such as the one small scalars carry into) is folded with XYZZ mixed
-// additions in chunks of BA_TS points, one thread per chunk; a bucket's
-// chunk sums are then added by one thread, or block-wide when there are many.
-constexpr uint32_t BA_TS = 16;    // points per tail chunk
-constexpr uint32_t BA_TSEQ = 16;  // chunk sums a bucket adds in one thread
+// bucket such as the one small scalars carry into), or, without rounds, the
+// entries themselves, is folded with XYZZ mixed additions in chunks of at most
+// BA_TS points, one thread per chunk; a bucket's chunk sums are then added by
+// one quad of lanes (quad.cuh), or by blocks when there are many.
+// Points per tail chunk: a chunk more costs an addition of two sums (14
+// products) for one of its mixed additions (10), and short chunks of equal
+// length keep a warp's lanes together.
+constexpr uint32_t BA_TS = 8;
+constexpr uint32_t BA_TSEQ = 24;     // chunk sums a bucket adds one by one
+constexpr uint32_t BA_HEAVY = 2048;  // chunk sums a block adds
 
+__device__ __forceinline__ uint32_t ba_chunk_count(uint32_t c) { return c <= 1 ? 1u : (c + BA_TS - 1) / BA_TS; }
 __global__ void ba_chunks_kernel(const uint32_t* cnt, uint32_t* nch, uint32_t T) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= T) return;
-  const uint32_t c = cnt[b];
-  nch[b] = c <= 1 ? 1u : (c + BA_TS - 1) / BA_TS;
+  nch[b] = ba_chunk_count(cnt[b]);
 }
 
-__global__ void __launch_bounds__(256) ba_fold_kernel(const uint32_t* cnt, const uint32_t* in_off, const fe* src,
-                                                      const fe* fin, const uint32_t* coff, const uint32_t* nch,
-                                                      uint32_t T, fe* chunk_res) {
+// ENTRIES: the points are the bases named by the sorted list; otherwise the
+// last round's sums (buckets of one point in `fin`).  A bucket's chunks share
+// its points evenly, so that a warp's lanes run chains of similar length.  The
+// next point is copied to the thread's slot of shared memory while the current
+// one is added (two stages, as in the rounds).
+template <bool ENTRIES>
+__global__ void __launch_bounds__(256, 2) ba_fold_kernel(const uint32_t* __restrict__ cnt,
+                                                         const uint32_t* __restrict__ in_off,
+                                                         const fe* __restrict__ src, const uint32_t* __restrict__ list,
+                                                         const fe* __restrict__ fin, const uint32_t* __restrict__ coff,
+                                                         uint32_t T, fe* __restrict__ chunk_res) {
+  __shared__ uint4 stage[2 * 4 * 256];
+  uint4* my = stage + threadIdx.x;
   const uint32_t C = coff[T];
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < C; u += gridDim.x * blockDim.x) {
     const uint32_t b = ba_search(coff, 0, T, u);
-    const uint32_t k = u - coff[b], c = cnt[b];
+    const uint32_t c = cnt[b], o = in_off[b], k = u - coff[b], nk = ba_chunk_count(c);
+    const uint32_t i0 = (uint32_t)((uint64_t)c * k / nk), i1 = (uint32_t)((uint64_t)c * (k + 1) / nk);
     xyzz_t acc;
     xyzz_set_inf(acc);
     aff_t p;
-    if (c <= 1) {
+    if (!ENTRIES && c <= 1) {
       ld_aff(p, fin + 2 * (uint64_t)b);
       xyzz_from_aff(acc, p);  // (0, 0) -> identity
-    } else {
-      const uint32_t o = in_off[b], i1 = min(c, (k + 1) * BA_TS);
-      for (uint32_t i = k * BA_TS; i < i1; i++) {
-        ld_aff(p, src + 2 * (uint64_t)(o + i));
-        xyzz_madd(acc, p);
+    } else if (i0 < i1) {
+      uint32_t e = ENTRIES ? list[o + i0] : o + i0, e1 = e;
+      const fe* g = ba_pt<ENTRIES>(src, e);
+      cp_fe(my, 256, 0, g);
+      cp_fe(my, 256, 2, g + 1);
+      cp_commit();
+      if (i0 + 1 < i1) e1 = ENTRIES ? list[o + i0 + 1] : o + i0 + 1;
+      for (uint32_t i = i0; i < i1; i++) {
+        const uint32_t s = (i - i0) & 1u;
+        uint32_t e2 = e1;
+        if (i + 1 < i1) {
+          g = ba_pt<ENTRIES>(src, e1);
+          cp_fe(my + (s ^ 1u) * 1024, 256, 0, g);
+          cp_fe(my + (s ^ 1u) * 1024, 256, 2, g + 1);
+          if (i + 2 < i1) e2 = ENTRIES ? list[o + i + 2] : o + i + 2;
+        }
+        cp_commit();
+        cp_wait<1>();
+        sm_fe(p.x, my + s * 1024, 256, 0);
+        sm_fe(p.y, my + s * 1024, 256, 2);
+        ba_sign<ENTRIES>(p, e);
+        xyzz_madd<true>(acc, p);
+        e = e1;
+        e1 = e2;
       }
     }
     st_xyzz(chunk_res + 4 * (uint64_t)u, acc);
   }
+  cp_wait<0>();
 }
 
-__global__ void ba_bucket_sum_kernel(const uint32_t* coff, const uint32_t* nch, const fe* chunk_res, fe* buckets,
-                                     uint32_t* heavy, uint32_t* heavy_count, uint32_t T) {
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+// heavy: items (bucket, first chunk) of the buckets with more than BA_TSEQ
+// chunk sums, one per BA_HEAVY of them; heavy_count = {items, buckets}
+__global__ void __launch_bounds__(128) ba_bucket_sum_kernel(const uint32_t* coff, const fe* chunk_res, fe* buckets,
+                                                            uint2* heavy, uint32_t* heavy_b, uint32_t* heavy_count,
+                                                            uint32_t T) {
+  const Quad z;
+  const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (b >= T) return;
-  const uint32_t k = nch[b], o = coff[b];
+  const uint32_t o = coff[b], k = coff[b + 1] - o;
   if (k > BA_TSEQ) {
-    heavy[atomicAdd(heavy_count, 1u)] = b;
+    if (z.j == 0) {
+      const uint32_t n = (k + BA_HEAVY - 1) / BA_HEAVY, at = atomicAdd(heavy_count, n);
+      for (uint32_t i = 0; i < n; i++) heavy[at + i] = make_uint2(b, i * BA_HEAVY);
+      heavy_b[atomicAdd(heavy_count + 1, 1u)] = b;
+    }
     return;
   }
-  xyzz_t acc, t;
-  ld_xyzz(acc, chunk_res + 4 * (uint64_t)o);
+  uint32_t acc[8], x[8];
+  const fe* src = chunk_res + 4 * (uint64_t)o + z.j;
+  ld_fe(acc, src);
   for (uint32_t j = 1; j < k; j++) {
-    ld_xyzz(t, chunk_res + 4 * (uint64_t)(o + j));
-    xyzz_add(acc, t);
+    ld_fe(x, src + 4 * j);
+    quad_add(z, acc, x);
   }
-  st_xyzz(buckets + 4 * (uint64_t)b, acc);
+  st_fe(buckets + 4 * (uint64_t)b + z.j, acc);
 }
 
-// One block per queued heavy bucket: strided partial sums, then a tree.
-__global__ void __launch_bounds__(256) ba_heavy_kernel(const uint32_t* coff, const uint32_t* nch, const fe* chunk_res,
-                                                       fe* buckets, const uint32_t* heavy,
-                                                       const uint32_t* heavy_count) {
-  __shared__ fe sh[256 * 4];
-  if (blockIdx.x >= *heavy_count) return;
-  const uint32_t b = heavy[blockIdx.x];
-  const uint32_t k = nch[b], o = coff[b];
-  xyzz_t acc, t;
-  xyzz_set_inf(acc);
-  for (uint32_t j = threadIdx.x; j < k; j += blockDim.x) {
-    ld_xyzz(t, chunk_res + 4 * (uint64_t)(o + j));
-    xyzz_add(acc, t);
+// The block's sum of points src[first], src[first + step], .. below `end`, by
+// its 64 quads: strided partial sums, then a tree in shared memory; quad 0
+// holds it.
+__device__ __forceinline__ void block_sum(const Quad& z, uint32_t acc[8], fe* sh, const fe* src, uint32_t first,
+                                          uint32_t end, uint32_t step) {
+  const uint32_t t = threadIdx.x >> 2, nt = blockDim.x >> 2;
+  uint32_t x[8];
+  set_zero(acc);
+  for (uint32_t j = first + t * step; j < end; j += nt * step) {
+    ld_fe(x, src + 4 * (uint64_t)j + z.j);
+    quad_add(z, acc, x);
   }
-  st_xyzz(sh + 4 * threadIdx.x, acc);
+  st_fe(sh + 4 * t + z.j, acc);
   __syncthreads();
-  for (uint32_t half = blockDim.x / 2; half > 0; half >>= 1) {
-    if (threadIdx.x < half) {
-      ld_xyzz(acc, sh + 4 * threadIdx.x);
-      ld_xyzz(t, sh + 4 * (threadIdx.x + half));
-      xyzz_add(acc, t);
-      st_xyzz(sh + 4 * threadIdx.x, acc);
+  for (uint32_t half = nt / 2; half > 0; half >>= 1) {
+    if (t < half) {
+      ld_fe(x, sh + 4 * (t + half) + z.j);
+      quad_add(z, acc, x);
+      st_fe(sh + 4 * t + z.j, acc);
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    ld_xyzz(acc, sh);
-    st_xyzz(buckets + 4 * (uint64_t)b, acc);
+}
+// Heavy buckets in two steps: each item's chunk sums into its first one, then
+// each bucket's items.
+__global__ void __launch_bounds__(256) ba_heavy_items_kernel(const uint32_t* coff, fe* chunk_res, const uint2* heavy,
+                                                             const uint32_t* heavy_count) {
+  __shared__ fe sh[256];
+  const Quad z;
+  const uint32_t n = heavy_count[0];
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    const uint2 it = heavy[i];
+    const uint32_t o = coff[it.x] + it.y, end = min(o + BA_HEAVY, coff[it.x + 1]);
+    uint32_t acc[8];
+    block_sum(z, acc, sh, chunk_res, o, end, 1);
+    if (threadIdx.x < 4) st_fe(chunk_res + 4 * (uint64_t)o + z.j, acc);
+    __syncthreads();
+  }
+}
+__global__ void __launch_bounds__(256) ba_heavy_kernel(const uint32_t* coff, const fe* chunk_res, fe* buckets,
+                                                       const uint32_t* heavy_b, const uint32_t* heavy_count) {
+  __shared__ fe sh[256];
+  const Quad z;
+  const uint32_t n = heavy_count[1];
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    const uint32_t b = heavy_b[i];
+    uint32_t acc[8];
+    block_sum(z, acc, sh, chunk_res, coff[b], coff[b + 1], BA_HEAVY);
+    if (threadIdx.x < 4) st_fe(buckets + 4 * (uint64_t)b + z.j, acc);
+    __syncthreads();
   }
 }
 
@@ -675,107 +776,73 @@ __global__ void __launch_bounds__(256) ba_heavy_kernel(const uint32_t* coff, con
 // buckets.  Level 1, one thread per segment of L buckets: running sums from
 // the top give T_s = sum_i (i + 1) B_{sL+i} and S_s = sum_i B_{sL+i}, so
 // W = sum_s T_s + L sum_s s S_s.
+// A quad of lanes per segment (quad.cuh).
 __global__ void __launch_bounds__(128) msm_segment_kernel(const fe* buckets, fe* seg_t, fe* seg_s, uint32_t B,
                                                           uint32_t L, uint32_t total_segs) {
-  const uint32_t gs = blockIdx.x * blockDim.x + threadIdx.x;
+  const Quad z;
+  const uint32_t gs = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (gs >= total_segs) return;
   const uint32_t S_per_w = B / L;
   const uint32_t w = gs / S_per_w, s = gs % S_per_w;
-  const uint32_t lo = s * L;
-  xyzz_t run, tot, bk;
-  xyzz_set_inf(run);
-  xyzz_set_inf(tot);
-  for (int j = (int)(lo + L) - 1; j >= (int)lo; j--) {
-    ld_xyzz(bk, buckets + 4 * ((uint64_t)w * B + j));
-    xyzz_add(run, bk);
-    xyzz_add(tot, run);
+  const fe* bk = buckets + 4 * ((uint64_t)w * B + (uint64_t)s * L) + z.j;
+  uint32_t run[8], tot[8], x[8];
+  ld_fe(run, bk + 4 * (L - 1));
+  cpy(tot, run);
+  for (int j = (int)L - 2; j >= 0; j--) {
+    ld_fe(x, bk + 4 * j);
+    quad_add(z, run, x);
+    quad_add(z, tot, run);
   }
-  st_xyzz(seg_t + 4 * (uint64_t)gs, tot);
-  st_xyzz(seg_s + 4 * (uint64_t)gs, run);
+  st_fe(seg_t + 4 * (uint64_t)gs + z.j, tot);
+  st_fe(seg_s + 4 * (uint64_t)gs + z.j, run);
 }
 
-// Level 2, one block per window, thread t owning M consecutive segments
-// (S_per_w and the block size are powers of two): A_t = sum_k T_{tM+k},
-// U_t = sum_k k S_{tM+k} and V_t = sum_k S_{tM+k} by running sums, so that
-// sum_s s S_s = sum_t U_t + M sum_t t V_t, and sum_t t V_t = sum_{t>=1} P_t
-// with P_t = sum_{u>=t} V_u (a block suffix scan).  Thread t contributes
-// c_t = A_t + L U_t + L M P_t (no P term for t = 0); a tree sum gives W.
-// The serial depth is about M + 2 log2(256) additions and log2(L M)
-// doublings per window, against L + c doublings and additions per segment
-// for multiplying every segment sum by its offset (measured on B200, 2^22
-// points, c = 16: 1.16 ms for both levels against 1.25 ms).  The
-// accumulator not being added to waits in the thread's slot of shared
-// memory (two slot arrays, 64 KiB of dynamic shared memory), so at most
-// two points are live in registers.
-constexpr int kWindowSmem = 2 * 256 * 128;
-__global__ void __launch_bounds__(256) msm_window_kernel(const fe* seg_t, const fe* seg_s, fe* winsum,
-                                                         uint32_t S_per_w, uint32_t L) {
-  extern __shared__ uint4 win_smem[];
-  fe* sc = reinterpret_cast<fe*>(win_smem);  // per thread: c_t, then the tree
-  fe* sv = sc + 4 * blockDim.x;               // per thread: V_t, then the scan
-  const uint32_t w = blockIdx.x, t = threadIdx.x, nt = blockDim.x;
-  const uint32_t M = S_per_w > nt ? S_per_w / nt : 1u;
-  const uint32_t active = S_per_w / M;
-  xyzz_t a, x;
-  xyzz_set_inf(a);
-  st_xyzz(sc + 4 * t, a);  // U_t accumulates here
-  if (t < active) {
-    const uint64_t base = (uint64_t)w * S_per_w + (uint64_t)t * M;
-    // a = V (running), U in sc
-    for (uint32_t k = M - 1; k >= 1; k--) {
-      ld_xyzz(x, seg_s + 4 * (base + k));
-      xyzz_add(a, x);
-      ld_xyzz(x, sc + 4 * t);
-      xyzz_add(x, a);
-      st_xyzz(sc + 4 * t, x);
-    }
-    ld_xyzz(x, seg_s + 4 * base);
-    xyzz_add(a, x);
-    st_xyzz(sv + 4 * t, a);  // V_t
-    // a = L U_t + A_t
-    ld_xyzz(a, sc + 4 * t);
-    for (uint32_t m = L; m > 1; m >>= 1) xyzz_dbl(a, a);  // L a power of two
-    for (uint32_t k = 0; k < M; k++) {
-      ld_xyzz(x, seg_t + 4 * (base + k));
-      xyzz_add(a, x);
-    }
-  } else {
-    st_xyzz(sv + 4 * t, a);
-  }
-  st_xyzz(sc + 4 * t, a);
+// Level 2 and up, a group of S <= 16 quads per S segments: with segments of L
+// buckets, (T_s, S_s), the group is a segment of S L buckets with
+// T = sum_t T_t + L sum_{t>=1} P_t, P_t = sum_{u>=t} S_u, and S = P_0.  A suffix
+// scan gives the P_t, a tree adds T_t + L P_t: logarithmic depth, where running
+// sums would take three additions per segment one after the other.  The last
+// level's groups are the windows.  Points pass between quads through shared
+// memory; a window's work is spread over groups because a block's products are
+// one SM's (one block per window, scanning 1024 segments, took 240 us).
+constexpr uint32_t kGroup = 16;
+__global__ void __launch_bounds__(4 * kGroup) msm_group_kernel(const fe* in_t, const fe* in_s, fe* out_t, fe* out_s,
+                                                               uint32_t S, uint32_t L) {
+  __shared__ fe sh[2][4 * kGroup];
+  const Quad z;
+  const uint32_t g = blockIdx.x, t = threadIdx.x >> 2;
+  uint32_t v[8], c[8], x[8];
+  const uint64_t base = 4 * ((uint64_t)g * S + t) + z.j;
+  ld_fe(v, in_s + base);
+  ld_fe(c, in_t + base);
+  uint32_t cur = 0;
+  st_fe(&sh[0][4 * t + z.j], v);
   __syncthreads();
-  // suffix sums of V across the block
-  ld_xyzz(a, sv + 4 * t);
-  for (uint32_t off = 1; off < nt; off <<= 1) {
-    const bool has = t + off < nt;
-    if (has) ld_xyzz(x, sv + 4 * (t + off));
-    __syncthreads();
-    if (has) {
-      xyzz_add(a, x);
-      st_xyzz(sv + 4 * t, a);
+  for (uint32_t off = 1; off < S; off <<= 1) {
+    if (t + off < S) {
+      ld_fe(x, &sh[cur][4 * (t + off) + z.j]);
+      quad_add(z, v, x);
     }
-    __syncthreads();
-  }
-  if (t > 0) {
-    for (uint32_t m = L * M; m > 1; m >>= 1) xyzz_dbl(a, a);  // L M P_t
-    ld_xyzz(x, sc + 4 * t);
-    xyzz_add(x, a);
-    st_xyzz(sc + 4 * t, x);
-  }
-  __syncthreads();
-  for (uint32_t half = nt / 2; half > 0; half >>= 1) {
-    if (t < half) {
-      ld_xyzz(a, sc + 4 * t);
-      ld_xyzz(x, sc + 4 * (t + half));
-      xyzz_add(a, x);
-      st_xyzz(sc + 4 * t, a);
-    }
+    cur ^= 1u;
+    st_fe(&sh[cur][4 * t + z.j], v);
     __syncthreads();
   }
   if (t == 0) {
-    ld_xyzz(a, sc);
-    st_xyzz(winsum + 4 * (uint64_t)w, a);
+    if (out_s) st_fe(out_s + 4 * (uint64_t)g + z.j, v);
+  } else {
+    for (uint32_t m = L; m > 1; m >>= 1) quad_dbl(z, v);
+    quad_add(z, c, v);
   }
+  for (uint32_t half = S / 2; half > 0; half >>= 1) {
+    cur ^= 1u;
+    if (t >= half && t < 2 * half) st_fe(&sh[cur][4 * t + z.j], c);
+    __syncthreads();
+    if (t < half) {
+      ld_fe(x, &sh[cur][4 * (t + half) + z.j]);
+      quad_add(z, c, x);
+    }
+  }
+  if (t == 0) st_fe(out_t + 4 * (uint64_t)g + z.j, c);
 }
 
 __global__ void zero_out_kernel(fe* out) {
@@ -843,8 +910,7 @@ constexpr uint32_t kFillK = 148 * 64;  // task threads that fill a B200 (148 SMs
 
 // dynamic shared memory of the round kernels at 256 threads (two stages)
 constexpr int kPrefixSmem = 2 * BA_CP * 16 * 256;  // 32 KiB
-constexpr int kApplySmem = 2 * BA_CA * 16 * 256;   // 80 KiB: above the 48 KiB default, opted in per device
-// (as is the window kernel's kWindowSmem, 64 KiB)
+constexpr int kApplySmem = 2 * BA_CA * 16 * BA_APPLY;   // 80 KiB: above the 48 KiB default, opted in per device
 
 cudaError_t ba_kernel_attrs(int device) {
   static std::mutex mu;
@@ -854,10 +920,15 @@ cudaError_t ba_kernel_attrs(int device) {
   cudaError_t e = cudaFuncSetAttribute(ba_apply_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kApplySmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ba_apply_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kApplySmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(msm_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWindowSmem);
   if (e == cudaSuccess && device < 64) done |= 1ull << device;
   return e;
+}
+
+int sm_count(int dev = -1) {
+  int sms = 148;
+  if (dev < 0) cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
 }
 
 // Buffer sizes of one MSM pass (msm_run_impl allocates exactly these;
@@ -869,19 +940,30 @@ struct MsmLayout {
   uint64_t jb[2] = {0, 0};       // pair sums of rounds 0 and 1, upper bounds
   uint64_t tasks0 = 0;
   uint64_t chunks = 0;           // tail chunks, upper bound
+  uint64_t heavy = 0;            // heavy buckets and their items, upper bound
   bool ok = false;
   uint64_t bytes(bool own_winsum) const {
     const uint64_t T1 = T + 1ull;
     uint64_t b = 0;
     b += T * 4ull * 2 + T1 * 4 + (nblk + 1ull) * 4 + E * 4;        // counts, cursor, offsets, bsums, list
-    b += T * 4ull * 3 + T1 * 4 * 2 + T * 64ull;                   // cnt, cprev, np, joff x2, fin
-    b += jb[0] * 64 + (rounds > 1 ? jb[1] * 64 : 0) + jb[0] * 32;  // round buffers, prefixes
-    b += tasks0 * 32 * 2;                                         // task products, their prefixes
-    b += T * 4ull * 2 + chunks * 128 + 4;                         // tail: chunk counts, heavy list, chunk sums
-    b += T * 128ull + segs * 256ull + (own_winsum ? W * 128ull : 0);  // buckets, segment T_s and S_s
-    return b + 24 * 256;  // pool granularity per allocation
+    b += T1 * 4;                                                  // chunk offsets
+    if (rounds) {
+      b += T * 4ull * 3 + T1 * 4 + T * 64ull;                        // cnt, cprev, np, second offsets, fin
+      b += jb[0] * 64 + (rounds > 1 ? jb[1] * 64 : 0) + jb[0] * 32;  // round buffers, prefixes
+      b += tasks0 * 32 * 2;                                         // task products, their prefixes
+    }
+    b += T * 4ull + chunks * 128 + heavy * 12 + 8;                // tail: chunk counts, chunk sums, heavy lists
+    b += T * 128ull + segs * 512ull + (own_winsum ? W * 128ull : 0);  // buckets, segment T_s and S_s
+    return b + 32 * 256;  // alignment of the pieces
   }
 };
+
+// Entries (point-window pairs) from which the batch-affine rounds pay: 6.2
+// products per addition against 10, but each round is a chain of launches
+// around an inversion, and its sums travel through memory.  MSM with rounds /
+// without on B200: 5.1e6 entries (300007 points) 2124 / 2054 us, 1.7e7 (2^20)
+// 4148 / 4496 us, 4.3e5 (2^14) 1042 / 766 us.
+constexpr uint64_t kRoundsMinEntries = 1ull << 23;
 
 MsmLayout msm_layout(uint64_t n, uint32_t jobs, int c_override, int device = -1) {
   MsmLayout l;
@@ -906,22 +988,19 @@ MsmLayout msm_layout(uint64_t n, uint32_t jobs, int c_override, int device = -1)
   while ((1ull << lg) < mean) lg++;
   // batch-affine rounds while buckets hold more than about four points;
   // later levels cost more in per-round latency than they save
-  l.rounds = lg > 3 ? lg - 2 : 1;
-  l.jb[0] = l.E / 2 + l.T;
-  l.jb[1] = l.jb[0] / 2 + l.T;
-  l.tasks0 = ba_tasks_bound(l.jb[0], kFillK);
-  uint64_t jlast = l.jb[0];
-  for (uint32_t r = 1; r < l.rounds; r++) jlast = jlast / 2 + l.T;
-  l.chunks = l.T + jlast / BA_TS + 1;  // bound on sum_b max(1, ceil(cnt_b / BA_TS))
+  l.rounds = l.E < kRoundsMinEntries ? 0 : lg > 3 ? lg - 2 : 1;
+  uint64_t left = l.E;  // points the tail folds, upper bound
+  if (l.rounds) {
+    l.jb[0] = l.E / 2 + l.T;
+    l.jb[1] = l.jb[0] / 2 + l.T;
+    l.tasks0 = ba_tasks_bound(l.jb[0], kFillK);
+    left = l.jb[0];
+    for (uint32_t r = 1; r < l.rounds; r++) left = left / 2 + l.T;
+  }
+  l.chunks = l.T + left / BA_TS + 1;  // bound on sum_b max(1, ceil(cnt_b / BA_TS))
+  l.heavy = std::min<uint64_t>(l.T, l.chunks / (BA_TSEQ + 1)) + l.chunks / BA_HEAVY + 1;
   l.ok = true;
   return l;
-}
-
-int sm_count() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
 }
 
 // n: scalars (all jobs); jobs > 1: job_off (device, jobs + 1 entries) splits
@@ -957,34 +1036,44 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
   fe *fin = nullptr, *buf[2] = {nullptr, nullptr}, *pre = nullptr, *tot = nullptr, *tpre = nullptr;
   fe *buckets = nullptr, *segres = nullptr, *segsum = nullptr, *winsum = nullptr;
   fe* chunk_res = nullptr;
-  uint32_t *nch = nullptr, *heavy = nullptr, *heavy_count = nullptr;
-  cudaError_t e = cudaSuccess;
+  uint32_t *nch = nullptr, *heavy_b = nullptr, *heavy_count = nullptr;
+  uint2* heavy = nullptr;
+  // one allocation, cut into aligned pieces
+  char* arena = nullptr;
+  const uint64_t arena_bytes = l.bytes(!wout);
+  uint64_t used = 0;
+  cudaError_t e = zk::dmalloc((void**)&arena, arena_bytes, s);
   auto alloc = [&](void** ptr, size_t bytes) {
-    if (e == cudaSuccess) e = zk::dmalloc(ptr, bytes ? bytes : 4, s);
+    *ptr = arena + used;
+    used += (bytes + 255) & ~(uint64_t)255;
+    if (e == cudaSuccess && used > arena_bytes) e = cudaErrorInvalidValue;
   };
   alloc((void**)&counts, T * 4ull);
   alloc((void**)&offsets, (T + 1ull) * 4);
   alloc((void**)&cursor, T * 4ull);
   alloc((void**)&bsums, (nblk + 1ull) * 4);
   alloc((void**)&list, entries * 4ull);
-  alloc((void**)&cnt, T * 4ull);
-  alloc((void**)&cprev, T * 4ull);
-  alloc((void**)&np, T * 4ull);
   alloc((void**)&joff[0], (T + 1ull) * 4);
-  alloc((void**)&joff[1], (T + 1ull) * 4);
-  alloc((void**)&fin, T * 64ull);
-  alloc((void**)&buf[0], l.jb[0] * 64);
-  if (l.rounds > 1) alloc((void**)&buf[1], l.jb[1] * 64);
-  alloc((void**)&pre, l.jb[0] * 32);
-  alloc((void**)&tot, l.tasks0 * 32);
-  alloc((void**)&tpre, l.tasks0 * 32);
+  if (l.rounds) {
+    alloc((void**)&cnt, T * 4ull);
+    alloc((void**)&cprev, T * 4ull);
+    alloc((void**)&np, T * 4ull);
+    alloc((void**)&joff[1], (T + 1ull) * 4);
+    alloc((void**)&fin, T * 64ull);
+    alloc((void**)&buf[0], l.jb[0] * 64);
+    if (l.rounds > 1) alloc((void**)&buf[1], l.jb[1] * 64);
+    alloc((void**)&pre, l.jb[0] * 32);
+    alloc((void**)&tot, l.tasks0 * 32);
+    alloc((void**)&tpre, l.tasks0 * 32);
+  }
   alloc((void**)&nch, T * 4ull);
-  alloc((void**)&heavy, T * 4ull);
-  alloc((void**)&heavy_count, 4);
+  alloc((void**)&heavy, l.heavy * 8);
+  alloc((void**)&heavy_b, l.heavy * 4);
+  alloc((void**)&heavy_count, 8);
   alloc((void**)&chunk_res, l.chunks * 128);
   alloc((void**)&buckets, T * 128ull);
-  alloc((void**)&segres, segs * 128ull);
-  alloc((void**)&segsum, segs * 128ull);
+  alloc((void**)&segres, segs * 256ull);  // one level and the next
+  alloc((void**)&segsum, segs * 256ull);
   if (wout)
     winsum = wout->d_winsum;  // caller's buffer, left for the host's Horner step
   else
@@ -1017,8 +1106,10 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
       // convention: 6 Fq products per point-window (the batch-affine cost);
       // algorithmic bytes: each entry's index and signed base read once
       ProfScope ps("msm_bucket", s, (double)entries * 6, (double)entries * 68);
-      ba_setup_kernel<<<gb, 256, 0, s>>>(counts, offsets, list, d_bases, cnt, fin, T);
-      nl++;
+      if (l.rounds) {
+        ba_setup_kernel<<<gb, 256, 0, s>>>(counts, offsets, list, d_bases, cnt, fin, T);
+        nl++;
+      }
       uint64_t jb = l.jb[0];
       for (uint32_t r = 0; r < l.rounds; r++) {
         const bool first = r == 0;
@@ -1036,6 +1127,7 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
         const uint64_t tasks = ba_tasks_bound(jb, fill_k);
         const uint32_t fill = (uint32_t)sms * 32;
         const unsigned gt = (unsigned)std::min<uint64_t>((tasks + 255) / 256, (uint64_t)sms * 6);
+        const unsigned ga = (unsigned)std::min<uint64_t>((tasks + BA_APPLY - 1) / BA_APPLY, (uint64_t)sms * 10);
         const uint64_t groups = tasks < fill ? tasks : std::max<uint64_t>(2ull * fill, tasks / BA_G + 1);
         const unsigned gi = (unsigned)std::min<uint64_t>((groups + 127) / 128, (uint64_t)sms * 8);
         if (first)
@@ -1044,44 +1136,52 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
           ba_prefix_kernel<false><<<gt, 256, kPrefixSmem, s>>>(src, list, in_off, cprev, jo, T, pre, tot, fill_k);
         ba_invert_kernel<<<gi, 128, 0, s>>>(tot, tpre, jo, T, fill, fill_k);
         if (first)
-          ba_apply_kernel<true><<<gt, 256, kApplySmem, s>>>(src, list, in_off, cprev, jo, np, T, pre, tot, dst, fin,
+          ba_apply_kernel<true><<<ga, BA_APPLY, kApplySmem, s>>>(src, list, in_off, cprev, jo, T, pre, tot, dst, fin,
                                                             cnt, fill_k);
         else
-          ba_apply_kernel<false><<<gt, 256, kApplySmem, s>>>(src, list, in_off, cprev, jo, np, T, pre, tot, dst, fin,
+          ba_apply_kernel<false><<<ga, BA_APPLY, kApplySmem, s>>>(src, list, in_off, cprev, jo, T, pre, tot, dst, fin,
                                                              cnt, fill_k);
         nl += 7;
         jb = jb / 2 + T;
       }
-      // tail: chunk counts -> scan (offsets in joff of the unused parity) -> folds -> bucket sums
+      // tail: chunk counts -> scan (offsets in the joff not in use) -> folds -> bucket sums
       const uint32_t last = (l.rounds - 1) & 1;
-      uint32_t* coff = joff[last ^ 1];
-      ba_chunks_kernel<<<gb, 256, 0, s>>>(cnt, nch, T);
+      uint32_t* coff = l.rounds ? joff[last ^ 1] : joff[0];
+      const uint32_t* left = l.rounds ? cnt : counts;
+      ba_chunks_kernel<<<gb, 256, 0, s>>>(left, nch, T);
       scan_block_kernel<<<nblk, 1024, 0, s>>>(nch, coff, bsums, T);
       scan_sums_kernel<<<1, 1024, 0, s>>>(bsums, nblk, coff + T);
       scan_add_kernel<<<nblk, 1024, 0, s>>>(coff, cursor, bsums, T);
-      cudaMemsetAsync(heavy_count, 0, 4, s);
-      const unsigned gf = (unsigned)std::min<uint64_t>((l.chunks + 255) / 256, (uint64_t)sms * 8);
-      ba_fold_kernel<<<gf, 256, 0, s>>>(cnt, joff[last], buf[last], fin, coff, nch, T, chunk_res);
-      ba_bucket_sum_kernel<<<gb, 256, 0, s>>>(coff, nch, chunk_res, buckets, heavy, heavy_count, T);
-      const uint64_t max_heavy = std::min<uint64_t>(T, l.chunks / (BA_TSEQ + 1) + 1);
-      ba_heavy_kernel<<<(unsigned)max_heavy, 256, 0, s>>>(coff, nch, chunk_res, buckets, heavy, heavy_count);
+      cudaMemsetAsync(heavy_count, 0, 8, s);
+      const unsigned gf = (unsigned)std::min<uint64_t>((l.chunks + 255) / 256, (uint64_t)sms * 16);
+      if (l.rounds)
+        ba_fold_kernel<false><<<gf, 256, 0, s>>>(cnt, joff[last], buf[last], nullptr, fin, coff, T, chunk_res);
+      else
+        ba_fold_kernel<true><<<gf, 256, 0, s>>>(counts, offsets, d_bases, list, nullptr, coff, T, chunk_res);
+      ba_bucket_sum_kernel<<<(T + 31) / 32, 128, 0, s>>>(coff, chunk_res, buckets, heavy, heavy_b, heavy_count, T);
+      const unsigned gh = (unsigned)std::min<uint64_t>(l.heavy, (uint64_t)sms * 2);
+      ba_heavy_items_kernel<<<gh, 256, 0, s>>>(coff, chunk_res, heavy, heavy_count);
+      ba_heavy_kernel<<<gh, 256, 0, s>>>(coff, chunk_res, buckets, heavy_b, heavy_count);
       nl += 8;
     }
     {
       ProfScope ps("msm_segment", s, (double)T * 2 * 14, T * 128.0);
-      msm_segment_kernel<<<(segs + 127) / 128, 128, 0, s>>>(buckets, segres, segsum, B, L, segs);
+      msm_segment_kernel<<<(segs + 31) / 32, 128, 0, s>>>(buckets, segres, segsum, B, L, segs);
     }
-    msm_window_kernel<<<W, 256, kWindowSmem, s>>>(segres, segsum, winsum, B / L, L);
+    uint32_t S = B / L, len = L;  // segments per window, buckets per segment
+    fe *it = segres, *is = segsum, *ot = segres + 4ull * segs, *os = segsum + 4ull * segs;
+    for (; S > kGroup; S /= kGroup, len *= kGroup) {
+      msm_group_kernel<<<W * (S / kGroup), 4 * kGroup, 0, s>>>(it, is, ot, os, kGroup, len);
+      std::swap(it, ot);
+      std::swap(is, os);
+      nl++;
+    }
+    msm_group_kernel<<<W, 4 * S, 0, s>>>(it, is, winsum, nullptr, S, len);
     nl += 2;
     e = cudaGetLastError();
     if (!wout && e == cudaSuccess) e = horner_on_host(winsum, W, (uint32_t)p.c, d_out, s);
   }
-  for (void* ptr : {(void*)counts, (void*)offsets, (void*)cursor, (void*)bsums, (void*)list, (void*)cnt,
-                    (void*)cprev, (void*)np, (void*)joff[0], (void*)joff[1], (void*)fin, (void*)buf[0],
-                    (void*)buf[1], (void*)pre, (void*)tot, (void*)tpre, (void*)buckets, (void*)segres, (void*)segsum,
-                    (void*)nch, (void*)heavy, (void*)heavy_count, (void*)chunk_res,
-                    (void*)(wout ? nullptr : winsum)})
-    if (ptr) cudaFreeAsync(ptr, s);
+  if (arena) cudaFreeAsync(arena, s);
   if (launches) *launches = nl;
   return e;
 }
