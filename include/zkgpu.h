@@ -161,8 +161,10 @@ int zkgpu_divide_by_vanishing_dev(int device, uint64_t *d_ext, uint32_t log_n, u
                                   const uint64_t omega_ext[4], void *stream);
 /* d_out_xyz receives the Jacobian sum (12 words, device memory), normalised
  * (Z = Montgomery one, or all zero for the identity); the call stays
- * asynchronous on `stream` (its last, serial step runs on the host as a
- * stream-ordered host function). */
+ * asynchronous on `stream`.  Its last, serial step runs on a thread of the
+ * library, to which the stream's last kernel hands the window sums; if that
+ * thread does not answer within ZKGPU_MSM_HOST_WAIT_US (environment, default
+ * 3000; 0: never asked), and under stream capture, the kernel does the step. */
 int zkgpu_msm_dev(int device, const uint64_t *d_scalars, const uint64_t *d_bases_xy, uint64_t n, uint64_t *d_out_xyz,
                   void *stream);
 /* d_out_xy[i] = k_i * base (affine, Fq Montgomery, (0, 0) for the identity),

@@ -176,6 +176,40 @@ def test_msm_in_bucket_doubling_and_cancellation(zk, oracle, n_pos, n_neg):
     assert np.array_equal(affine_of(zk.msm(s, bases)), want)
 
 
+@pytest.mark.parametrize("n", [1, 300, 5000])
+def test_msm_window_sums_combined_on_the_device(oracle, n):
+    """msm_dev without the host's answer (ZKGPU_MSM_HOST_WAIT_US = 0): the
+    stream's last kernel does the Horner step and the normalisation itself,
+    identity and cancellation included."""
+    import os
+    import subprocess
+    import sys
+    s = oracle.rand_fr(n, 810 + n)
+    pts = oracle.rand_bases(n, 811 + n)
+    code = """
+import sys
+import numpy as np, torch
+import zk_gpu_b200 as zk
+s, b = np.load(sys.argv[1]), np.load(sys.argv[2])
+ds, db = (torch.from_numpy(x.view(np.int64)).cuda() for x in (s, b))
+out = torch.zeros((2, 12), dtype=torch.int64, device="cuda")
+zk.msm_dev(ds, db, out[0])
+zk.msm_dev(torch.zeros_like(ds), db, out[1])
+np.save(sys.argv[3], out.cpu().numpy().view(np.uint64))
+"""
+    import tempfile
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    with tempfile.TemporaryDirectory() as d:
+        files = [os.path.join(d, f) for f in ("s.npy", "b.npy", "o.npy")]
+        np.save(files[0], s)
+        np.save(files[1], pts)
+        env = dict(os.environ, ZKGPU_MSM_HOST_WAIT_US="0")
+        subprocess.run([sys.executable, "-c", code, *files], cwd=root, env=env, check=True, timeout=300)
+        got = np.load(files[2])
+    assert np.array_equal(affine_of(got[0]), oracle.multiexp(s, pts))
+    assert not got[1].any()
+
+
 @pytest.mark.parametrize("n_pos,n_neg", [(1 << 19, 5), (300_000, 300_000), (1 << 20, 0)])
 def test_msm_rounds_doubling_and_cancellation(zk, oracle, n_pos, n_neg):
     """enough entries for the batch-affine rounds, in one bucket per window:

@@ -5,9 +5,8 @@
 #include <vector>
 
 #include "curve.cuh"
-#include "fq_inv.cuh"
-#include "host_field.hpp"
 #include "msm.cuh"
+#include "msm_field.cuh"
 #include "quad.cuh"
 #include "prof.cuh"
 #include "runtime.cuh"
@@ -188,18 +187,6 @@ constexpr uint32_t BA_G = 32;  // task products per inversion
 // Apply blocks: five of 128 threads per SM fit at the 96 registers the kernel
 // needs (MSM of 2^22: 11.95 ms with two of 256, 11.73 ms so).
 constexpr uint32_t BA_APPLY = 128;
-
-// a^-1 for a != 0 in Montgomery form, lazy in, canonical out: the divstep
-// inversion (fq_inv.cuh) of the representative a 2^256 gives a^-1 2^-256,
-// and one product with 2^768 mod q returns it to Montgomery form.
-__device__ __forceinline__ void fq_inv_mont(uint32_t r[8], const uint32_t a[8]) {
-  const uint32_t k768[8] = {0xda1530dfu, 0xb1cd6dafu, 0xa7283db6u, 0x62f210e6u, 0x0ada0afbu, 0xef7f0b0cu, 0x2d592544u, 0x20fd6e90u};
-  uint32_t c[8], t[8];
-  reduce_once<FqP>(c, a);
-  fq_inv_divsteps(t, c);
-  qmul(r, t, k768);
-  reduce_once<FqP>(r, r);
-}
 
 // ---- per-thread copy pipeline ---------------------------------------------
 // The prefix and apply passes are chains of dependent gathers (bucket
@@ -853,55 +840,6 @@ __global__ void zero_out_kernel(fe* out) {
 }
 
 namespace {
-// The Horner step over the window sums (sum_w 2^(c w) W_w, ~250 dependent
-// doublings) is serial: one GPU thread needs over a millisecond for it, the
-// host well under 0.1 ms.  The device-resident call keeps stream order and
-// asynchrony by running it as a host function on the stream: window sums to
-// a pinned slot, host_horner() on the stream, the normalised Jacobian result
-// back to the caller's device buffer.  Slots are per host thread and reused
-// round robin once the event of their last use has completed.
-struct HornerSlot {
-  uint64_t win[MSM_MAX_WINDOWS * 16];
-  uint64_t out[12];
-  uint32_t windows = 0, c = 0;
-  cudaEvent_t done = nullptr;
-};
-constexpr int kHornerSlots = 8;
-struct HornerRing {
-  HornerSlot* slots = nullptr;  // pinned, kHornerSlots entries
-  int next = 0;
-};
-thread_local HornerRing t_horner;
-
-void CUDART_CB host_horner(void* arg) {
-  HornerSlot* h = static_cast<HornerSlot*>(arg);
-  host::fq::msm_combine_windows(h->win, h->windows, h->c, h->out);
-}
-
-cudaError_t horner_on_host(const fe* d_winsum, uint32_t windows, uint32_t c, fe* d_out, cudaStream_t s) {
-  HornerRing& r = t_horner;
-  if (!r.slots) {
-    cudaError_t e = cudaMallocHost((void**)&r.slots, sizeof(HornerSlot) * kHornerSlots);
-    if (e != cudaSuccess) return e;
-    for (int i = 0; i < kHornerSlots; i++) {
-      new (&r.slots[i]) HornerSlot();
-      e = cudaEventCreateWithFlags(&r.slots[i].done, cudaEventDisableTiming);
-      if (e != cudaSuccess) return e;
-    }
-  }
-  HornerSlot* h = &r.slots[r.next];
-  r.next = (r.next + 1) % kHornerSlots;
-  cudaError_t e = cudaEventSynchronize(h->done);  // its last use has finished (normally long ago)
-  if (e != cudaSuccess) return e;
-  h->windows = windows;
-  h->c = c;
-  e = cudaMemcpyAsync(h->win, d_winsum, windows * 128ull, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaLaunchHostFunc(s, host_horner, h);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_out, h->out, 96, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaEventRecord(h->done, s);
-  return e;
-}
-
 // tasks of a round of at most jb pair sums (ba_task_len: K = clamp(J / fill_k, 1, BA_K))
 uint64_t ba_tasks_bound(uint64_t jb, uint64_t fill_k) {
   return std::max<uint64_t>(2 * fill_k, jb / BA_K + 1);
@@ -1179,7 +1117,10 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe*
     msm_group_kernel<<<W, 4 * S, 0, s>>>(it, is, winsum, nullptr, S, len);
     nl += 2;
     e = cudaGetLastError();
-    if (!wout && e == cudaSuccess) e = horner_on_host(winsum, W, (uint32_t)p.c, d_out, s);
+    if (!wout && e == cudaSuccess) {
+      e = msm_combine(winsum, W, (uint32_t)p.c, d_out, s);
+      nl++;
+    }
   }
   if (arena) cudaFreeAsync(arena, s);
   if (launches) *launches = nl;

@@ -38,8 +38,8 @@ int tuned_msm_window(int device, int log_n);
 
 // Enqueue the MSM on `s`; d_out receives the Jacobian sum (X, Y, Z: 12 u64,
 // normalised to Z = one; all zero for the identity), the last step (Horner
-// over the windows) running as a host function on the stream.  Scratch
-// comes from the library pool.
+// over the windows) being handed to the host by the stream's last kernel
+// (msm_combine.cu).  Scratch comes from the library pool.
 // Optional: stop before the last step and leave the per-window sums for the
 // host (host::fq::msm_combine_windows), which does the ~250 dependent
 // doublings of the Horner step far faster than one GPU thread.
@@ -51,6 +51,9 @@ struct MsmWindowsOut {
 constexpr uint32_t MSM_MAX_WINDOWS = 64;  // c >= 4
 cudaError_t msm_run(const fe* d_scalars, const fe* d_bases_xy, uint64_t n, fe* d_out, cudaStream_t s,
                     int c_override = 0, uint64_t* launches = nullptr, MsmWindowsOut* wout = nullptr);
+// The last step on the stream (msm_combine.cu): Horner over `windows` window
+// sums, the normalised Jacobian result to d_out.
+cudaError_t msm_combine(const fe* d_winsum, uint32_t windows, uint32_t c, fe* d_out, cudaStream_t s);
 // Several MSMs over one base array (the serving loop's jobs against resident
 // bases) in one pass: job j's scalars are [off[j], off[j+1]) of d_scalars
 // (d_job_off: jobs + 1 offsets in device memory, off[0] = 0), each against

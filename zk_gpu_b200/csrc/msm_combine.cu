@@ -1,0 +1,282 @@
+// msm_combine.cu — the last step of a device-resident MSM: Horner over the
+// window sums, sum_w 2^(c w) W_w, and the normalisation.
+//
+// The ~250 doublings of this step depend on one another: a GPU thread needs
+// 1.3 ms for them, a host core 70 us.  A host function on the stream
+// (cudaLaunchHostFunc) gives them to the host, but starts 50 us after the work
+// before it when the caller waits and 170-420 us after it when the caller goes
+// on enqueueing (measured on B200 hosts), which was half of a 2^14-point MSM.
+// So the stream's last kernel hands the sums over itself: it writes them to a
+// pinned slot, raises its flag and waits for the answer, which a library thread
+// that watches the slots writes next to them.
+//
+// The wait is bounded (ZKGPU_MSM_HOST_WAIT_US, default 3000): when the host has
+// not answered by then (it is stopped, or overcommitted), the kernel does the
+// step by itself, as it does at once while the stream is being captured into a
+// graph, whose replays have no slot.  Either way the result is the same.
+//
+// Slots are pooled per device, at most kMaxSlots; one is used again when its
+// kernel has finished and the library thread is done with it.
+#include <atomic>
+#include <chrono>
+#include <condition_variable>
+#include <cstdlib>
+#include <cstring>
+#include <memory>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+#include "curve.cuh"
+#include "fq_inv.cuh"
+#include "host_field.hpp"
+#include "msm.cuh"
+#include "msm_field.cuh"
+#include "runtime.cuh"
+
+namespace zk {
+
+namespace {
+
+// pinned, read and written by both sides
+struct Mail {
+  uint32_t ready;  // the kernel's: sequence number of the sums in `win`
+  uint32_t done;   // the host's: sequence number of the answer in `out`
+  uint32_t pad[2];
+  uint64_t win[MSM_MAX_WINDOWS * 16];
+  uint64_t out[12];
+};
+
+__device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release_sys(uint32_t* p, uint32_t v) {
+  asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint64_t now_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+__device__ __noinline__ void combine_here(const fe* winsum, uint32_t windows, uint32_t c, fe* out) {
+  xyzz_t acc, w;
+  ld_xyzz(acc, winsum + 4 * (uint64_t)(windows - 1));
+#pragma unroll 1
+  for (int i = (int)windows - 2; i >= 0; i--) {
+#pragma unroll 1
+    for (uint32_t k = 0; k < c; k++) xyzz_dbl(acc, acc);
+    ld_xyzz(w, winsum + 4 * (uint64_t)i);
+    xyzz_add(acc, w);
+  }
+  aff_t p;
+  uint32_t z[8];
+  set_zero(p.x);
+  set_zero(p.y);
+  set_zero(z);
+  if (!xyzz_is_inf(acc)) {
+    uint32_t t[8];
+    qmul(t, acc.zz, acc.zzz);
+    fq_inv_mont(t, t);
+    qmul(z, t, acc.zzz);  // 1 / ZZ
+    qmul(p.x, acc.x, z);
+    qmul(z, t, acc.zz);   // 1 / ZZZ
+    qmul(p.y, acc.y, z);
+    reduce_once<P_q>(p.x, p.x);
+    reduce_once<P_q>(p.y, p.y);
+    set_one<P_q>(z);
+  }
+  st_fe(out, p.x);
+  st_fe(out + 1, p.y);
+  st_fe(out + 2, z);
+}
+
+__global__ void __launch_bounds__(128) msm_combine_kernel(const fe* winsum, uint32_t windows, uint32_t c, fe* out,
+                                                          Mail* mail, uint32_t seq, uint64_t wait_ns) {
+  if (mail) {
+    __shared__ uint32_t answered;
+    const uint4* src = reinterpret_cast<const uint4*>(winsum);
+    uint4* dst = reinterpret_cast<uint4*>(mail->win);
+    for (uint32_t i = threadIdx.x; i < windows * 8; i += blockDim.x) dst[i] = src[i];
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      st_release_sys(&mail->ready, seq);
+      const uint64_t t0 = now_ns();
+      uint32_t got;
+      while (!(got = ld_acquire_sys(&mail->done) == seq) && now_ns() - t0 < wait_ns) __nanosleep(100);
+      answered = got;
+    }
+    __syncthreads();
+    if (answered) {
+      if (threadIdx.x < 12)
+        reinterpret_cast<uint64_t*>(out)[threadIdx.x] = *(volatile const uint64_t*)&mail->out[threadIdx.x];
+      return;
+    }
+  }
+  if (threadIdx.x == 0) combine_here(winsum, windows, c, out);
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+struct Slot {
+  Mail* mail = nullptr;
+  cudaEvent_t used = nullptr;  // its last kernel has finished
+  uint32_t seq = 0, windows = 0, c = 0;
+  bool taken = false;                  // between acquire and the event record
+  std::atomic<bool> watched{false};    // the library thread has not answered yet
+};
+constexpr size_t kMaxSlots = 64;
+
+// The thread that answers.  It polls while slots are watched (falling back to
+// short sleeps when nothing has come for a while) and sleeps otherwise.
+class Answerer {
+ public:
+  static Answerer& get() {
+    static Answerer* a = new Answerer();  // stopped at exit, never destroyed
+    return *a;
+  }
+  void watch(Slot* s) {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (stop_) {
+      s->watched.store(false);
+      return;
+    }
+    if (!thread_.joinable()) {
+      thread_ = std::thread([this] { run(); });
+      // registered after the CUDA runtime's own handlers, so it runs before
+      // they unmap the slots; kernels still waiting do the step themselves
+      std::atexit([] { get().stop(); });
+    }
+    queue_.push_back(s);
+    queued_.store(true);
+    cv_.notify_one();
+  }
+
+ private:
+  void stop() {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      stop_ = true;
+      queued_.store(true);
+      cv_.notify_one();
+    }
+    if (thread_.joinable()) thread_.join();
+  }
+  void run() {
+    using clk = std::chrono::steady_clock;
+    std::vector<Slot*> watched;
+    clk::time_point last = clk::now();
+    for (;;) {
+      if (queued_.load() || watched.empty()) {
+        std::unique_lock<std::mutex> lk(mu_);
+        cv_.wait(lk, [&] { return stop_ || !queue_.empty() || !watched.empty(); });
+        if (stop_) return;
+        watched.insert(watched.end(), queue_.begin(), queue_.end());
+        queue_.clear();
+        queued_.store(false);
+        last = clk::now();
+      }
+      for (size_t i = 0; i < watched.size();) {
+        Slot* s = watched[i];
+        if (__atomic_load_n(&s->mail->ready, __ATOMIC_ACQUIRE) != s->seq) {
+          i++;
+          continue;
+        }
+        host::fq::msm_combine_windows(s->mail->win, s->windows, s->c, s->mail->out);
+        __atomic_store_n(&s->mail->done, s->seq, __ATOMIC_RELEASE);
+        s->watched.store(false, std::memory_order_release);
+        watched[i] = watched.back();
+        watched.pop_back();
+        last = clk::now();
+      }
+      if (!watched.empty() && clk::now() - last > std::chrono::milliseconds(20))
+        std::this_thread::sleep_for(std::chrono::microseconds(20));
+    }
+  }
+  std::mutex mu_;
+  std::condition_variable cv_;
+  std::vector<Slot*> queue_;
+  std::atomic<bool> queued_{false};
+  bool stop_ = false;
+  std::thread thread_;
+};
+
+std::mutex g_slot_mu;
+std::vector<std::vector<std::unique_ptr<Slot>>> g_slots;  // per device
+
+// A free slot, made if there is none, or null when all kMaxSlots are in use
+// (the caller's kernel then does the step itself) or a new one cannot be had.
+Slot* acquire_slot(int dev) {
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  if ((int)g_slots.size() <= dev) g_slots.resize(dev + 1);
+  auto& pool = g_slots[dev];
+  for (auto& s : pool) {
+    if (s->taken || s->watched.load(std::memory_order_acquire)) continue;
+    const cudaError_t q = cudaEventQuery(s->used);
+    if (q == cudaErrorNotReady) {
+      cudaGetLastError();
+      continue;
+    }
+    if (q != cudaSuccess) return nullptr;
+    s->taken = true;
+    return s.get();
+  }
+  if (pool.size() >= kMaxSlots) return nullptr;
+  auto s = std::make_unique<Slot>();
+  if (cudaMallocHost((void**)&s->mail, sizeof(Mail)) != cudaSuccess ||
+      cudaEventCreateWithFlags(&s->used, cudaEventDisableTiming) != cudaSuccess) {
+    if (s->mail) cudaFreeHost(s->mail);
+    cudaGetLastError();
+    return nullptr;
+  }
+  std::memset(s->mail, 0, sizeof(Mail));
+  s->taken = true;
+  pool.push_back(std::move(s));
+  return pool.back().get();
+}
+
+uint64_t host_wait_ns() {
+  static const uint64_t ns = [] {
+    const char* v = std::getenv("ZKGPU_MSM_HOST_WAIT_US");
+    return (v && *v ? std::strtoull(v, nullptr, 10) : 3000ull) * 1000ull;
+  }();
+  return ns;
+}
+
+}  // namespace
+
+cudaError_t msm_combine(const fe* d_winsum, uint32_t windows, uint32_t c, fe* d_out, cudaStream_t s) {
+  if (windows == 0 || windows > MSM_MAX_WINDOWS) return cudaErrorInvalidValue;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  e = cudaStreamIsCapturing(s, &cap);
+  if (e != cudaSuccess) return e;
+  const uint64_t wait = host_wait_ns();
+  Slot* slot = cap == cudaStreamCaptureStatusNone && wait ? acquire_slot(dev) : nullptr;
+  if (!slot) {
+    msm_combine_kernel<<<1, 128, 0, s>>>(d_winsum, windows, c, d_out, nullptr, 0, 0);
+    return cudaGetLastError();
+  }
+  slot->seq++;
+  slot->windows = windows;
+  slot->c = c;
+  slot->watched.store(true);
+  msm_combine_kernel<<<1, 128, 0, s>>>(d_winsum, windows, c, d_out, slot->mail, slot->seq, wait);
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaEventRecord(slot->used, s);
+  if (e == cudaSuccess)
+    Answerer::get().watch(slot);
+  else
+    slot->watched.store(false);
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  slot->taken = false;
+  return e;
+}
+
+}  // namespace zk
