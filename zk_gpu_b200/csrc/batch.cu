@@ -9,6 +9,7 @@
 // of CTA tiles in one level-ordered work list, and a persistent kernel
 // (ntt_batch_kernel) drains the list; a graph holding {counter reset, kernel}
 // is replayed for each run.
+#include <algorithm>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -105,9 +106,15 @@ extern "C" int zkgpu_ntt_batch_create(int device, const zkgpu_ntt_job* jobs, uin
   std::vector<uint32_t> prev_index(njobs, ~0u);
   uint64_t tiles = 0;
   for (int lvl = 0; lvl < max_pass; lvl++) {
-    for (uint32_t j = 0; j < njobs; j++) {
+    // a level's passes by width, so that the blocks of an SM run the same code
+    std::vector<uint32_t> order;
+    for (uint32_t j = 0; j < njobs; j++)
+      if (lvl < info[j].t->plan.npass) order.push_back(j);
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t c) {
+      return info[a].t->plan.bits[lvl] > info[c].t->plan.bits[lvl];
+    });
+    for (uint32_t j : order) {
       const zk::NttTables& t = *info[j].t;
-      if (lvl >= t.plan.npass) continue;
       zk::BatchPass bp{};
       zk::NttFuse f;
       f.pre = info[j].pre.get();

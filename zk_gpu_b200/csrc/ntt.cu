@@ -69,49 +69,75 @@ __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
   return v;
 }
 
+//
+// A block takes its next item while it still works on the current one, so the
+// atomic's latency is hidden; it waits for nothing but items before its own,
+// so the argument above holds with it (the first unfinished item is always
+// one being worked on).  Warp 0 finds the item's pass by a 32-way search (two
+// or three dependent loads among the passes of 512 transforms; a binary search
+// by one thread took eleven), and the roots stay in shared memory while items
+// of the same pass width and table follow one another.
 __global__ void __launch_bounds__(256, 2) ntt_batch_kernel(const BatchPass* passes, uint32_t npass,
                                                           uint32_t total_tiles, uint32_t* next, uint32_t* done,
                                                           uint32_t* err, uint64_t spin_cycles) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint32_t s_w, s_k, s_stop;
+  uint32_t taken = 0;  // thread 0: the item taken ahead
+  if (threadIdx.x == 0) taken = atomicAdd(next, 1u);
+  const fe* roots = nullptr;  // table in shared memory, its pass width and place
+  uint32_t roots_b = 0, roots_at = 0;
   for (;;) {
-    if (threadIdx.x == 0) {
-      uint32_t w = atomicAdd(next, 1u);
-      s_stop = (w >= total_tiles || ld_acquire_u32(err) != 0) ? 1u : 0u;
-      if (!s_stop) {
+    if (threadIdx.x < 32) {
+      const uint32_t w = __shfl_sync(0xffffffffu, taken, 0);
+      uint32_t lo = 0;
+      if (w < total_tiles) {
         // last pass whose first tile index is <= w
-        uint32_t lo = 0, hi = npass;
-        while (hi - lo > 1) {
-          const uint32_t mid = (lo + hi) / 2;
-          if (passes[mid].tile_base <= w) lo = mid; else hi = mid;
+        uint32_t n = npass;  // it is among [lo, lo + n)
+        while (n > 1) {
+          const uint32_t step = (n + 31) / 32, at = lo + threadIdx.x * step;
+          const bool le = threadIdx.x * step < n && passes[at].tile_base <= w;
+          const uint32_t k = 31 - __clz(__ballot_sync(0xffffffffu, le));  // lane 0 always holds
+          n = min(step, n - k * step);
+          lo += k * step;
         }
-        const BatchPass& bp = passes[lo];
-        if (bp.dep != 0xffffffffu) {
-          const uint64_t t0 = clock64();
-          while (ld_acquire_u32(done + bp.dep) < bp.dep_tiles) {
-            if (clock64() - t0 > spin_cycles) {
-              atomicExch(err, 1u);
-              s_stop = 1;
-              break;
+      }
+      if (threadIdx.x == 0) {
+        s_stop = (w >= total_tiles || ld_acquire_u32(err) != 0) ? 1u : 0u;
+        if (!s_stop) {
+          const BatchPass& bp = passes[lo];
+          if (bp.dep != 0xffffffffu) {
+            const uint64_t t0 = clock64();
+            while (ld_acquire_u32(done + bp.dep) < bp.dep_tiles) {
+              if (clock64() - t0 > spin_cycles) {
+                atomicExch(err, 1u);
+                s_stop = 1;
+                break;
+              }
+              __nanosleep(64);
             }
-            __nanosleep(64);
           }
+          s_w = w;
+          s_k = lo;
         }
-        s_w = w;
-        s_k = lo;
       }
     }
     __syncthreads();
     if (s_stop) return;
+    if (threadIdx.x == 0) taken = atomicAdd(next, 1u);
     const BatchPass& bp = passes[s_k];
     const uint64_t tile = s_w - bp.tile_base;
+    const uint32_t at = bp.p.ntile * bp.p.G;
+    const bool have = bp.p.inner == roots && bp.B == roots_b && at == roots_at;
+    roots = bp.p.inner;
+    roots_b = bp.B;
+    roots_at = at;
     switch (bp.B) {
-      case 3: ntt_pass_tile<3, true>(bp.p, nullptr, tile, smem); break;
-      case 4: ntt_pass_tile<4, true>(bp.p, nullptr, tile, smem); break;
-      case 5: ntt_pass_tile<5, true>(bp.p, nullptr, tile, smem); break;
-      case 6: ntt_pass_tile<6, true>(bp.p, nullptr, tile, smem); break;
-      case 7: ntt_pass_tile<7, true>(bp.p, nullptr, tile, smem); break;
-      case 8: ntt_pass_tile<8, true>(bp.p, nullptr, tile, smem); break;
+      case 3: ntt_pass_tile<3, true>(bp.p, nullptr, tile, smem, have); break;
+      case 4: ntt_pass_tile<4, true>(bp.p, nullptr, tile, smem, have); break;
+      case 5: ntt_pass_tile<5, true>(bp.p, nullptr, tile, smem, have); break;
+      case 6: ntt_pass_tile<6, true>(bp.p, nullptr, tile, smem, have); break;
+      case 7: ntt_pass_tile<7, true>(bp.p, nullptr, tile, smem, have); break;
+      case 8: ntt_pass_tile<8, true>(bp.p, nullptr, tile, smem, have); break;
       case 9: ntt_pass_tile<9, true>(bp.p, nullptr, tile, smem); break;
       case 10: ntt_pass_tile<10, true>(bp.p, nullptr, tile, smem); break;
       case 11: ntt_pass_tile<11, true>(bp.p, nullptr, tile, smem); break;
@@ -200,10 +226,18 @@ __global__ void roots_w4_kernel(fe* out, fe wm, const Special special, const Tab
   if (e < 3) {
     cpy(v, special.v[e].w);
   } else {
-    int lo = B - 3, at = 3;
-    while (e >= at + (7 << lo)) at += 7 << lo, lo -= 3;
+    // the round's lowest bit, its first entry, and log2 of its size below m
+    int lo = B - B % 3, at = 3, up = 0;
+    if (e < at + tw_first(B)) {
+      up = 0;
+    } else {
+      at += tw_first(B);
+      lo -= 3;
+      while (e >= at + (7 << lo)) at += 7 << lo, lo -= 3;
+      up = B - 3 - lo;
+    }
     const uint32_t f = (uint32_t)((e - at) >> lo) + 1, low = (uint32_t)(e - at) & ((1u << lo) - 1u);
-    pow_u64<P_r>(v, wm.w, (uint64_t)(f * low) << (B - 3 - lo));
+    pow_u64<P_r>(v, wm.w, (uint64_t)(f * low) << up);
   }
   mul<P_r>(v, v, sc.w4[i & 3].w);
   st_fe(out + i, v);

@@ -53,6 +53,11 @@ __device__ __forceinline__ void st_smem_fe(uint32_t* plane0, uint32_t plane_stri
 //    for E_1 = (w + w^3) / 2 (t_1 + t_3), E_2 = (w - w^3) / 2 (t_1 - t_3);
 //  * eight twiddle-free stages and seven products by f, low instead of twelve
 //    butterflies with a product each: 11 products per 8 elements and 3 bits;
+//  * the bits that do not make up a round of three come first, as a radix-2 or
+//    radix-4 round (4 or 8 products per 8 elements), so that the last round,
+//    which has no twiddles, is always a whole one: B = 7 takes 19 products,
+//    with the short round last 22 (2^21 as 7+7+7: 354 -> 338 us, 2^24 as 8+8+8:
+//    2674 -> 2586);
 //  * every multiplicand is known beforehand, so each product is a mul_w4 over
 //    a table in shared memory (about 390 cycles against mul_lazy's 555).
 //  * the DFT's three constants are the same for the whole pass: the per-pass
@@ -60,9 +65,10 @@ __device__ __forceinline__ void st_smem_fe(uint32_t* plane0, uint32_t plane_stri
 //    no loads).
 // Forward NTT of 2^24 (8+8+8) on B200: 4320 us with a mul_lazy in each radix-2
 // butterfly, 2685 us in this form; the multiply pipe is then busy for 73 % of a
-// pass (ncu, sm__pipe_fmaheavy_cycles_active).  The per-pass kernels inline every
-// product; the batch kernel, which holds all pass widths, calls one out of
-// line, as its dozens of copies would miss the instruction cache.
+// pass (ncu, sm__pipe_fmaheavy_cycles_active).  Every product is inlined; the
+// batch kernel, which holds all pass widths, orders its work by width so that
+// the blocks of an SM run the same code (512 transforms of 2^10..2^20: 20.0 ms
+// with one product called out of line, 18.0 ms inlined).
 //
 // Ranges, with 1 for p (1 + 2^-29), the bound of a mul_w4 result: inputs <= 1;
 // a difference gets the multiple of p that keeps it positive, and a sum that
@@ -70,16 +76,19 @@ __device__ __forceinline__ void st_smem_fe(uint32_t* plane0, uint32_t plane_stri
 // ---------------------------------------------------------------------------
 constexpr int kNarrowMax = 8;  // widest pass of this form: its tables take 32 KiB of shared memory
 
-// twiddle table of a pass: I = w_4, (w_8 + w_8^3) / 2, (w_8 - w_8^3) / 2, then
-// per round with LO > 0 the roots w_(8 2^LO)^(f low) at [(f - 1) 2^LO + low]
+// Twiddle table of a pass: I = w_4, (w_8 + w_8^3) / 2, (w_8 - w_8^3) / 2; then
+// the short first round's, if there is one (B mod 3 = F bits): the roots
+// w_m^(f low), 1 <= f < 2^F, low < 2^(B - F), at [(f - 1) 2^(B - F) + low]; then
+// per later round with LO > 0 w_(8 2^LO)^(f low) at [(f - 1) 2^LO + low].
+__host__ __device__ constexpr int tw_first(int B) { return ((1 << B % 3) - 1) << (B - B % 3); }
 __host__ __device__ constexpr int tw_entries(int B) {
-  int n = 3;
-  for (int lo = B - 3; lo > 0; lo -= 3) n += 7 << lo;
+  int n = 3 + tw_first(B);
+  for (int lo = B - B % 3 - 3; lo > 0; lo -= 3) n += 7 << lo;
   return n;
 }
 __host__ __device__ constexpr int tw_offset(int B, int LO) {
-  int n = 3;
-  for (int lo = B - 3; lo > LO; lo -= 3) n += 7 << lo;
+  int n = 3 + tw_first(B);
+  for (int lo = B - B % 3 - 3; lo > LO; lo -= 3) n += 7 << lo;
   return n;
 }
 
@@ -98,25 +107,10 @@ struct SmemW4 {  // entry at `addr` of a table stored as eight planes of 16 byte
     lds_v4(v + 4, addr + (2 * k + 1) * plane);
   }
 };
-template <class P>
-__device__ __noinline__ Fe8 mul_w4_call(const Fe8 a, uint32_t addr, uint32_t plane) {
-  Fe8 r;
-  mul_w4<P>(r.w, a.w, SmemW4{addr, plane});
-  return r;
-}
 // r = a times table entry e
-template <int B, bool INLINE = false>
+template <int B>
 __device__ __forceinline__ void tw_mul(uint32_t r[8], const uint32_t a[8], uint32_t tab, uint32_t e) {
-  if constexpr (INLINE) {
-    mul_w4<P_r>(r, a, SmemW4{tab + 16 * e, 16 * tw_entries(B)});
-    return;
-  }
-  Fe8 av;
-#pragma unroll
-  for (int k = 0; k < 8; k++) av.w[k] = a[k];
-  const Fe8 rv = mul_w4_call<P_r>(av, tab + 16 * e, 16 * tw_entries(B));
-#pragma unroll
-  for (int k = 0; k < 8; k++) r[k] = rv.w[k];
+  mul_w4<P_r>(r, a, SmemW4{tab + 16 * e, 16 * tw_entries(B)});
 }
 
 struct ParamC8 {
@@ -180,46 +174,63 @@ __device__ __forceinline__ void dft8(uint32_t x[8][8], const C& c) {
   add_raw(x[2], s0, s1);              // 0 .. 4
   sub_off<P_r, 2>(x[3], s0, s1);      // 1 .. 5
 }
-// 4-point DFT of x[0..3], position r <- output rev2(r); outputs <= 5
+// 4-point DFT of a, b, c, d (positions 0..3), position r <- output rev2(r);
+// inputs <= 1, outputs <= 5, the first <= 4
 template <class C>
-__device__ __forceinline__ void dft4(uint32_t x[4][8], const C& c) {
+__device__ __forceinline__ void dft4(uint32_t x0[8], uint32_t x1[8], uint32_t x2[8], uint32_t x3[8], const C& c) {
   uint32_t s0[8], s1[8], d[8];
-  sub_off<P_r, 2>(d, x[1], x[3]);
+  sub_off<P_r, 2>(d, x1, x3);
   c.mul(d, d, 0);
-  add_raw(s0, x[0], x[2]);
-  add_raw(s1, x[1], x[3]);
-  sub_off<P_r, 2>(x[0], x[0], x[2]);
-  add_raw(x[2], x[0], d);             // 1 .. 4
-  sub_off<P_r, 2>(x[3], x[0], d);     // 2 .. 5
-  add_raw(x[0], s0, s1);
-  sub_off<P_r, 3>(x[1], s0, s1);      // 1 .. 5
+  add_raw(s0, x0, x2);
+  add_raw(s1, x1, x3);
+  sub_off<P_r, 2>(x0, x0, x2);
+  add_raw(x2, x0, d);             // 1 .. 4
+  sub_off<P_r, 2>(x3, x0, d);     // 2 .. 5
+  add_raw(x0, s0, s1);
+  sub_off<P_r, 3>(x1, s0, s1);    // 1 .. 5
 }
 
-template <int B, int LO, int HI, bool INLINE, class C>
-__device__ __forceinline__ void narrow_round(uint32_t x[8][8], uint32_t q, uint32_t tab, const C& c) {
-  if constexpr (HI - LO == 3) {
-    dft8(x, c);
-  } else if constexpr (HI - LO == 2) {
-    dft4(x, c);
-    dft4(x + 4, c);
+// The short first round (F = 1 or 2 bits): the thread holds the column's top
+// three bits, x[r] at r 2^(B - 3) + q.
+template <int B, class C>
+__device__ __forceinline__ void short_round(uint32_t x[8][8], uint32_t q, uint32_t tab, const C& c) {
+  constexpr int F = B % 3;
+  if constexpr (F == 1) {
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      uint32_t t[8];
+      sub_off<P_r, 2>(t, x[r], x[r + 4]);
+      add_raw(x[r], x[r], x[r + 4]);
+      cond_sub<P_r, 1>(x[r]);
+      tw_mul<B>(x[r + 4], t, tab, 3 + (r << (B - 3)) + q);
+    }
   } else {
 #pragma unroll
-    for (int r = 0; r < 8; r += 2) {
-      uint32_t t[8];
-      sub_off<P_r, 2>(t, x[r], x[r + 1]);
-      add_raw(x[r], x[r], x[r + 1]);
-      cpy(x[r + 1], t);
+    for (int h = 0; h < 2; h++) {  // elements h, h + 2, h + 4, h + 6
+      dft4(x[h], x[h + 2], x[h + 4], x[h + 6], c);
+      cond_sub<P_r, 2>(x[h]);
+      cond_sub<P_r, 1>(x[h]);
+      const uint32_t low = (h << (B - 3)) + q;
+#pragma unroll
+      for (int r = 1; r < 4; r++) {  // position r <- output rev2(r)
+        const uint32_t f = (uint32_t)((r & 1) << 1 | r >> 1);
+        tw_mul<B>(x[h + 2 * r], x[h + 2 * r], tab, 3 + ((f - 1) << (B - 2)) + low);
+      }
     }
   }
+}
+
+template <int B, int LO, class C>
+__device__ __forceinline__ void narrow_round(uint32_t x[8][8], uint32_t q, uint32_t tab, const C& c) {
+  dft8(x, c);
   if constexpr (LO > 0) {
-    static_assert(HI - LO == 3, "only the last round has fewer than three bits");
     const uint32_t low = q & ((1u << LO) - 1u);
     cond_sub<P_r, 2>(x[0]);
     cond_sub<P_r, 1>(x[0]);
 #pragma unroll
     for (int r = 1; r < 8; r++) {
       const uint32_t f = (uint32_t)((r & 1) << 2 | (r & 2) | r >> 2);
-      tw_mul<B, INLINE>(x[r], x[r], tab, tw_offset(B, LO) + ((f - 1) << LO) + low);
+      tw_mul<B>(x[r], x[r], tab, tw_offset(B, LO) + ((f - 1) << LO) + low);
     }
   }
 }
@@ -331,28 +342,40 @@ __device__ __forceinline__ void twist_fetch(const PassParams& p, int B, const Ti
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
+// Rounds from index bit HI down.  Narrow passes: a short round if HI = B is no
+// multiple of three, then rounds of three bits; wide ones: rounds of three bits
+// from the top, the last taking what is left.
 template <int B, int HI, bool BATCH>
 __device__ __forceinline__ void ntt_rounds(const PassParams& p, const DftConsts* dft, uint32_t x[8][8],
                                            TilePos pos, uint32_t col,
                                            uint32_t* sm, uint32_t plane_stride, const uint4* tws) {
-  constexpr int LO = HI - 3 > 0 ? HI - 3 : 0;
+  constexpr bool NARROW = B <= kNarrowMax, SHORT = NARROW && HI % 3 != 0;
+  constexpr int LO = SHORT ? B - B % 3 : HI - 3 > 0 ? HI - 3 : 0;  // lowest bit of this round
+  constexpr int MAP = SHORT ? B - 3 : LO;                          // lowest bit the thread holds
   if constexpr (LO == 0) {
     if (!p.is_final) {
 #pragma unroll
       for (int r = 0; r < 4; r++) twist_fetch(p, B, pos, col, (uint32_t)__cvta_generic_to_shared(sm), r);
     }
   }
-  if constexpr (B <= kNarrowMax) {
+  if constexpr (NARROW) {
     const uint32_t tab = (uint32_t)__cvta_generic_to_shared(tws);
+    auto round = [&](const auto& c) {
+      if constexpr (SHORT)
+        short_round<B>(x, pos.q, tab, c);
+      else
+        narrow_round<B, LO>(x, pos.q, tab, c);
+    };
     if constexpr (BATCH)
-      narrow_round<B, LO, HI, false>(x, pos.q, tab, SmemC4<B>{tab});
+      round(SmemC4<B>{tab});
     else
-      narrow_round<B, LO, HI, true>(x, pos.q, tab, ParamC8{*dft});
-  } else
+      round(ParamC8{*dft});
+  } else {
     ntt_round<B, LO, HI>(x, pos.q, tws);
+  }
   if constexpr (LO > 0) {
     constexpr int LO_N = LO - 3 > 0 ? LO - 3 : 0;
-    ntt_exchange<B, LO, LO_N>(x, pos, sm, plane_stride);
+    ntt_exchange<B, MAP, LO_N>(x, pos, sm, plane_stride);
     // what follows depends on the thread's position through this copy: the
     // addresses of later phases are not computed ahead and kept (spills)
     asm volatile("" : "+r"(pos.q), "+r"(col));
@@ -360,14 +383,9 @@ __device__ __forceinline__ void ntt_rounds(const PassParams& p, const DftConsts*
   }
 }
 
-
-// One CTA tile of one pass.  `tile` plays the role of the block index.  In
-// BATCH mode the CTA may be wider than the tile (G * T threads are active,
-// the rest only join the barriers) and data is read through L2 only, since
-// other CTAs of the same launch produced it.
 template <int B, bool BATCH>
 __device__ __forceinline__ void ntt_pass_tile(const PassParams& p, const DftConsts* dft, uint64_t tile,
-                                              uint32_t* smem) {
+                                              uint32_t* smem, bool have_roots = false) {
   constexpr uint32_t M = 1u << B;
   constexpr uint32_t T = M / 8;  // threads per column
   const uint32_t G = p.G;
@@ -385,7 +403,8 @@ __device__ __forceinline__ void ntt_pass_tile(const PassParams& p, const DftCons
   if constexpr (B <= kNarrowMax) {
     constexpr uint32_t N = tw_entries(B);
     const uint4* src = reinterpret_cast<const uint4*>(p.inner);
-    for (uint32_t e = tid; e < 8 * N; e += blockDim.x) tws[(e & 7) * N + (e >> 3)] = __ldg(src + e);
+    if (!have_roots)
+      for (uint32_t e = tid; e < 8 * N; e += blockDim.x) tws[(e & 7) * N + (e >> 3)] = __ldg(src + e);
   } else {
     for (uint32_t e = tid; e < M / 2; e += blockDim.x) {
       uint32_t w[8];
