@@ -221,10 +221,12 @@ struct Special {
 __global__ void roots_w4_kernel(fe* out, fe wm, const Special special, const TableScale sc, int B) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const int e = (int)(i >> 2);
-  if (e >= tw_entries(B)) return;
+  if (e >= roots_entries(B)) return;
   uint32_t v[8];
   if (e < 3) {
     cpy(v, special.v[e].w);
+  } else if (e >= tw_entries(B)) {
+    pow_u64<P_r>(v, wm.w, (uint64_t)(e - tw_entries(B)));
   } else {
     // the round's lowest bit, its first entry, and log2 of its size below m
     int lo = B - B % 3, at = 3, up = 0;
@@ -333,7 +335,7 @@ void pow_tables_free(PowTables* t, cudaStream_t s) {
 }
 
 // elements of a pass's root table, and its launch
-static uint64_t inner_elems(int B) { return B <= kNarrowMax ? 4ull * tw_entries(B) : 1ull << (B - 1); }
+static uint64_t inner_elems(int B) { return B <= kNarrowMax ? 4ull * roots_entries(B) : 1ull << (B - 1); }
 static void fill_inner(fe* out, DftConsts* dft, const host::Fr& wm, int B, cudaStream_t s) {
   const unsigned count = (unsigned)inner_elems(B), grid = (count + 255) / 256;
   if (B > kNarrowMax) {
@@ -477,6 +479,24 @@ void ntt_tables_release(NttTables* t) {
 static uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* out,
                                 bool batch);
 
+// Largest transform whose passes run two elements per thread (ntt_tile.cuh):
+// above it the tile kernel fills the GPU.  B200, pair / tile kernel (us): 2^10
+// 19.5 / 22.8 (both near the host's time to enqueue a call), 2^14 15.3 / 33.0,
+// 2^16 26.9 / 35.8, 2^17 47.1 / 41.2, 2^18 84 / 58.
+constexpr int kPairMaxLog = 16;
+
+static cudaError_t dispatch_pair(int B, const PassParams& pp, int log_n, cudaStream_t s) {
+  switch (B) {
+    case 3: return launch_pair<3>(pp, log_n, s);
+    case 4: return launch_pair<4>(pp, log_n, s);
+    case 5: return launch_pair<5>(pp, log_n, s);
+    case 6: return launch_pair<6>(pp, log_n, s);
+    case 7: return launch_pair<7>(pp, log_n, s);
+    case 8: return launch_pair<8>(pp, log_n, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 static cudaError_t dispatch_pass(int B, const PassParams& pp, const DftConsts& dft, uint64_t ncta, cudaStream_t s) {
   switch (B) {
     case 3: return launch_pass<3>(pp, dft, ncta, s);
@@ -598,7 +618,8 @@ cudaError_t ntt_run(const NttTables& t, fe* d_a, fe* d_tmp, const NttFuse& f, cu
     const double nel = (double)(1ull << L);
     // algorithmic work: radix-2 convention (n/2) * b products; bytes: read + write (+ twist table)
     ProfScope prof(names[b], s, nel / 2 * b, nel * 32.0 * (pp.is_final ? 2 : 4));
-    cudaError_t e = dispatch_pass(b, pp, t.dft[k], ncta, s);
+    const bool small = L <= kPairMaxLog && b <= kNarrowMax;
+    cudaError_t e = small ? dispatch_pair(b, pp, L, s) : dispatch_pass(b, pp, t.dft[k], ncta, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

@@ -342,6 +342,65 @@ __device__ __forceinline__ void twist_fetch(const PassParams& p, int B, const Ti
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
+// The first output index of the last pass's column o, its mixed-radix digits
+// reversed: o = k_1 2^(b_2+..) + ... + k_(p-1) gives k_1 + 2^b_1 k_2 + ...;
+// total = their bits
+__device__ __forceinline__ uint32_t rev_digits(const PassParams& p, uint32_t o, uint32_t& total) {
+  uint32_t rev = 0, low_bits = 0;
+  total = 0;
+#pragma unroll
+  for (int t = 0; t < NTT_MAX_PASS; t++)
+    if (t < (int)p.nprev) total += p.prev_bits[t];
+  uint32_t above = total;
+#pragma unroll
+  for (int t = 0; t < NTT_MAX_PASS; t++) {
+    if (t < (int)p.nprev) {
+      above -= p.prev_bits[t];
+      const uint32_t digit = o >> above;
+      o &= (1u << above) - 1u;
+      rev |= digit << low_bits;
+      low_bits += p.prev_bits[t];
+    }
+  }
+  return rev;
+}
+// input element xi of the first pass, scaled by its coset power or, as the
+// caller gave it (taken up to 2p), below p
+__device__ __forceinline__ void prepare_first(const PassParams& p, uint32_t x[8], uint32_t xi) {
+  if (p.pre_lo) {
+    uint32_t a[8], b[8];
+    ld_fe_nc(a, p.pre_lo + (xi & ((1u << p.pre_shift) - 1u)));
+    ld_fe_nc(b, p.pre_hi + (xi >> p.pre_shift));
+    mul_out<P_r>(a, a, b);
+    mul_out<P_r>(x, a, x);  // < 3p for any input
+    cond_sub<P_r, 2>(x);
+  }
+  cond_sub<P_r, 1>(x);
+}
+// output kout, scaled and made canonical; WIDE_RANGE: x is below 5p, else 2p
+template <bool WIDE_RANGE>
+__device__ __forceinline__ void store_final(const PassParams& p, const uint32_t x[8], uint32_t kout) {
+  uint32_t v[8];
+  if (p.post_lo) {
+    uint32_t a[8], b[8];
+    ld_fe_nc(a, p.post_lo + (kout & ((1u << p.post_shift) - 1u)));
+    ld_fe_nc(b, p.post_hi + (kout >> p.post_shift));
+    mul_out<P_r>(a, a, b);
+    mul_out<P_r>(v, a, x);  // < 3p
+    cond_sub<P_r, 2>(v);
+  } else if (p.has_post) {
+    mul_out<P_r>(v, p.post.w, x);  // < 2p
+  } else {
+    cpy(v, x);
+    if (WIDE_RANGE) {
+      cond_sub<P_r, 4>(v);
+      cond_sub<P_r, 2>(v);
+    }
+  }
+  cond_sub<P_r, 1>(v);
+  st_fe(p.out + kout, v);
+}
+
 // Rounds from index bit HI down.  Narrow passes: a short round if HI = B is no
 // multiple of three, then rounds of three bits; wide ones: rounds of three bits
 // from the top, the last taking what is left.
@@ -451,22 +510,9 @@ __device__ __forceinline__ void ntt_pass_tile(const PassParams& p, const DftCons
     for (int r = 0; r < 8; r++) set_zero(x[r]);
   }
 
-  if (p.pre_lo && active) {
-    const uint32_t mask = (1u << p.pre_shift) - 1u;
+  if (p.is_first && active) {
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const uint32_t xi = base + (q + T * r) * stride;  // first pass: global input index
-      uint32_t a[8], b[8];
-      ld_fe_nc(a, p.pre_lo + (xi & mask));
-      ld_fe_nc(b, p.pre_hi + (xi >> p.pre_shift));
-      mul_out<P_r>(a, a, b);
-      mul_out<P_r>(x[r], a, x[r]);  // < 3p for any input
-      cond_sub<P_r, 2>(x[r]);
-      cond_sub<P_r, 1>(x[r]);
-    }
-  } else if (p.is_first) {  // the caller's values, taken up to 2p
-#pragma unroll
-    for (int r = 0; r < 8; r++) cond_sub<P_r, 1>(x[r]);
+    for (int r = 0; r < 8; r++) prepare_first(p, x[r], base + (q + T * r) * stride);
   }
   __syncthreads();
 
@@ -493,48 +539,12 @@ __device__ __forceinline__ void ntt_pass_tile(const PassParams& p, const DftCons
       st_fe(p.out + ((o << B << p.log_J) + twist_index(p, B, q, col, r)), x[r]);
     }
   } else {
-    // rev(o): o = k_1 * 2^(b_2+..) + ... + k_(p-1);  rev = k_1 + 2^b_1 k_2 + ...
-    uint32_t rev = 0, rem = o;
-    uint32_t low_bits = 0, total = 0;
-#pragma unroll
-    for (int t = 0; t < NTT_MAX_PASS; t++)
-      if (t < (int)p.nprev) total += p.prev_bits[t];
-    uint32_t above = total;
-#pragma unroll
-    for (int t = 0; t < NTT_MAX_PASS; t++) {
-      if (t < (int)p.nprev) {
-        above -= p.prev_bits[t];
-        const uint32_t digit = rem >> above;
-        rem &= (1u << above) - 1u;
-        rev |= digit << low_bits;
-        low_bits += p.prev_bits[t];
-      }
-    }
+    uint32_t total;
+    const uint32_t rev = rev_digits(p, o, total);
 #pragma unroll
     for (int r = 0; r < 8; r++) {
       const uint32_t k = __brev(8 * q + r) >> (32 - B);
-      uint32_t v[8];
-      const uint32_t kout = rev + (k << total);  // natural output index
-      if (p.post_lo) {
-        uint32_t a[8], b[8];
-        ld_fe_nc(a, p.post_lo + (kout & ((1u << p.post_shift) - 1u)));
-        ld_fe_nc(b, p.post_hi + (kout >> p.post_shift));
-        mul_out<P_r>(a, a, b);
-        mul_out<P_r>(v, a, x[r]);  // < 3p
-        cond_sub<P_r, 2>(v);
-        cond_sub<P_r, 1>(v);
-      } else if (p.has_post) {
-        mul_out<P_r>(v, p.post.w, x[r]);  // < 2p
-        cond_sub<P_r, 1>(v);
-      } else {  // the rounds leave up to 5 p
-        cpy(v, x[r]);
-        if constexpr (B <= kNarrowMax) {
-          cond_sub<P_r, 4>(v);
-          cond_sub<P_r, 2>(v);
-        }
-        cond_sub<P_r, 1>(v);
-      }
-      st_fe(p.out + kout, v);
+      store_final<(B <= kNarrowMax)>(p, x[r], rev + (k << total));
     }
   }
 }
@@ -543,6 +553,131 @@ template <int B>
 __global__ void __launch_bounds__(256, 2) ntt_pass_kernel(const PassParams p, const DftConsts dft) {
   extern __shared__ __align__(16) uint32_t smem[];
   ntt_pass_tile<B, false>(p, &dft, blockIdx.x, smem);
+}
+
+// ---------------------------------------------------------------------------
+// Passes of small transforms.  A tile's thread runs the products of its eight
+// elements one after the other (some 20 per pass, 0.3 us each when the SM has
+// nothing else), and a small transform leaves most SMs without a tile.  Here a
+// thread holds two elements: a radix-2 stage costs it one product, stages
+// exchange one element between the lanes of a warp by shuffles (between warps
+// through shared memory where a column has more than 64 elements), and the
+// next stage's root is loaded while the product runs.  That is as much work in
+// all (B - 1 products per two elements) on four times the threads, with
+// 4 to 7 us per pass (2^10, 2^13) instead of 9 to 17.  Roots: w_m^e, e < m / 2, after the
+// entries of the tile kernel's rounds.
+// ---------------------------------------------------------------------------
+__host__ __device__ constexpr int roots_entries(int B) { return tw_entries(B) + (1 << (B - 1)); }
+
+struct W4Regs {
+  uint32_t w[4][8];
+  __device__ __forceinline__ void load(const fe* entry) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) ld_fe_nc(w[k], entry + k);
+  }
+  __device__ __forceinline__ void operator()(int k, uint32_t v[8]) const { cpy(v, w[k]); }
+};
+
+// stages b .. 0 of a column: thread q of 2^(B - 1) holds the elements whose
+// index has bit b clear and set and its other bits from q
+template <int B, int b>
+__device__ __forceinline__ void pair_stages(uint32_t x0[8], uint32_t x1[8], uint32_t q, const fe* roots,
+                                            const W4Regs& w, uint32_t* sm, unsigned mask) {
+  uint32_t d[8];
+  sub_off<P_r, 2>(d, x0, x1);
+  add_raw(x0, x0, x1);
+  if constexpr (b == 0) {
+    cpy(x1, d);  // <= 2 and <= 3
+  } else {
+    W4Regs next;
+    if constexpr (b > 1) next.load(roots + 4 * ((q & ((1u << (b - 1)) - 1u)) << (B - b)));
+    cond_sub<P_r, 1>(x0);
+    mul_w4<P_r>(x1, d, w);
+    // the lane whose bit b - 1 is clear keeps x0 and gets the other's x0
+    const bool up = (q >> (b - 1)) & 1u;
+    uint32_t s[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) s[k] = up ? x0[k] : x1[k];
+    if constexpr (b - 1 < 5) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) s[k] = __shfl_xor_sync(mask, s[k], 1 << (b - 1));
+    } else {
+      constexpr uint32_t T = 1u << (B - 1);
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 8; k++) sm[k * T + q] = s[k];
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 8; k++) s[k] = sm[k * T + (q ^ (1u << (b - 1)))];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      x0[k] = up ? s[k] : x0[k];
+      x1[k] = up ? x1[k] : s[k];
+    }
+    pair_stages<B, b - 1>(x0, x1, q, roots, next, sm, mask);
+  }
+}
+
+// One column per 2^(B - 1) threads; a block of more than 32 threads is one column.
+template <int B>
+__global__ void __launch_bounds__(B > 6 ? 1 << (B - 1) : 32) ntt_pair_kernel(const PassParams p) {
+  constexpr uint32_t T = 1u << (B - 1), M = 1u << B;
+  __shared__ uint32_t sm[B > 6 ? 8 * T : 1];
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t c = t >> (B - 1), q = t & (T - 1);
+  const unsigned mask = blockDim.x < 32 ? (1u << blockDim.x) - 1u : 0xffffffffu;
+  uint32_t o = c, col = 0, base = c << B, stride = 1;
+  if (!p.is_final) {
+    o = c >> p.log_J;
+    col = c & ((1u << p.log_J) - 1u);
+    base = (o << B << p.log_J) + col;
+    stride = 1u << p.log_J;
+  }
+  const fe* roots = p.inner + 4 * tw_entries(B);
+  W4Regs w;
+  w.load(roots + 4 * q);
+  uint32_t x0[8], x1[8];
+  const uint32_t rows = p.in_rows ? p.in_rows : M;
+  set_zero(x0);
+  set_zero(x1);
+  if (q < rows) ld_fe(x0, p.in + (base + q * stride));
+  if (q + T < rows) ld_fe(x1, p.in + (base + (q + T) * stride));
+  if (p.is_first) {
+    prepare_first(p, x0, base + q * stride);
+    prepare_first(p, x1, base + (q + T) * stride);
+  }
+  // where the outputs go: positions 2 q and 2 q + 1 hold outputs bitrev
+  const uint32_t k0 = __brev(2 * q) >> (32 - B), k1 = k0 + M / 2;
+  uint32_t v[2][2][8];
+  if (!p.is_final) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const fe* tw = p.twist + 2 * (size_t)(((h ? k1 : k0) << p.log_J) + col);
+      ld_fe_nc(v[h][0], tw);
+      ld_fe_nc(v[h][1], tw + 1);
+    }
+  }
+  pair_stages<B, B - 1>(x0, x1, q, roots, w, sm, mask);
+  if (!p.is_final) {
+    mul_w2<P_r>(x0, x0, v[0][0], v[0][1]);
+    mul_w2<P_r>(x1, x1, v[1][0], v[1][1]);
+    fe* out = p.out + (o << B << p.log_J) + col;
+    st_fe(out + (k0 << p.log_J), x0);
+    st_fe(out + (k1 << p.log_J), x1);
+  } else {
+    uint32_t total;
+    const uint32_t rev = rev_digits(p, o, total);
+    store_final<true>(p, x0, rev + (k0 << total));
+    store_final<true>(p, x1, rev + (k1 << total));
+  }
+}
+template <int B>
+inline cudaError_t launch_pair(const PassParams& pp, int log_n, cudaStream_t s) {
+  const unsigned threads = 1u << (log_n - 1);
+  const unsigned block = threads < 32 ? threads : (B > 6 ? 1u << (B - 1) : 32u);
+  ntt_pair_kernel<B><<<threads / block, block, 0, s>>>(pp);
+  return cudaGetLastError();
 }
 
 template <int B>
