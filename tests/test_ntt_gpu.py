@@ -217,3 +217,24 @@ def test_extreme_values(zk, oracle, log_n):
         assert np.array_equal(zk.ifft(a, wi, log_n, d), oracle.ifft(a, wi, log_n, d))
         c = oracle.from_int(B.R_MOD - 1)
         assert np.array_equal(zk.coset_fft(a, w, log_n, c), oracle.best_fft(oracle.distribute_powers(a, c), w, log_n))
+
+
+@pytest.mark.parametrize("log_ext,m", [(2, 1), (3, 5), (8, 1), (9, 511), (16, 40001), (17, 1), (20, (1 << 20) - 1)])
+def test_extended_to_coeff_writes_the_wanted_outputs_only(zk, oracle, log_ext, m):
+    """the first m coefficients, nothing beyond them; also with the output over the input"""
+    torch = pytest.importorskip("torch")
+    ext = oracle.rand_fr(1 << log_ext, 90 + log_ext)
+    ext[0], ext[-1] = oracle.from_int(B.R_MOD - 1), 0
+    w_inv, d = oracle.inv(oracle.omega(log_ext)), inv_n(oracle, log_ext)
+    g_inv = oracle.inv(oracle.to_mont(7))
+    ref = oracle.extended_to_coeff(ext, log_ext, m, w_inv, d, g_inv)
+    d_ext = torch.from_numpy(ext.view(np.int64)).cuda()
+    out = torch.full((m + 64, 4), -1, dtype=torch.int64, device="cuda")
+    zk.extended_to_coeff_dev(d_ext, out[:m], log_ext, w_inv, d, g_inv)
+    torch.cuda.synchronize()
+    assert np.array_equal(out[:m].cpu().numpy().view(np.uint64), ref)
+    assert (out[m:] == -1).all().item()
+    zk.extended_to_coeff_dev(d_ext, d_ext[:m], log_ext, w_inv, d, g_inv)
+    torch.cuda.synchronize()
+    got = d_ext.cpu().numpy().view(np.uint64)
+    assert np.array_equal(got[:m], ref) and np.array_equal(got[m:], ext[m:])

@@ -43,7 +43,7 @@ int ntt_device(int device, fe* d_a, uint32_t log_n, const hf::Fr& w, const hf::F
       if (tmp) cudaFreeAsync(tmp, s);
       return zk::status_of("pow_tables_make", e);
     }
-    zk::count_launches(2);
+    zk::count_launches(1);
   }
   e = zk::ntt_run(*t, d_a, tmp, coset ? &pre : nullptr, post, s);
   zk::count_launches(t->plan.npass > 0 ? t->plan.npass : 1);
@@ -129,29 +129,21 @@ int ext_to_coeff_device(int device, const fe* d_ext, uint32_t log_ext, const hf:
   const bool tiny = t->plan.npass == 0;  // direct kernel: constant scale only
   const zk::PowTablesRef gd = zk::pow_tables_get(device, g_inv, (int)log_ext, s, &e, tiny ? nullptr : &divisor);
   if (!gd) return zk::status_of("pow_tables_get", e);
-  fe *work = nullptr, *tmp = nullptr;
-  ZK_TRY("zk::dmalloc(ext_to_coeff work)", zk::dmalloc((void**)&work, N * sizeof(fe), s));
-  if (t->plan.npass > 1) {
-    e = zk::dmalloc((void**)&tmp, N * sizeof(fe), s);
-    if (e != cudaSuccess) {
-      cudaFreeAsync(work, s);
-      return zk::status_of("zk::dmalloc(ext_to_coeff scratch)", e);
-    }
-  }
+  fe* tmp = nullptr;
+  if (tiny || t->plan.npass > 1) ZK_TRY("zk::dmalloc(ext_to_coeff scratch)", zk::dmalloc((void**)&tmp, N * sizeof(fe), s));
   if (tiny) {
-    e = cudaMemcpyAsync(work, d_ext, N * sizeof(fe), cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = zk::ntt_run(*t, work, tmp, nullptr, &divisor, s);
-    if (e == cudaSuccess) e = zk::fr_scale_copy(d_out, work, m, 1, gd.get(), s);
+    e = cudaMemcpyAsync(tmp, d_ext, N * sizeof(fe), cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess) e = zk::ntt_run(*t, tmp, nullptr, nullptr, &divisor, s);
+    if (e == cudaSuccess) e = zk::fr_scale_copy(d_out, tmp, m, 1, gd.get(), s);
     zk::count_launches(2);
-  } else {
+  } else {  // the last pass writes the m wanted coefficients only
     zk::NttFuse f;
     f.src = d_ext;
     f.post_tab = gd.get();
-    e = zk::ntt_run(*t, work, tmp, f, s);
+    f.wanted = m;
+    e = zk::ntt_run(*t, d_out, tmp, f, s);
     zk::count_launches(t->plan.npass);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_out, work, m * sizeof(fe), cudaMemcpyDeviceToDevice, s);
   }
-  cudaFreeAsync(work, s);
   if (tmp) cudaFreeAsync(tmp, s);
   return zk::status_of("ext_to_coeff", e);
 }

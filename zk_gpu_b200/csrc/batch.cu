@@ -120,7 +120,7 @@ extern "C" int zkgpu_ntt_batch_create(int device, const zkgpu_ntt_job* jobs, uin
       f.pre = info[j].pre.get();
       f.post = info[j].has_post ? &info[j].post : nullptr;
       const uint64_t ncta = zk::ntt_batch_pass_params(t, lvl, reinterpret_cast<fe*>(jobs[j].data),
-                                                      b->d_tmp + info[j].tmp_off, f, &bp.p);
+                                                      b->d_tmp + info[j].tmp_off, f, &bp);
       bp.B = (uint32_t)t.plan.bits[lvl];
       bp.ntiles = (uint32_t)ncta;
       bp.tile_base = (uint32_t)tiles;
@@ -210,7 +210,7 @@ extern "C" int zkgpu_selftest_wait_timeout(int device, const uint64_t omega12[4]
   zk::BatchPass bp[2] = {};
   uint64_t tiles = 0;
   for (int k = 0; k < 2; k++) {
-    bp[k].ntiles = (uint32_t)zk::ntt_batch_pass_params(*t, k, d, tmp, zk::NttFuse{}, &bp[k].p);
+    bp[k].ntiles = (uint32_t)zk::ntt_batch_pass_params(*t, k, d, tmp, zk::NttFuse{}, &bp[k]);
     bp[k].B = (uint32_t)t->plan.bits[k];
     bp[k].tile_base = (uint32_t)tiles;
     tiles += bp[k].ntiles;

@@ -27,8 +27,22 @@ namespace {
 
 using P_r = FrP;
 
+// A constant multiplicand as a kernel parameter (mul_w8: 350 cycles per warp
+// and scheduler against 555 of the Montgomery product).  These vectors are
+// bound by the products as long as they fit into L2.
+struct ConstW8 {
+  uint32_t w[64];
+};
+__device__ __forceinline__ void mul_const(uint32_t r[8], const uint32_t a[8], const ConstW8& c) {
+  mul_w8<P_r>(r, a, [&](int k, uint32_t v[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = c.w[8 * k + j];
+  });
+  reduce_once<P_r>(r, r);
+}
+
 template <int OP>
-__device__ __forceinline__ void ew_one(fe* out, const fe* a, const fe* b, const fe& c, uint64_t i) {
+__device__ __forceinline__ void ew_one(fe* out, const fe* a, const fe* b, const ConstW8& c, uint64_t i) {
   uint32_t x[8], y[8], r[8];
   ld_fe(x, a + i);
   if (OP == ZKGPU_EW_MUL) {
@@ -41,44 +55,56 @@ __device__ __forceinline__ void ew_one(fe* out, const fe* a, const fe* b, const 
     ld_fe(y, b + i);
     sub<P_r>(r, x, y);
   } else if (OP == ZKGPU_EW_SCALE) {
-    mul<P_r>(r, x, c.w);
+    mul_const(r, x, c);
   } else {  // AXPY
     ld_fe(y, b + i);
-    mul<P_r>(r, x, c.w);
+    mul_const(r, x, c);
     add<P_r>(r, r, y);
   }
   st_fe(out + i, r);
 }
 
 template <int OP>
-__global__ void __launch_bounds__(256) ew_kernel(fe* out, const fe* a, const fe* b, const fe c_fe, uint64_t n) {
+__global__ void __launch_bounds__(256) ew_kernel(fe* out, const fe* a, const fe* b, const ConstW8 c, uint64_t n) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   for (; i + stride < n; i += 2 * stride) {
-    ew_one<OP>(out, a, b, c_fe, i);
-    ew_one<OP>(out, a, b, c_fe, i + stride);
+    ew_one<OP>(out, a, b, c, i);
+    ew_one<OP>(out, a, b, c, i + stride);
   }
-  if (i < n) ew_one<OP>(out, a, b, c_fe, i);
+  if (i < n) ew_one<OP>(out, a, b, c, i);
 }
 
 constexpr int kMaxVanish = 64;  // distinct values of X^n - 1 on the coset (extension factor <= 64)
 struct VanishInv {
-  fe v[kMaxVanish];  // 1 / t_j
+  fe v[kMaxVanish];  // 1 / t_j, the first element of its form for mul_w2
+  fe step;           // a Montgomery product with it gives the second
 };
 
-__global__ void __launch_bounds__(256) vanish_kernel(fe* d, const VanishInv tinv, uint32_t mask, uint64_t n) {
+// The grid's stride is a multiple of the number of distinct values, so a
+// thread's elements all take the same one, tabulated once (mul_w2: 441 cycles
+// per warp and scheduler against 555).
+__global__ void __launch_bounds__(256) vanish_kernel(fe* d, const __grid_constant__ VanishInv tinv, uint32_t mask,
+                                                     uint64_t n) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
+  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  uint32_t v[8], w[8];
+  cpy(v, tinv.v[i & mask].w);
+  mul<P_r>(w, v, tinv.step.w);
+  for (; i < n; i += stride) {
     uint32_t x[8];
     ld_fe(x, d + i);
-    mul<P_r>(x, x, tinv.v[i & mask].w);
+    mul_w2<P_r>(x, x, v, w);
+    reduce_once<P_r>(x, x);
     st_fe(d + i, x);
   }
 }
 
-fe to_fe(const host::Fr& a) {
+// c (Montgomery form) times the integer s, as words
+fe scaled(const host::Fr& c, const host::Fr& s) {
+  const host::Fr r = host::mul(c, s);
   fe out;
-  std::memcpy(out.w, a.v, 32);
+  std::memcpy(out.w, r.v, 32);
   return out;
 }
 
@@ -103,12 +129,14 @@ extern "C" int zkgpu_ew_dev(int device, uint32_t op, uint64_t* d_out, const uint
   const bool needs_b = op != ZKGPU_EW_SCALE;
   const bool needs_c = op == ZKGPU_EW_SCALE || op == ZKGPU_EW_AXPY;
   if (!d_out || !d_a || (needs_b && !d_b) || (needs_c && !c)) return ZKGPU_EINVAL;
-  fe c_fe{};
+  zk::ConstW8 cw{};
   if (needs_c) {
     zk::host::Fr cc;
     std::memcpy(cc.v, c, 32);
     if (!zk::host::is_canonical(cc)) return ZKGPU_EINVAL;
-    c_fe = zk::to_fe(cc);
+    using zk::host::pow2;
+    static const zk::host::Fr scale[8] = {pow2(64), pow2(96), pow2(128), pow2(160), pow2(192), pow2(224), pow2(256), pow2(288)};
+    for (int k = 0; k < 8; k++) std::memcpy(cw.w + 8 * k, zk::scaled(cc, scale[k]).w, 32);
   }
   cudaStream_t own;
   int st = zk::bind_device(device, &own);
@@ -123,11 +151,11 @@ extern "C" int zkgpu_ew_dev(int device, uint32_t op, uint64_t* d_out, const uint
   {
     zk::ProfScope ps(names[op], s, products, (double)n * (needs_b ? 96.0 : 64.0));
     switch (op) {
-      case ZKGPU_EW_MUL: zk::ew_kernel<ZKGPU_EW_MUL><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
-      case ZKGPU_EW_ADD: zk::ew_kernel<ZKGPU_EW_ADD><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
-      case ZKGPU_EW_SUB: zk::ew_kernel<ZKGPU_EW_SUB><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
-      case ZKGPU_EW_SCALE: zk::ew_kernel<ZKGPU_EW_SCALE><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
-      default: zk::ew_kernel<ZKGPU_EW_AXPY><<<grid, 256, 0, s>>>(out, a, b, c_fe, n); break;
+      case ZKGPU_EW_MUL: zk::ew_kernel<ZKGPU_EW_MUL><<<grid, 256, 0, s>>>(out, a, b, cw, n); break;
+      case ZKGPU_EW_ADD: zk::ew_kernel<ZKGPU_EW_ADD><<<grid, 256, 0, s>>>(out, a, b, cw, n); break;
+      case ZKGPU_EW_SUB: zk::ew_kernel<ZKGPU_EW_SUB><<<grid, 256, 0, s>>>(out, a, b, cw, n); break;
+      case ZKGPU_EW_SCALE: zk::ew_kernel<ZKGPU_EW_SCALE><<<grid, 256, 0, s>>>(out, a, b, cw, n); break;
+      default: zk::ew_kernel<ZKGPU_EW_AXPY><<<grid, 256, 0, s>>>(out, a, b, cw, n); break;
     }
   }
   zk::count_launches(1);
@@ -148,10 +176,13 @@ extern "C" int zkgpu_divide_by_vanishing_dev(int device, uint64_t* d_ext, uint32
   const hf::Fr step = hf::pow_2k(we, log_n);
   hf::Fr cur = hf::pow_2k(gg, log_n);
   zk::VanishInv tinv{};
+  static const hf::Fr s0 = hf::pow2(160), s1 = hf::pow2(256 + 128);
+  std::memcpy(tinv.step.w, s1.v, 32);
   for (uint32_t j = 0; j < J; j++) {
     const hf::Fr t = hf::sub(cur, hf::one());
     if (hf::eq(t, hf::zero())) return ZKGPU_EINVAL;  // X^n - 1 vanishes on this coset
-    tinv.v[j] = zk::to_fe(hf::inv(t));
+    const hf::Fr ti = hf::inv(t);
+    tinv.v[j] = zk::scaled(ti, s0);
     cur = hf::mul(cur, step);
   }
   cudaStream_t own;

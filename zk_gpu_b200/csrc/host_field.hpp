@@ -104,6 +104,11 @@ inline Fr add(const Fr& a, const Fr& b) {  // canonical inputs
   return r;
 }
 inline Fr sub(const Fr& a, const Fr& b) { return add(a, neg(b)); }
+inline Fr pow2(int e) {  // the integer 2^e mod r
+  Fr x{{1, 0, 0, 0}};
+  for (int i = 0; i < e; i++) x = add(x, x);
+  return x;
+}
 inline Fr pow_u64(Fr a, uint64_t e) {
   Fr r = one();
   while (e) {

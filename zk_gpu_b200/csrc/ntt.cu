@@ -132,15 +132,15 @@ __global__ void __launch_bounds__(256, 2) ntt_batch_kernel(const BatchPass* pass
     roots_b = bp.B;
     roots_at = at;
     switch (bp.B) {
-      case 3: ntt_pass_tile<3, true>(bp.p, nullptr, tile, smem, have); break;
-      case 4: ntt_pass_tile<4, true>(bp.p, nullptr, tile, smem, have); break;
-      case 5: ntt_pass_tile<5, true>(bp.p, nullptr, tile, smem, have); break;
-      case 6: ntt_pass_tile<6, true>(bp.p, nullptr, tile, smem, have); break;
-      case 7: ntt_pass_tile<7, true>(bp.p, nullptr, tile, smem, have); break;
-      case 8: ntt_pass_tile<8, true>(bp.p, nullptr, tile, smem, have); break;
-      case 9: ntt_pass_tile<9, true>(bp.p, nullptr, tile, smem); break;
-      case 10: ntt_pass_tile<10, true>(bp.p, nullptr, tile, smem); break;
-      case 11: ntt_pass_tile<11, true>(bp.p, nullptr, tile, smem); break;
+      case 3: ntt_pass_tile<3, true>(bp.p, nullptr, bp.post, tile, smem, have); break;
+      case 4: ntt_pass_tile<4, true>(bp.p, nullptr, bp.post, tile, smem, have); break;
+      case 5: ntt_pass_tile<5, true>(bp.p, nullptr, bp.post, tile, smem, have); break;
+      case 6: ntt_pass_tile<6, true>(bp.p, nullptr, bp.post, tile, smem, have); break;
+      case 7: ntt_pass_tile<7, true>(bp.p, nullptr, bp.post, tile, smem, have); break;
+      case 8: ntt_pass_tile<8, true>(bp.p, nullptr, bp.post, tile, smem, have); break;
+      case 9: ntt_pass_tile<9, true>(bp.p, nullptr, bp.post, tile, smem); break;
+      case 10: ntt_pass_tile<10, true>(bp.p, nullptr, bp.post, tile, smem); break;
+      case 11: ntt_pass_tile<11, true>(bp.p, nullptr, bp.post, tile, smem); break;
       default: break;
     }
     __threadfence();  // every thread publishes its own stores before the tile is counted
@@ -202,14 +202,9 @@ __global__ void pow_seq_kernel(fe* out, fe base, uint64_t count, uint64_t step) 
 struct TableScale {
   fe w4[4], w2[2];
 };
-static host::Fr pow2(int e) {  // the integer 2^e mod r, e < 512
-  host::Fr x{{1, 0, 0, 0}};
-  for (int i = 0; i < e; i++) x = host::add(x, x);
-  return x;
-}
 static TableScale table_scale() {
-  static const TableScale s = {{to_fe(pow2(96)), to_fe(pow2(160)), to_fe(pow2(224)), to_fe(pow2(288))},
-                               {to_fe(pow2(160)), to_fe(pow2(288))}};
+  static const TableScale s = {{to_fe(host::pow2(96)), to_fe(host::pow2(160)), to_fe(host::pow2(224)), to_fe(host::pow2(288))},
+                               {to_fe(host::pow2(160)), to_fe(host::pow2(288))}};
   return s;
 }
 
@@ -308,25 +303,57 @@ static cudaError_t pow_two_level(fe** lo, fe** hi, uint32_t* shift, const host::
   return cudaGetLastError();
 }
 
-// t[i] *= scale
-__global__ void scale_table_kernel(fe* t, fe scale, uint64_t count) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= count) return;
+// Both power tables in one launch: entry e of lo is scale base^e, of hi
+// base^(e 2^shift), as products of the host's base^(2^k) by the bits of e
+// (without squarings, which would double the chain of dependent products).
+struct PowArgs {
+  fe pw[NTT_MAX_LOG];  // base^(2^k), Montgomery form
+  fe scale;
+  uint32_t has_scale, shift, nlo, nhi;
+};
+__global__ void pow_tables_kernel(fe* lo, fe* hi, const PowArgs a) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.nlo + a.nhi) return;
+  const bool low = i < a.nlo;
+  const uint32_t e = low ? i : i - a.nlo;
   uint32_t v[8];
-  ld_fe(v, t + i);
-  mul<P_r>(v, v, scale.w);
-  st_fe(t + i, v);
+  if (low && a.has_scale)
+    cpy(v, a.scale.w);
+  else
+    set_one<P_r>(v);
+  for (uint32_t k = 0, b = e; b; k++, b >>= 1)
+    if (b & 1u) mul_lazy<P_r>(v, v, a.pw[(low ? 0 : a.shift) + k].w);
+  reduce_once<P_r>(v, v);
+  st_fe((low ? lo : hi) + e, v);
 }
 
 cudaError_t pow_tables_make(PowTables* t, const host::Fr& c, int log_n, cudaStream_t s, const host::Fr* scale,
                             bool pooled) {
-  cudaError_t e = pow_two_level(&t->lo, &t->hi, &t->shift, c, log_n, s, pooled);
-  if (e == cudaSuccess && scale) {
-    const uint64_t nlo = 1ull << t->shift;
-    scale_table_kernel<<<(unsigned)((nlo + 255) / 256), 256, 0, s>>>(t->lo, to_fe(*scale), nlo);
-    e = cudaGetLastError();
+  PowArgs a{};
+  a.shift = (uint32_t)((log_n + 1) / 2);
+  a.nlo = 1u << a.shift;
+  a.nhi = 1u << (log_n - (int)a.shift);
+  host::Fr x = c;
+  for (int k = 0; k < log_n; k++, x = host::mul(x, x)) a.pw[k] = to_fe(x);
+  if (scale) {
+    a.has_scale = 1;
+    a.scale = to_fe(*scale);
   }
-  return e;
+  t->lo = t->hi = nullptr;
+  t->shift = a.shift;
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+    void** p = (void**)(k ? &t->hi : &t->lo);
+    const size_t bytes = (size_t)(k ? a.nhi : a.nlo) * sizeof(fe);
+    e = pooled ? zk::dmalloc(p, bytes, s) : cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) {
+    if (t->lo) pooled ? cudaFreeAsync(t->lo, s) : cudaFree(t->lo);
+    t->lo = t->hi = nullptr;
+    return e;
+  }
+  pow_tables_kernel<<<(a.nlo + a.nhi + 127) / 128, 128, 0, s>>>(t->lo, t->hi, a);
+  return cudaGetLastError();
 }
 void pow_tables_free(PowTables* t, cudaStream_t s) {
   if (t->lo) cudaFreeAsync(t->lo, s);
@@ -348,7 +375,7 @@ static void fill_inner(fe* out, DftConsts* dft, const host::Fr& wm, int B, cudaS
   const host::Fr c[3] = {w4, host::mul(half, host::add(w8, w83)), host::mul(half, host::sub(w8, w83))};
   for (int k = 0; k < 3; k++) {
     sp.v[k] = to_fe(c[k]);
-    for (int j = 0; j < 8; j++) std::memcpy(dft->w[k] + 8 * j, host::mul(c[k], pow2(32 * j + 64)).v, 32);
+    for (int j = 0; j < 8; j++) std::memcpy(dft->w[k] + 8 * j, host::mul(c[k], host::pow2(32 * j + 64)).v, 32);
   }
   roots_w4_kernel<<<grid, 256, 0, s>>>(out, to_fe(wm), sp, table_scale(), B);
 }
@@ -508,8 +535,12 @@ static cudaError_t dispatch_pass(int B, const PassParams& pp, const DftConsts& d
   }
 }
 
-uint64_t ntt_batch_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* out) {
-  return ntt_pass_params(t, k, d_a, d_tmp, f, out, true);
+uint64_t ntt_batch_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, BatchPass* out) {
+  if (f.post) {
+    static const host::Fr w2[2] = {host::pow2(160), host::pow2(288)};
+    for (int j = 0; j < 2; j++) out->post[j] = to_fe(host::mul(*f.post, w2[j]));
+  }
+  return ntt_pass_params(t, k, d_a, d_tmp, f, &out->p, true);
 }
 
 static uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* out,
@@ -543,6 +574,7 @@ static uint64_t ntt_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, c
     pp.has_post = 1;
     pp.post = to_fe(*post);
   }
+  pp.out_count = (uint32_t)(f.wanted ? f.wanted : 1ull << L);
   if (final_pass && f.post_tab) {
     pp.post_lo = f.post_tab->lo;
     pp.post_hi = f.post_tab->hi;

@@ -45,6 +45,16 @@ NttPlan tuned_ntt_plan(int device, int log_n);
 struct DftConsts {
   uint32_t w[3][64];
 };
+// As the parameter of a pass of B bits.  Where they start decides how wide
+// the compiler's constant loads are, and with that the pass's registers: on a
+// 16-byte boundary passes of 6 bits are fastest (2^24 as 6+6+6+6: 2520 us,
+// 2590 eight bytes past it), eight bytes past it those of 7 (2^21 as 7+7+7: 331
+// against 337) and of 8 (2^24 as 8+8+8: 2556 against 2580).
+template <int B>
+struct alignas(16) DftParam {
+  uint32_t lead[B >= 7 ? 2 : 4];
+  DftConsts c;
+};
 
 // Device tables for one (omega, log_n): per pass the roots its rounds use and,
 // for non-final passes, the twist table [k * J + j] (two entries of mul_w2).
@@ -57,8 +67,7 @@ struct NttTables {
   size_t bytes = 0;
 };
 
-// Coset pre-multiplication: input element x is multiplied by c^x, read as
-// lo[x & (2^shift - 1)] * hi[x >> shift].
+// Powers c^x = lo[x & (2^shift - 1)] * hi[x >> shift].
 struct PowTables {
   fe* lo = nullptr;
   fe* hi = nullptr;
@@ -118,13 +127,14 @@ struct PassParams {
   uint32_t is_first;
   uint32_t is_final;
   uint32_t has_post;
-  fe post;
+  fe post;  // output scale
   // final pass: output k multiplied by post_lo[k & mask] * post_hi[k >> shift]
   const fe* post_lo;
   const fe* post_hi;
   uint32_t post_shift;
   // first pass: rows >= in_rows are known zeros (zero-padded input), 0 = all
   uint32_t in_rows;
+  uint32_t out_count;  // final pass with post_lo: outputs from here on are not written
 };
 
 // Optional work fused into a transform.
@@ -134,21 +144,22 @@ struct NttFuse {
   const PowTables* post_tab = nullptr;  // output k times the table's k-th power
   uint64_t nonzero = 0;                 // only inputs [0, nonzero) may be non-zero (0 = all)
   const fe* src = nullptr;              // read the input from here instead of d_a (d_a gets the result)
+  uint64_t wanted = 0;                  // only outputs [0, wanted) are written to d_a (0 = all)
 };
-
-// Pass k of the plan in `t` over d_a / d_tmp as the batch kernel runs it;
-// returns its tile count.
-uint64_t ntt_batch_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, PassParams* pp);
 
 // One pass of one transform inside a batch launch.
 struct BatchPass {
   PassParams p;
+  fe post[2];  // p.post as the two elements of mul_w2
   uint32_t B;
   uint32_t ntiles;
   uint32_t tile_base;  // global index of this pass's first tile
   uint32_t dep;        // index of the pass this one waits for, or ~0u
   uint32_t dep_tiles;  // tiles of that pass
 };
+// Pass k of the plan in `t` over d_a / d_tmp as the batch kernel runs it (p
+// and post of *out); returns its tile count.
+uint64_t ntt_batch_pass_params(const NttTables& t, int k, fe* d_a, fe* d_tmp, const NttFuse& f, BatchPass* out);
 // Launch the persistent batch kernel over `npass` descriptors (device memory,
 // ordered by level), with counters next/done/err zeroed by the caller.
 // Every dependency wait gives up after spin_cycles SM clocks (default about

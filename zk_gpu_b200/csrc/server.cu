@@ -513,7 +513,7 @@ class Server {
           fu.post = it.has_post ? &it.post : nullptr;
           fu.post_tab = it.post_tab.get();
           fu.nonzero = it.nonzero;
-          const uint64_t ncta = ntt_batch_pass_params(*it.t, k, it.data, it.tmp, fu, &bp.p);
+          const uint64_t ncta = ntt_batch_pass_params(*it.t, k, it.data, it.tmp, fu, &bp);
           bp.B = (uint32_t)it.t->plan.bits[k];
           bp.ntiles = (uint32_t)ncta;
           bp.tile_base = (uint32_t)tiles;
