@@ -201,9 +201,9 @@ void zkgpu_ntt_batch_destroy(void *handle);
 
 /* ======================================================================
  * Autotuner: per device and size, the NTT plan (pass widths b_k, 3..11 bits;
- * each pass runs radix-2^b_k columns in CTA tiles of 2^b_k x G elements,
- * G = 2^(11 - b_k)) and the MSM window width c, picked by timing candidates
- * on the device.  Replaces the fixed 1024 x n/1024 split of
+ * each pass runs radix-2^b_k columns in tiles of 2^10 elements, 2^11 above
+ * eight bits) and the MSM window width c, picked by timing candidates on the
+ * device.  Replaces the fixed 1024 x n/1024 split of
  * cuda/fft.cu:275-405 and the ceil(ln len) window of cuda/fft.cu:165-172.
  * Choices change speed only: every plan and window is bit-exact.  Installed
  * choices apply to later calls on that device (tables of a new plan are built
