@@ -1024,22 +1024,22 @@ HBM_GBS = 6543.1
 # DRAM bytes (read + write) per launch over algorithmic bytes, from one ncu
 # capture of the same kernel on a smaller case (traffic grows with the
 # elements processed): ntt_pass_kernel<6> on a 2^24 transform, plan 6+6+6+6,
-# launches 1.588 / 1.611 GB and 1.051 / 1.082 GB.
-TRAFFIC_RATIO = {"ntt_pass_b6": 0.97}
-TRAFFIC_SOURCE = {"ntt_pass_b6": "ncu dram__bytes_read.sum + dram__bytes_write.sum of ntt_pass_kernel<6> on a "
+# launches 2.131 / 2.147 GB and 1.070 / 1.091 GB.
+TRAFFIC_RATIO = {"ntt_pass_b6": 0.98}
+TRAFFIC_SOURCE = {"ntt_pass_b6": "ncu dram__bytes.sum.per_second x duration of ntt_pass_kernel<6> on a "
                                  "2^24 transform (plan 6+6+6+6), scaled by algorithmic bytes"}
-# Pipe utilisation of the dominant kernels from one ncu --set full capture
-# each (ntt_pass_kernel<6> on a 2^24 transform, ba_apply_kernel<1> in the
-# 2^22 MSM): the IMAD-convention frac counts products per second, these say
-# how busy the pipes the FP64-limb product actually uses are.
+# Pipe utilisation of the dominant kernels from one ncu capture each
+# (ntt_pass_kernel<6> on a 2^24 transform, ba_apply_kernel<1> in the 2^22
+# MSM): the IMAD-convention frac counts products per second, these say how
+# busy the pipe of the wide integer multiplications actually is.
 PIPE_FRACS = {
-    "ntt_pass_b6": {"fp64": 0.398, "alu": 0.525, "fma_imad": 0.097, "issue_active": 0.579, "warps_active": 0.245,
-                    "source": "ncu sm__inst_executed_pipe_{fp64,alu,fma}, smsp__issue_active, sm__warps_active of "
+    "ntt_pass_b6": {"fma_heavy": 0.776, "alu": 0.281, "issue_active": 0.401, "warps_active": 0.241,
+                    "source": "ncu sm__pipe_{fmaheavy,alu}_cycles_active, sm__issue_active, sm__warps_active of "
                               "ntt_pass_kernel<6> on a 2^24 transform (second pass)"},
-    "msm_apply": {"kernel": "ba_apply_kernel<1> (round 0, 55 % of the MSM with the other rounds)",
-                  "fp64": 0.350, "alu": 0.504, "fma_imad": 0.105, "issue_active": None, "warps_active": 0.238,
-                  "source": "ncu sections SpeedOfLight, WarpStateStats, ComputeWorkloadAnalysis and LaunchStats "
-                            "of ba_apply_kernel<1> in the 2^22 MSM (issue active not in those sections)"},
+    "msm_apply": {"kernel": "ba_apply_kernel<1> (round 0, 50 % of the MSM with the other rounds)",
+                  "fma_heavy": 0.747, "alu": 0.329, "issue_active": 0.381, "warps_active": 0.272,
+                  "source": "ncu sm__pipe_{fmaheavy,alu}_cycles_active, sm__issue_active, sm__warps_active of "
+                            "ba_apply_kernel<1> in the 2^22 MSM"},
 }
 
 

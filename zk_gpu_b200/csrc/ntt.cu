@@ -649,7 +649,8 @@ cudaError_t ntt_run(const NttTables& t, fe* d_a, fe* d_tmp, const NttFuse& f, cu
     const uint64_t ncta = ntt_pass_params(t, k, d_a, d_tmp, f, &pp, false);
     const double nel = (double)(1ull << L);
     // algorithmic work: radix-2 convention (n/2) * b products; bytes: read + write (+ twist table)
-    ProfScope prof(names[b], s, nel / 2 * b, nel * 32.0 * (pp.is_final ? 2 : 4));
+    ProfScope prof(names[b], s, nel / 2 * b,
+                   nel * 64.0 + (pp.is_final ? 0.0 : 64.0 * (double)(1ull << (L - (int)pp.log_O))));
     const bool small = L <= kPairMaxLog && b <= kNarrowMax;
     cudaError_t e = small ? dispatch_pair(b, pp, L, s) : dispatch_pass(b, pp, t.dft[k], ncta, s);
     if (e != cudaSuccess) return e;
