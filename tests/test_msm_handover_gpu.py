@@ -1,0 +1,49 @@
+"""GPU: the last step of zkgpu_msm_dev, which the stream's last kernel hands to
+a thread of the library and otherwise does itself (msm_combine.cu).  Every
+case runs in a process of its own, since ZKGPU_MSM_HOST_WAIT_US is read once;
+results are compared with the oracle here."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PRELUDE = """
+import sys, threading, time
+import numpy as np, torch
+import zk_gpu_b200 as zk
+data = np.load(sys.argv[1])
+ds, db = (torch.from_numpy(data[k].view(np.int64)).cuda() for k in ("s", "b"))
+save = lambda x: np.save(sys.argv[2], x.cpu().numpy().view(np.uint64))
+"""
+
+
+def run_child(tmp_path, code, s, pts, **env):
+    inp, out = str(tmp_path / "in.npz"), str(tmp_path / "out.npy")
+    np.savez(inp, s=s, b=pts)
+    subprocess.run([sys.executable, "-c", PRELUDE + code, inp, out], cwd=ROOT, env=dict(os.environ, **env),
+                   check=True, timeout=300)
+    return np.load(out)
+
+
+@pytest.mark.parametrize("wait_us", ["0", "3000"])
+def test_result_pointer_aligned_to_its_words_only(oracle, tmp_path, wait_us):
+    """d_out_xyz is an array of 64-bit words and may start at any of them,
+    whoever does the last step; the sum over no points too."""
+    n = 100
+    s, pts = oracle.rand_fr(n, 901), oracle.rand_bases(n, 902)
+    got = run_child(tmp_path, """
+out = torch.full((2, 15), 7, dtype=torch.int64, device="cuda")  # both results 8 bytes past a 16-byte boundary
+zk.msm_dev(ds, db, out[0, 1:13])
+zk.msm_dev(ds[:0], db[:0], out[1, 2:14])
+save(out)
+""", s, pts, ZKGPU_MSM_HOST_WAIT_US=wait_us)
+    assert np.array_equal(got[0, 1:9], oracle.multiexp(s, pts))
+    assert np.array_equal(got[0, 9:13], oracle.to_mont(1, oracle.FQ))
+    assert not got[1, 2:14].any()
+    for row, a, b in ((got[0], 1, 13), (got[1], 2, 14)):
+        assert (row[:a] == 7).all() and (row[b:] == 7).all()

@@ -72,7 +72,7 @@ extern "C" int zkgpu_msm_dev(int device, const uint64_t* d_scalars, const uint64
   if (st) return st;
   uint64_t nl = 0;
   cudaError_t e = zk::msm_run(reinterpret_cast<const fe*>(d_scalars), reinterpret_cast<const fe*>(d_bases_xy), n,
-                              reinterpret_cast<fe*>(d_out_xyz), (cudaStream_t)stream, 0, &nl);
+                              d_out_xyz, (cudaStream_t)stream, 0, &nl);
   zk::count_launches(nl);
   return zk::status_of("msm_dev", e);
 }

@@ -832,11 +832,8 @@ __global__ void __launch_bounds__(4 * kGroup) msm_group_kernel(const fe* in_t, c
   if (t == 0) st_fe(out_t + 4 * (uint64_t)g + z.j, c);
 }
 
-__global__ void zero_out_kernel(fe* out) {
-  if (threadIdx.x < 3) {
-    uint32_t z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    st_fe(out + threadIdx.x, z);
-  }
+__global__ void zero_out_kernel(uint64_t* out) {
+  if (threadIdx.x < 12) out[threadIdx.x] = 0;
 }
 
 namespace {
@@ -944,7 +941,7 @@ MsmLayout msm_layout(uint64_t n, uint32_t jobs, int c_override, int device = -1)
 // n: scalars (all jobs); jobs > 1: job_off (device, jobs + 1 entries) splits
 // them and every job reads bases [0, nbases); the window sums of job j are
 // windows [j W, (j + 1) W) of wout.
-cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, fe* d_out, cudaStream_t s,
+cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, uint64_t* d_out, cudaStream_t s,
                          int c_override, uint64_t* launches, MsmWindowsOut* wout, const uint32_t* job_off,
                          uint32_t jobs) {
   uint64_t nl = 0;
@@ -1135,8 +1132,8 @@ uint64_t msm_scratch_bytes(uint64_t n_total, uint32_t jobs, bool own_winsum, int
   return l.bytes(own_winsum);
 }
 
-cudaError_t msm_run(const fe* d_scalars, const fe* d_bases, uint64_t n, fe* d_out, cudaStream_t s, int c_override,
-                    uint64_t* launches, MsmWindowsOut* wout) {
+cudaError_t msm_run(const fe* d_scalars, const fe* d_bases, uint64_t n, uint64_t* d_out, cudaStream_t s,
+                    int c_override, uint64_t* launches, MsmWindowsOut* wout) {
   return msm_run_impl(d_scalars, d_bases, n, d_out, s, c_override, launches, wout, nullptr, 1);
 }
 

@@ -49,11 +49,11 @@ struct MsmWindowsOut {
   uint32_t c = 0;
 };
 constexpr uint32_t MSM_MAX_WINDOWS = 64;  // c >= 4
-cudaError_t msm_run(const fe* d_scalars, const fe* d_bases_xy, uint64_t n, fe* d_out, cudaStream_t s,
+cudaError_t msm_run(const fe* d_scalars, const fe* d_bases_xy, uint64_t n, uint64_t* d_out, cudaStream_t s,
                     int c_override = 0, uint64_t* launches = nullptr, MsmWindowsOut* wout = nullptr);
 // The last step on the stream (msm_combine.cu): Horner over `windows` window
 // sums, the normalised Jacobian result to d_out.
-cudaError_t msm_combine(const fe* d_winsum, uint32_t windows, uint32_t c, fe* d_out, cudaStream_t s);
+cudaError_t msm_combine(const fe* d_winsum, uint32_t windows, uint32_t c, uint64_t* d_out, cudaStream_t s);
 // Several MSMs over one base array (the serving loop's jobs against resident
 // bases) in one pass: job j's scalars are [off[j], off[j+1]) of d_scalars
 // (d_job_off: jobs + 1 offsets in device memory, off[0] = 0), each against

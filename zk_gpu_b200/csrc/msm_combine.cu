@@ -61,7 +61,13 @@ __device__ __forceinline__ uint64_t now_ns() {
   return t;
 }
 
-__device__ __noinline__ void combine_here(const fe* winsum, uint32_t windows, uint32_t c, fe* out) {
+// The caller's result is an array of 64-bit words: 8-byte stores.
+__device__ __forceinline__ void st_words(uint64_t* out, const uint32_t r[8]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) out[k] = (uint64_t)r[2 * k + 1] << 32 | r[2 * k];
+}
+
+__device__ __noinline__ void combine_here(const fe* winsum, uint32_t windows, uint32_t c, uint64_t* out) {
   xyzz_t acc, w;
   ld_xyzz(acc, winsum + 4 * (uint64_t)(windows - 1));
 #pragma unroll 1
@@ -88,12 +94,12 @@ __device__ __noinline__ void combine_here(const fe* winsum, uint32_t windows, ui
     reduce_once<P_q>(p.y, p.y);
     set_one<P_q>(z);
   }
-  st_fe(out, p.x);
-  st_fe(out + 1, p.y);
-  st_fe(out + 2, z);
+  st_words(out, p.x);
+  st_words(out + 4, p.y);
+  st_words(out + 8, z);
 }
 
-__global__ void __launch_bounds__(128) msm_combine_kernel(const fe* winsum, uint32_t windows, uint32_t c, fe* out,
+__global__ void __launch_bounds__(128) msm_combine_kernel(const fe* winsum, uint32_t windows, uint32_t c, uint64_t* out,
                                                           Mail* mail, uint32_t seq, uint64_t wait_ns) {
   if (mail) {
     __shared__ uint32_t answered;
@@ -111,8 +117,7 @@ __global__ void __launch_bounds__(128) msm_combine_kernel(const fe* winsum, uint
     }
     __syncthreads();
     if (answered) {
-      if (threadIdx.x < 12)
-        reinterpret_cast<uint64_t*>(out)[threadIdx.x] = *(volatile const uint64_t*)&mail->out[threadIdx.x];
+      if (threadIdx.x < 12) out[threadIdx.x] = *(volatile const uint64_t*)&mail->out[threadIdx.x];
       return;
     }
   }
@@ -249,7 +254,7 @@ uint64_t host_wait_ns() {
 
 }  // namespace
 
-cudaError_t msm_combine(const fe* d_winsum, uint32_t windows, uint32_t c, fe* d_out, cudaStream_t s) {
+cudaError_t msm_combine(const fe* d_winsum, uint32_t windows, uint32_t c, uint64_t* d_out, cudaStream_t s) {
   if (windows == 0 || windows > MSM_MAX_WINDOWS) return cudaErrorInvalidValue;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);

@@ -253,10 +253,11 @@ cudaError_t tune_ntt_batched(int device, int log_n, int reps, cudaStream_t s, Nt
 
 cudaError_t tune_msm(int device, int log_n, int reps, cudaStream_t s, int* best_c, float* best_ms) {
   const uint64_t n = 1ull << log_n;
-  fe *sc = nullptr, *bs = nullptr, *out = nullptr;
+  fe *sc = nullptr, *bs = nullptr;
+  uint64_t* out = nullptr;
   cudaError_t e = cudaMalloc((void**)&sc, n * sizeof(fe));
   if (e == cudaSuccess) e = cudaMalloc((void**)&bs, 2 * n * sizeof(fe));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&out, 3 * sizeof(fe));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&out, 96);
   if (e == cudaSuccess) {
     fill_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(sc, n, 99, 0x0fffffffu);
     fill_kernel<<<(unsigned)((2 * n + 255) / 256), 256, 0, s>>>(bs, 2 * n, 98, 0x0fffffffu);
