@@ -238,3 +238,20 @@ def test_extended_to_coeff_writes_the_wanted_outputs_only(zk, oracle, log_ext, m
     torch.cuda.synchronize()
     got = d_ext.cpu().numpy().view(np.uint64)
     assert np.array_equal(got[:m], ref) and np.array_equal(got[m:], ext[m:])
+
+
+@pytest.mark.parametrize("log_ext,m", [(2, 3), (5, 32), (9, 300), (17, 4097)])
+def test_extended_to_coeff_output_on_an_odd_word(zk, oracle, log_ext, m):
+    """d_out is an array of 64-bit words and may start at any of them"""
+    torch = pytest.importorskip("torch")
+    ext = oracle.rand_fr(1 << log_ext, 190 + log_ext)
+    w_inv, d = oracle.inv(oracle.omega(log_ext)), inv_n(oracle, log_ext)
+    g_inv = oracle.inv(oracle.to_mont(7))
+    buf = torch.full((4 * m + 2,), -1, dtype=torch.int64, device="cuda")
+    zk.extended_to_coeff_dev(torch.from_numpy(ext.view(np.int64)).cuda(), buf[1:-1].view(m, 4), log_ext, w_inv, d,
+                             g_inv)
+    torch.cuda.synchronize()
+    got = buf.cpu().numpy().view(np.uint64)
+    ref = oracle.extended_to_coeff(ext, log_ext, m, w_inv, d, g_inv)
+    assert np.array_equal(got[1:-1].reshape(m, 4), ref)
+    assert got[0] == got[-1] == (1 << 64) - 1

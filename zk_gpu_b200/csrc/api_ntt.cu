@@ -119,7 +119,9 @@ int lde_device(int device, const fe* d_values, uint32_t log_n, fe* d_ext, uint32
 
 // Extended -> coefficient form (the inverse of the LDE): ifft over the
 // extended domain, times N^-1 * g_inv^i, first m coefficients to d_out.
-// The scale and the coset powers ride on the ifft's last pass (one table).
+// The scale and the coset powers ride on the ifft's last pass (one table),
+// which writes the coefficients in 16-byte vectors; a d_out on an odd 64-bit
+// word gets them by a copy.
 int ext_to_coeff_device(int device, const fe* d_ext, uint32_t log_ext, const hf::Fr& w_inv, const hf::Fr& divisor,
                         const hf::Fr& g_inv, fe* d_out, uint64_t m, cudaStream_t s) {
   const size_t N = (size_t)1 << log_ext;
@@ -129,20 +131,31 @@ int ext_to_coeff_device(int device, const fe* d_ext, uint32_t log_ext, const hf:
   const bool tiny = t->plan.npass == 0;  // direct kernel: constant scale only
   const zk::PowTablesRef gd = zk::pow_tables_get(device, g_inv, (int)log_ext, s, &e, tiny ? nullptr : &divisor);
   if (!gd) return zk::status_of("pow_tables_get", e);
-  fe* tmp = nullptr;
+  fe *tmp = nullptr, *out = d_out;
   if (tiny || t->plan.npass > 1) ZK_TRY("zk::dmalloc(ext_to_coeff scratch)", zk::dmalloc((void**)&tmp, N * sizeof(fe), s));
+  if (reinterpret_cast<uintptr_t>(d_out) % 16 != 0) {
+    e = zk::dmalloc((void**)&out, m * sizeof(fe), s);
+    if (e != cudaSuccess) {
+      if (tmp) cudaFreeAsync(tmp, s);
+      return zk::status_of("zk::dmalloc(ext_to_coeff out)", e);
+    }
+  }
   if (tiny) {
     e = cudaMemcpyAsync(tmp, d_ext, N * sizeof(fe), cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = zk::ntt_run(*t, tmp, nullptr, nullptr, &divisor, s);
-    if (e == cudaSuccess) e = zk::fr_scale_copy(d_out, tmp, m, 1, gd.get(), s);
+    if (e == cudaSuccess) e = zk::fr_scale_copy(out, tmp, m, 1, gd.get(), s);
     zk::count_launches(2);
   } else {  // the last pass writes the m wanted coefficients only
     zk::NttFuse f;
     f.src = d_ext;
     f.post_tab = gd.get();
     f.wanted = m;
-    e = zk::ntt_run(*t, d_out, tmp, f, s);
+    e = zk::ntt_run(*t, out, tmp, f, s);
     zk::count_launches(t->plan.npass);
+  }
+  if (out != d_out) {
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_out, out, m * sizeof(fe), cudaMemcpyDeviceToDevice, s);
+    cudaFreeAsync(out, s);
   }
   if (tmp) cudaFreeAsync(tmp, s);
   return zk::status_of("ext_to_coeff", e);
