@@ -733,7 +733,7 @@ __device__ __forceinline__ void block_sum(const Quad& z, uint32_t acc[8], fe* sh
 // each bucket's items.
 __global__ void __launch_bounds__(256) ba_heavy_items_kernel(const uint32_t* coff, fe* chunk_res, const uint2* heavy,
                                                              const uint32_t* heavy_count) {
-  __shared__ fe sh[256];
+  __shared__ __align__(16) fe sh[256];
   const Quad z;
   const uint32_t n = heavy_count[0];
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
@@ -747,7 +747,7 @@ __global__ void __launch_bounds__(256) ba_heavy_items_kernel(const uint32_t* cof
 }
 __global__ void __launch_bounds__(256) ba_heavy_kernel(const uint32_t* coff, const fe* chunk_res, fe* buckets,
                                                        const uint32_t* heavy_b, const uint32_t* heavy_count) {
-  __shared__ fe sh[256];
+  __shared__ __align__(16) fe sh[256];
   const Quad z;
   const uint32_t n = heavy_count[1];
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(128) msm_segment_kernel(const fe* buckets, fe*
 constexpr uint32_t kGroup = 16;
 __global__ void __launch_bounds__(4 * kGroup) msm_group_kernel(const fe* in_t, const fe* in_s, fe* out_t, fe* out_s,
                                                                uint32_t S, uint32_t L) {
-  __shared__ fe sh[2][4 * kGroup];
+  __shared__ __align__(16) fe sh[2][4 * kGroup];
   const Quad z;
   const uint32_t g = blockIdx.x, t = threadIdx.x >> 2;
   uint32_t v[8], c[8], x[8];
