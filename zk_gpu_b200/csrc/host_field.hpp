@@ -7,6 +7,9 @@
 #include <cstring>
 
 namespace zk {
+
+constexpr uint32_t MSM_MAX_WINDOWS = 64;  // windows of an MSM: at least 4 bits each
+
 namespace host {
 
 struct Fr {

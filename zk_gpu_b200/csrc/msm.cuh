@@ -21,6 +21,7 @@
 #include <cstdint>
 
 #include "field.cuh"
+#include "host_field.hpp"
 
 namespace zk {
 
@@ -48,7 +49,6 @@ struct MsmWindowsOut {
   uint32_t windows = 0;    // set by msm_run (0 for n = 0)
   uint32_t c = 0;
 };
-constexpr uint32_t MSM_MAX_WINDOWS = 64;  // c >= 4
 cudaError_t msm_run(const fe* d_scalars, const fe* d_bases_xy, uint64_t n, uint64_t* d_out, cudaStream_t s,
                     int c_override = 0, uint64_t* launches = nullptr, MsmWindowsOut* wout = nullptr);
 // The last step on the stream (msm_combine.cu): Horner over `windows` window

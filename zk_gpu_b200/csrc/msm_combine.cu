@@ -18,34 +18,23 @@
 // Slots are pooled per device, at most kMaxSlots; one is used again when its
 // kernel has finished and the library thread is done with it.
 #include <atomic>
-#include <chrono>
-#include <condition_variable>
 #include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <mutex>
-#include <thread>
+#include <new>
 #include <vector>
 
 #include "curve.cuh"
 #include "fq_inv.cuh"
-#include "host_field.hpp"
 #include "msm.cuh"
+#include "msm_answer.hpp"
 #include "msm_field.cuh"
 #include "runtime.cuh"
 
 namespace zk {
 
 namespace {
-
-// pinned, read and written by both sides
-struct Mail {
-  uint32_t ready;  // the kernel's: sequence number of the sums in `win`
-  uint32_t done;   // the host's: sequence number of the answer in `out`
-  uint32_t pad[2];
-  uint64_t win[MSM_MAX_WINDOWS * 16];
-  uint64_t out[12];
-};
 
 __device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t* p) {
   uint32_t v;
@@ -127,95 +116,18 @@ __global__ void __launch_bounds__(128) msm_combine_kernel(const fe* winsum, uint
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-struct Slot {
-  Mail* mail = nullptr;
+struct Slot : Watch {
   cudaEvent_t used = nullptr;  // its last kernel has finished
-  uint32_t seq = 0, windows = 0, c = 0;
-  bool taken = false;                  // between acquire and the event record
-  std::atomic<bool> watched{false};    // the library thread has not answered yet
+  bool taken = false;          // between acquire and the event record
 };
 constexpr size_t kMaxSlots = 64;
-
-// The thread that answers.  It polls while slots are watched (falling back to
-// short sleeps when nothing has come for a while) and sleeps otherwise.
-class Answerer {
- public:
-  static Answerer& get() {
-    static Answerer* a = new Answerer();  // stopped at exit, never destroyed
-    return *a;
-  }
-  void watch(Slot* s) {
-    std::lock_guard<std::mutex> lk(mu_);
-    if (stop_) {
-      s->watched.store(false);
-      return;
-    }
-    if (!thread_.joinable()) {
-      thread_ = std::thread([this] { run(); });
-      // registered after the CUDA runtime's own handlers, so it runs before
-      // they unmap the slots; kernels still waiting do the step themselves
-      std::atexit([] { get().stop(); });
-    }
-    queue_.push_back(s);
-    queued_.store(true);
-    cv_.notify_one();
-  }
-
- private:
-  void stop() {
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      stop_ = true;
-      queued_.store(true);
-      cv_.notify_one();
-    }
-    if (thread_.joinable()) thread_.join();
-  }
-  void run() {
-    using clk = std::chrono::steady_clock;
-    std::vector<Slot*> watched;
-    clk::time_point last = clk::now();
-    for (;;) {
-      if (queued_.load() || watched.empty()) {
-        std::unique_lock<std::mutex> lk(mu_);
-        cv_.wait(lk, [&] { return stop_ || !queue_.empty() || !watched.empty(); });
-        if (stop_) return;
-        watched.insert(watched.end(), queue_.begin(), queue_.end());
-        queue_.clear();
-        queued_.store(false);
-        last = clk::now();
-      }
-      for (size_t i = 0; i < watched.size();) {
-        Slot* s = watched[i];
-        if (__atomic_load_n(&s->mail->ready, __ATOMIC_ACQUIRE) != s->seq) {
-          i++;
-          continue;
-        }
-        host::fq::msm_combine_windows(s->mail->win, s->windows, s->c, s->mail->out);
-        __atomic_store_n(&s->mail->done, s->seq, __ATOMIC_RELEASE);
-        s->watched.store(false, std::memory_order_release);
-        watched[i] = watched.back();
-        watched.pop_back();
-        last = clk::now();
-      }
-      if (!watched.empty() && clk::now() - last > std::chrono::milliseconds(20))
-        std::this_thread::sleep_for(std::chrono::microseconds(20));
-    }
-  }
-  std::mutex mu_;
-  std::condition_variable cv_;
-  std::vector<Slot*> queue_;
-  std::atomic<bool> queued_{false};
-  bool stop_ = false;
-  std::thread thread_;
-};
 
 std::mutex g_slot_mu;
 std::vector<std::vector<std::unique_ptr<Slot>>> g_slots;  // per device
 
 // A free slot, made if there is none, or null when all kMaxSlots are in use
 // (the caller's kernel then does the step itself) or a new one cannot be had.
-Slot* acquire_slot(int dev) {
+Slot* acquire_slot(int dev) try {
   std::lock_guard<std::mutex> lk(g_slot_mu);
   if ((int)g_slots.size() <= dev) g_slots.resize(dev + 1);
   auto& pool = g_slots[dev];
@@ -231,6 +143,7 @@ Slot* acquire_slot(int dev) {
     return s.get();
   }
   if (pool.size() >= kMaxSlots) return nullptr;
+  pool.reserve(kMaxSlots);
   auto s = std::make_unique<Slot>();
   if (cudaMallocHost((void**)&s->mail, sizeof(Mail)) != cudaSuccess ||
       cudaEventCreateWithFlags(&s->used, cudaEventDisableTiming) != cudaSuccess) {
@@ -242,6 +155,8 @@ Slot* acquire_slot(int dev) {
   s->taken = true;
   pool.push_back(std::move(s));
   return pool.back().get();
+} catch (const std::bad_alloc&) {
+  return nullptr;
 }
 
 uint64_t host_wait_ns() {
@@ -271,14 +186,10 @@ cudaError_t msm_combine(const fe* d_winsum, uint32_t windows, uint32_t c, uint64
   slot->seq++;
   slot->windows = windows;
   slot->c = c;
-  slot->watched.store(true);
   msm_combine_kernel<<<1, 128, 0, s>>>(d_winsum, windows, c, d_out, slot->mail, slot->seq, wait);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaEventRecord(slot->used, s);
-  if (e == cudaSuccess)
-    Answerer::get().watch(slot);
-  else
-    slot->watched.store(false);
+  if (e == cudaSuccess) Answerer::get().watch(slot);
   std::lock_guard<std::mutex> lk(g_slot_mu);
   slot->taken = false;
   return e;
