@@ -89,6 +89,13 @@ int main(int, char** argv) {
     u.raise(3);
     return u.answered(5000) && u.released(5000) ? 0 : 1;
   }
+  if (!std::strcmp(what, "kernel not launched")) {  // dropped, then used again
+    static Use u;
+    u.prepare(6);
+    if (!Answerer::get().watch(&u.w)) return 1;
+    Answerer::drop(&u.w);
+    return u.released(5000) && u.mail.done == 0 && once(u, 7) ? 0 : 1;
+  }
   if (!std::strcmp(what, "many at once")) {  // 64 slots over four threads, used again and again
     std::atomic<int> bad{0};
     std::vector<std::thread> ts;

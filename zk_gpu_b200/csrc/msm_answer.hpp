@@ -31,6 +31,7 @@ struct Watch {
   uint32_t seq = 0, windows = 0, c = 0;
   Watch* next = nullptr;
   std::atomic<bool> watched{false};  // the library thread has not answered yet
+  std::atomic<bool> dropped{false};  // its kernel will not come
 };
 
 // The thread that answers.  It polls while slots are watched (falling back to
@@ -42,7 +43,9 @@ class Answerer {
     return *a;
   }
   // Answer w (not watched now) once its kernel is ready.  False, and nothing
-  // started, if nobody will: at exit, or when the thread cannot be had.
+  // started, if nobody will: at exit, or when the thread cannot be had.  Asked
+  // before the kernel is launched: where launches wait for their kernels
+  // (CUDA_LAUNCH_BLOCKING, a serialising profiler) nobody would answer it else.
   bool watch(Watch* w) {
     std::lock_guard<std::mutex> lk(mu_);
     if (stop_) return false;
@@ -56,6 +59,7 @@ class Answerer {
       // they unmap the slots; kernels still waiting do the step themselves
       std::atexit([] { get().stop(); });
     }
+    w->dropped.store(false);
     w->watched.store(true);
     w->next = queue_;
     queue_ = w;
@@ -63,6 +67,9 @@ class Answerer {
     cv_.notify_one();
     return true;
   }
+  // w's kernel was not launched after all; it stays watched until the thread
+  // has let go of it.
+  static void drop(Watch* w) { w->dropped.store(true); }
 
  private:
   void stop() {
@@ -93,12 +100,13 @@ class Answerer {
       }
       for (Watch** at = &watched; *at;) {
         Watch* w = *at;
-        if (__atomic_load_n(&w->mail->ready, __ATOMIC_ACQUIRE) != w->seq) {
+        if (__atomic_load_n(&w->mail->ready, __ATOMIC_ACQUIRE) == w->seq) {
+          host::fq::msm_combine_windows(w->mail->win, w->windows, w->c, w->mail->out);
+          __atomic_store_n(&w->mail->done, w->seq, __ATOMIC_RELEASE);
+        } else if (!w->dropped.load()) {
           at = &w->next;
           continue;
         }
-        host::fq::msm_combine_windows(w->mail->win, w->windows, w->c, w->mail->out);
-        __atomic_store_n(&w->mail->done, w->seq, __ATOMIC_RELEASE);
         *at = w->next;  // before the slot may be used again
         w->watched.store(false, std::memory_order_release);
         last = clk::now();

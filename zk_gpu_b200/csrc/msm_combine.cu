@@ -159,6 +159,11 @@ Slot* acquire_slot(int dev) try {
   return nullptr;
 }
 
+void release_slot(Slot* s) {
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  s->taken = false;
+}
+
 uint64_t host_wait_ns() {
   static const uint64_t ns = [] {
     const char* v = std::getenv("ZKGPU_MSM_HOST_WAIT_US");
@@ -179,19 +184,24 @@ cudaError_t msm_combine(const fe* d_winsum, uint32_t windows, uint32_t c, uint64
   if (e != cudaSuccess) return e;
   const uint64_t wait = host_wait_ns();
   Slot* slot = cap == cudaStreamCaptureStatusNone && wait ? acquire_slot(dev) : nullptr;
-  if (!slot) {
-    msm_combine_kernel<<<1, 128, 0, s>>>(d_winsum, windows, c, d_out, nullptr, 0, 0);
-    return cudaGetLastError();
+  if (slot) {
+    slot->seq++;
+    slot->windows = windows;
+    slot->c = c;
+    if (!Answerer::get().watch(slot)) {
+      release_slot(slot);
+      slot = nullptr;
+    }
   }
-  slot->seq++;
-  slot->windows = windows;
-  slot->c = c;
-  msm_combine_kernel<<<1, 128, 0, s>>>(d_winsum, windows, c, d_out, slot->mail, slot->seq, wait);
+  msm_combine_kernel<<<1, 128, 0, s>>>(d_winsum, windows, c, d_out, slot ? slot->mail : nullptr, slot ? slot->seq : 0,
+                                       wait);
   e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaEventRecord(slot->used, s);
-  if (e == cudaSuccess) Answerer::get().watch(slot);
-  std::lock_guard<std::mutex> lk(g_slot_mu);
-  slot->taken = false;
+  if (!slot) return e;
+  if (e == cudaSuccess)
+    e = cudaEventRecord(slot->used, s);
+  else
+    Answerer::drop(slot);
+  release_slot(slot);
   return e;
 }
 
