@@ -66,3 +66,62 @@ save(out)
 """, s, pts, CUDA_LAUNCH_BLOCKING="1", ZKGPU_MSM_HOST_WAIT_US="300000")
     want = oracle.multiexp(s, pts)
     assert all(np.array_equal(row[:8], want) for row in got)
+
+
+def test_captured_call_replays_on_new_scalars(oracle, tmp_path):
+    """under stream capture the kernel does the last step: a replay sums whatever the buffers hold then"""
+    n = 700
+    s, pts = oracle.rand_fr(2 * n, 931), oracle.rand_bases(n, 932)
+    got = run_child(tmp_path, """
+st = torch.cuda.Stream()
+cur = ds[:len(db)].clone()
+out = torch.zeros(12, dtype=torch.int64, device="cuda")
+rows = torch.zeros((3, 12), dtype=torch.int64, device="cuda")
+zk.msm_dev(cur, db, out, stream=st)
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph, stream=st):
+    zk.msm_dev(cur, db, out, stream=st)
+for k in range(3):
+    cur.copy_(ds[len(db):] if k == 1 else ds[:len(db)])
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    rows[k] = out
+    out.zero_()
+    torch.cuda.synchronize()
+save(rows)
+""", s, pts)
+    want = [oracle.multiexp(np.ascontiguousarray(v), pts) for v in (s[:n], s[n:])]
+    assert np.array_equal(got[:, :8], np.stack([want[0], want[1], want[0]]))
+
+
+@pytest.mark.parametrize("wait_us", ["1", "20", "3000"])
+def test_late_answers_and_full_slots(oracle, tmp_path, wait_us):
+    """Four threads with a stream each and more calls in flight than there are
+    slots.  With a wait of 1 us the kernels give up before the answer and it
+    comes late, into slots that are used again; with 20 us it is a race."""
+    n, calls = 64, 400
+    s, pts = oracle.rand_fr(n + calls, 941), oracle.rand_bases(n, 942)
+    got = run_child(tmp_path, """
+n = len(db)
+calls = len(ds) - n
+out = torch.zeros((calls, 12), dtype=torch.int64, device="cuda")
+streams = [torch.cuda.Stream() for _ in range(4)]
+errors = []
+def work(t):
+    try:
+        for i in range(t, calls, 4):
+            zk.msm_dev(ds[i:i + n], db, out[i], stream=streams[t])
+    except Exception as e:
+        errors.append(e)
+torch.cuda.synchronize()
+threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+for t in threads: t.start()
+for t in threads: t.join()
+assert not errors, errors
+torch.cuda.synchronize()
+save(out)
+""", s, pts, ZKGPU_MSM_HOST_WAIT_US=wait_us)
+    for i in range(calls):
+        assert np.array_equal(got[i, :8], oracle.multiexp(np.ascontiguousarray(s[i:i + n]), pts)), i

@@ -125,8 +125,9 @@ constexpr size_t kMaxSlots = 64;
 std::mutex g_slot_mu;
 std::vector<std::vector<std::unique_ptr<Slot>>> g_slots;  // per device
 
-// A free slot, made if there is none, or null when all kMaxSlots are in use
-// (the caller's kernel then does the step itself) or a new one cannot be had.
+// A free slot, made if there is none, or null when all kMaxSlots are in use, a
+// new one cannot be had or an event cannot be asked (the caller's kernel then
+// does the step itself); no error is left behind.
 Slot* acquire_slot(int dev) try {
   std::lock_guard<std::mutex> lk(g_slot_mu);
   if ((int)g_slots.size() <= dev) g_slots.resize(dev + 1);
@@ -134,10 +135,8 @@ Slot* acquire_slot(int dev) try {
   for (auto& s : pool) {
     if (s->taken || s->watched.load(std::memory_order_acquire)) continue;
     const cudaError_t q = cudaEventQuery(s->used);
-    if (q == cudaErrorNotReady) {
-      cudaGetLastError();
-      continue;
-    }
+    if (q != cudaSuccess) cudaGetLastError();
+    if (q == cudaErrorNotReady) continue;
     if (q != cudaSuccess) return nullptr;
     s->taken = true;
     return s.get();
