@@ -196,10 +196,14 @@ cudaError_t msm_combine(const fe* d_winsum, uint32_t windows, uint32_t c, uint64
                                        wait);
   e = cudaGetLastError();
   if (!slot) return e;
-  if (e == cudaSuccess)
-    e = cudaEventRecord(slot->used, s);
-  else
+  if (e != cudaSuccess) {
     Answerer::drop(slot);
+  } else {
+    // without the event nobody can tell when the kernel is done with its slot:
+    // it stays taken
+    e = cudaEventRecord(slot->used, s);
+    if (e != cudaSuccess) return e;
+  }
   release_slot(slot);
   return e;
 }
