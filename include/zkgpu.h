@@ -308,8 +308,10 @@ int zkgpu_field_op(int device, int op, int fid, const uint64_t *a, const uint64_
 int zkgpu_selftest_wait_timeout(int device, const uint64_t omega12[4], uint32_t spin_us);
 /* Give back the device memory the library keeps cached on `device`: the
  * NTT / coset table caches (capped at ZKGPU_TABLE_CACHE_MB per device,
- * default 8192, least recently used first; a serving loop counts them against
- * its HBM budget) and the unused blocks of the library's own memory pool.
+ * default an eighth of its memory and at least 8192, least recently used first,
+ * and dropped when an allocation of the library does not fit beside them; a
+ * serving loop counts them against its HBM budget) and the unused blocks of the
+ * library's own memory pool.
  * Tables still read by live batches or in-flight work stay allocated until
  * that work lets go of them.  No counterpart in the reference, which
  * allocates and frees everything per call (cuda/fft.cu:282-328). */

@@ -78,9 +78,9 @@ struct PowTables {
 // thread-safe.  Returns null and sets *err on failure.  The reference keeps
 // the tables alive: work that reads them (an enqueued transform, a batch
 // graph, a serving wave) holds it until the work is done or destroyed.  The
-// cache is capped per device (ZKGPU_TABLE_CACHE_MB, default 8192) and evicts
-// its least recently used entries; an evicted table is freed when its last
-// holder lets go (cudaFree, which waits for the device).
+// cache is capped per device (ZKGPU_TABLE_CACHE_MB, default an eighth of its
+// memory) and evicts its least recently used entries; an evicted table is freed
+// when its last holder lets go (cudaFree, which waits for the device).
 using NttTablesRef = std::shared_ptr<const NttTables>;
 NttTablesRef ntt_tables_get(int device, const host::Fr& omega, int log_n, cudaStream_t s, cudaError_t* err);
 // Uncached tables for an explicit plan (the autotuner's trials); free with
@@ -103,10 +103,11 @@ using PowTablesRef = std::shared_ptr<const PowTables>;
 PowTablesRef pow_tables_get(int device, const host::Fr& c, int log_n, cudaStream_t s, cudaError_t* err,
                             const host::Fr* scale = nullptr);
 // Bytes the device's table caches hold, and dropping every cached entry
-// (entries still held by work stay alive until it lets go).
+// (entries still held by work stay alive until it lets go; false if there was
+// none).
 uint64_t table_cache_bytes(int device);
 uint64_t table_cache_builds(int device);  // tables built so far on `device` (cache misses)
-void table_cache_clear(int device);
+bool table_cache_clear(int device);
 
 // Parameters of one pass launch (kernel argument / batch descriptor).
 struct PassParams {

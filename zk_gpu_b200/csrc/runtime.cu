@@ -4,6 +4,7 @@
 #include <mutex>
 #include <vector>
 
+#include "ntt.cuh"
 #include "runtime.cuh"
 
 namespace zk {
@@ -43,19 +44,31 @@ static cudaError_t library_pool(int device, cudaMemPool_t* out) {
   return cudaSuccess;
 }
 
-cudaError_t dmalloc(void** ptr, size_t bytes, cudaStream_t s) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
+static cudaError_t pool_malloc(void** ptr, size_t bytes, int dev, cudaStream_t s) {
   cudaMemPool_t pool;
-  e = library_pool(dev, &pool);
+  cudaError_t e = library_pool(dev, &pool);
   if (e != cudaSuccess) return e;
   return cudaMallocFromPoolAsync(ptr, bytes, pool, s);
 }
 
+cudaError_t dmalloc(void** ptr, size_t bytes, cudaStream_t s) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  e = pool_malloc(ptr, bytes, dev, s);
+  if (e == cudaErrorMemoryAllocation && table_cache_clear(dev)) {
+    cudaGetLastError();
+    e = pool_malloc(ptr, bytes, dev, s);
+  }
+  return e;
+}
+
 cudaError_t reserve_pool(size_t bytes, cudaStream_t s) {
   void* p = nullptr;
-  cudaError_t e = dmalloc(&p, bytes, s);
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  e = pool_malloc(&p, bytes, dev, s);
   if (e != cudaSuccess) {
     cudaGetLastError();  // a failed reservation is not an error of the caller's next call
     return e;

@@ -27,7 +27,8 @@ int bind_device(int device, cudaStream_t* stream);
 // Stream-ordered device allocation from the library's own memory pool on the
 // current device (created on first use).  The pool keeps freed memory cached
 // for reuse by later calls; the process's default pool, which the caller's
-// own allocations may use, is left as the caller configured it.  Free with
+// own allocations may use, is left as the caller configured it.  If the memory
+// is not to be had, the table cache is dropped and asked again.  Free with
 // cudaFreeAsync.  zkgpu_release_cached returns the cached memory.
 cudaError_t dmalloc(void** ptr, size_t bytes, cudaStream_t s);
 // Take `bytes` of device memory into the library pool of the current device

@@ -6,11 +6,12 @@
 // (cuda/fft.cu:282-285).  Entries are reference-counted: the cache holds one
 // reference, and work that reads a table (an enqueued transform, a batch
 // graph, a serving wave) holds another until it is done.  The cache is capped
-// per device (ZKGPU_TABLE_CACHE_MB, default 8192 MiB) and evicts its least
-// recently used entries when a new one would exceed the cap; an evicted table
-// is freed (cudaFree, which waits for the device) when its last holder lets
-// go.  Tables are built outside the cache lock, so a first use on one thread
-// does not stall lookups on others.
+// per device (cap_bytes) and evicts its least recently used entries when a new
+// one would exceed the cap; an evicted table is freed (cudaFree, which waits
+// for the device) when its last holder lets go.  It gives way when the
+// library's own allocations do not fit beside it.  Tables are built outside the
+// cache lock, so a first use on one thread does not stall lookups on others.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -57,13 +58,26 @@ std::map<int, uint64_t> g_bytes;  // per device
 std::map<int, uint64_t> g_builds;  // tables built (misses), per device
 uint64_t g_tick = 0;
 
-uint64_t cap_bytes() {
-  static const uint64_t cap = [] {
-    const char* v = std::getenv("ZKGPU_TABLE_CACHE_MB");
-    const uint64_t mb = v && *v ? std::strtoull(v, nullptr, 10) : 8192ull;
-    return mb << 20;
-  }();
-  return cap;
+// With g_mu held: ZKGPU_TABLE_CACHE_MB, or an eighth of the device's memory
+// but at least 8 GiB.  A table takes 64 B per element of its domain (4.1 GiB
+// for 2^26, 8.1 GiB for 2^27), and a prover goes back and forth between two
+// domains: values of 2^25 extended to 2^27 and back take 18.3 GiB, and 22.4 GiB
+// are an eighth of a B200.  Under a cap of 8 GiB the same way at 2^24 and 2^26
+// (9.1 GiB) built all its tables again on each pair of calls, which then waited
+// for the device too.
+uint64_t cap_bytes(int dev) {
+  static std::map<int, uint64_t> caps;
+  const auto it = caps.find(dev);
+  if (it != caps.end()) return it->second;
+  uint64_t cap = 8192ull << 20;
+  const char* v = std::getenv("ZKGPU_TABLE_CACHE_MB");
+  if (v && *v) {
+    cap = std::strtoull(v, nullptr, 10) << 20;
+  } else {
+    cudaDeviceProp prop;
+    if (cudaGetDeviceProperties(&prop, dev) == cudaSuccess) cap = std::max<uint64_t>(cap, prop.totalGlobalMem / 8);
+  }
+  return caps[dev] = cap;
 }
 
 uint32_t plan_code(const NttPlan& p) {
@@ -78,7 +92,7 @@ uint32_t plan_code(const NttPlan& p) {
 template <class V>
 void evict_for(int dev, uint64_t extra, V& drop) {
   for (;;) {
-    if (g_bytes[dev] + extra <= cap_bytes()) return;
+    if (g_bytes[dev] + extra <= cap_bytes(dev)) return;
     uint64_t oldest = ~0ull;
     int which = -1;
     auto n_old = g_ntt.end();
@@ -141,6 +155,10 @@ NttTablesRef ntt_tables_get(int device, const host::Fr& omega, int log_n, cudaSt
   }
   NttTables* t = new NttTables();
   cudaError_t e = ntt_tables_build(t, plan, omega, s);  // synchronises s
+  if (e == cudaErrorMemoryAllocation && table_cache_clear(device)) {
+    cudaGetLastError();
+    e = ntt_tables_build(t, plan, omega, s);
+  }
   if (e != cudaSuccess) {
     delete t;
     *err = e;
@@ -227,7 +245,7 @@ uint64_t table_cache_bytes(int device) {
   return it == g_bytes.end() ? 0 : it->second;
 }
 
-void table_cache_clear(int device) {
+bool table_cache_clear(int device) {
   std::vector<std::shared_ptr<const void>> drop;  // released after the lock (cudaFree waits for the device)
   std::lock_guard<std::mutex> lk(g_mu);
   for (auto it = g_ntt.begin(); it != g_ntt.end();) {
@@ -247,6 +265,7 @@ void table_cache_clear(int device) {
     }
   }
   g_bytes[device] = 0;
+  return !drop.empty();
 }
 
 }  // namespace zk
