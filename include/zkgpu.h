@@ -164,7 +164,10 @@ int zkgpu_divide_by_vanishing_dev(int device, uint64_t *d_ext, uint32_t log_n, u
  * asynchronous on `stream`.  Its last, serial step runs on a thread of the
  * library, to which the stream's last kernel hands the window sums; if that
  * thread does not answer within ZKGPU_MSM_HOST_WAIT_US (environment, default
- * 3000; 0: never asked), and under stream capture, the kernel does the step. */
+ * 3000; 0: never asked), and under stream capture, the kernel does the step.
+ * The thread polls while such calls are in flight and keeps a core busy until
+ * 20 ms after the last event (it yields to other threads); with 0 there is no
+ * thread, and a call takes about 4 ms longer on its stream. */
 int zkgpu_msm_dev(int device, const uint64_t *d_scalars, const uint64_t *d_bases_xy, uint64_t n, uint64_t *d_out_xyz,
                   void *stream);
 /* d_out_xy[i] = k_i * base (affine, Fq Montgomery, (0, 0) for the identity),

@@ -3,9 +3,10 @@
 // the kernel's place.  Exits 0 if the case named by argv[1] holds.
 #include <dlfcn.h>
 #include <pthread.h>
+#include <sched.h>
+#include <time.h>
 
 #include <cerrno>
-#include <cstdio>
 #include <cstring>
 #include <vector>
 
@@ -115,6 +116,31 @@ int main(int, char** argv) {
       });
     for (auto& t : ts) t.join();
     return bad ? 1 : 0;
+  }
+  if (!std::strcmp(what, "one core for both")) {  // a program at work leaves its core only to the answers
+    cpu_set_t set;
+    CPU_ZERO(&set);
+    CPU_SET(sched_getcpu(), &set);
+    if (sched_setaffinity(0, sizeof(set), &set)) return 1;
+    auto seconds = [](clockid_t c) {
+      timespec t;
+      clock_gettime(c, &t);
+      return (double)t.tv_sec + 1e-9 * (double)t.tv_nsec;
+    };
+    static Use u;
+    double mine = 0, all = 0;
+    for (uint32_t r = 0; r < 20; r++) {
+      u.prepare(r);
+      if (!Answerer::get().watch(&u.w)) return 1;
+      const double t0 = seconds(CLOCK_THREAD_CPUTIME_ID), p0 = seconds(CLOCK_PROCESS_CPUTIME_ID);
+      for (const double end = seconds(CLOCK_MONOTONIC) + 0.015; seconds(CLOCK_MONOTONIC) < end;) {
+      }
+      mine += seconds(CLOCK_THREAD_CPUTIME_ID) - t0;
+      all += seconds(CLOCK_PROCESS_CPUTIME_ID) - p0;
+      u.raise(r);
+      if (!u.answered(5000) || !u.released(5000)) return 1;
+    }
+    return mine > 0.75 * all ? 0 : 1;
   }
   if (!std::strcmp(what, "exit while watched")) {  // the thread is stopped, nobody is asked afterwards
     static Use u, v;

@@ -8,7 +8,8 @@ import subprocess
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-CASES = ["no thread to be had", "ready long after", "kernel not launched", "many at once", "exit while watched"]
+CASES = ["no thread to be had", "ready long after", "kernel not launched", "many at once", "one core for both",
+         "exit while watched"]
 
 
 @pytest.fixture(scope="module")

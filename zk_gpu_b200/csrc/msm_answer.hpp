@@ -34,8 +34,9 @@ struct Watch {
   std::atomic<bool> dropped{false};  // its kernel will not come
 };
 
-// The thread that answers.  It polls while slots are watched (falling back to
-// short sleeps when nothing has come for a while) and sleeps otherwise.
+// The thread that answers.  It polls while slots are watched, for 20 ms after
+// the last event without pause but yielding its core, then with short sleeps,
+// and sleeps otherwise.
 class Answerer {
  public:
   static Answerer& get() {
@@ -113,6 +114,8 @@ class Answerer {
       }
       if (watched && clk::now() - last > std::chrono::milliseconds(20))
         std::this_thread::sleep_for(std::chrono::microseconds(20));
+      else
+        std::this_thread::yield();  // the core to whoever else wants it
     }
   }
   std::mutex mu_;
