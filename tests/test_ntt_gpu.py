@@ -1,6 +1,8 @@
 """GPU parity: the sm_100a NTT through the C ABI against the CPU oracle
 (bit-exact), at every plan shape (1..4 passes), plus size-independent
 properties at the full benchmark sizes."""
+import random
+
 import numpy as np
 import pytest
 
@@ -255,3 +257,26 @@ def test_extended_to_coeff_output_on_an_odd_word(zk, oracle, log_ext, m):
     ref = oracle.extended_to_coeff(ext, log_ext, m, w_inv, d, g_inv)
     assert np.array_equal(got[1:-1].reshape(m, 4), ref)
     assert got[0] == got[-1] == (1 << 64) - 1
+
+
+@pytest.mark.parametrize("op,slack", [("mul_w2", 29), ("mul_w4", 29), ("mul_w8", 28)])
+def test_tabulated_products_over_their_whole_range(zk, op, slack):
+    """a b 2^-256 mod r for any a < 2^256, at the ends of the range too, below
+    r (1 + 2^-slack): the bound the unreduced sums of a butterfly are built on."""
+    p, top = B.R_MOD, 1 << 256
+    rng = random.Random(7)
+    xs = [0, 1, top - 1, top - 2, top >> 1, (top >> 1) - 1] + [k * p + d for k in range(1, 6) for d in (-1, 0, 1)]
+    xs += [top - (1 << k) for k in range(0, 256, 16)] + [(1 << k) - 1 for k in range(16, 256, 16)]
+    xs += [sum(0xFFFFFFFF << (64 * j) for j in range(4)), sum(0xFFFFFFFF << (64 * j + 32) for j in range(4))]
+    xs += [rng.randrange(top - (1 << 200), top) for _ in range(20)] + [rng.randrange(top) for _ in range(60)]
+    ys = [0, 1, p - 1, p - 2, (p - 1) // 2, top % p, -top % p, pow(top, -1, p)]
+    ys += [(1 << k) - 1 for k in range(32, 254, 32)] + [p - (1 << k) for k in range(32, 254, 32)]
+    ys += [rng.randrange(p) for _ in range(40)]
+    pairs = [(x, y) for x in xs for y in ys]
+    words = lambda v: [(v >> (64 * j)) & ((1 << 64) - 1) for j in range(4)]
+    a = np.array([words(x) for x, _ in pairs], np.uint64)
+    b = np.array([words(y) for _, y in pairs], np.uint64)
+    r_inv = pow(top, -1, p)
+    for (x, y), row in zip(pairs, zk.field_op(op, a, b)):
+        got = sum(int(w) << (64 * j) for j, w in enumerate(row))
+        assert got % p == x * y * r_inv % p and got < p + (p >> slack) + 1, (hex(x), hex(y))

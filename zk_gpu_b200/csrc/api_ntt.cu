@@ -357,8 +357,13 @@ extern "C" int zkgpu_extended_to_coeff_dev(int device, const uint64_t* d_ext, ui
 // diagnostics
 // ===========================================================================
 namespace {
+// what a Montgomery product with the multiplicand makes its table of (op 4..6)
+struct TableScales {
+  fe v[8];
+};
+
 template <class P>
-__global__ void field_op_kernel(int op, const fe* a, const fe* b, fe* out, uint64_t n) {
+__global__ void field_op_kernel(int op, const fe* a, const fe* b, fe* out, uint64_t n, const TableScales sc) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t x[8], y[8], r[8];
@@ -370,15 +375,28 @@ __global__ void field_op_kernel(int op, const fe* a, const fe* b, fe* out, uint6
     zk::add<P>(r, x, y);
   else if (op == 2)
     zk::sub<P>(r, x, y);
-  else
-    zk::fq_inv_divsteps(r, x);  // op 3, Fq only (checked on the host): the MSM rounds' inversion
+  else if (op == 3)
+    zk::fq_inv_divsteps(r, x);  // Fq only (checked on the host): the MSM rounds' inversion
+  else {  // Fr only: products by tabulated multiplicands
+    uint32_t w[8][8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) zk::mul<P>(w[k], y, sc.v[k].w);
+    const auto table = [&w](int k, uint32_t v[8]) { zk::cpy(v, w[k]); };
+    if (op == 4)
+      zk::mul_w2<P>(r, x, w[0], w[1]);
+    else if (op == 5)
+      zk::mul_w4<P>(r, x, table);
+    else
+      zk::mul_w8<P>(r, x, table);
+  }
   zk::st_fe(out + i, r);
 }
 }  // namespace
 
 extern "C" int zkgpu_field_op(int device, int op, int fid, const uint64_t* a, const uint64_t* b, uint64_t* out,
                               uint64_t n) {
-  if (!a || (op != 3 && !b) || !out || op < 0 || op > 3 || fid < 0 || fid > 1 || (op == 3 && fid != 1))
+  if (!a || (op != 3 && !b) || !out || op < 0 || op > 6 || fid < 0 || fid > 1 || (op == 3 && fid != 1) ||
+      (op > 3 && fid != 0))
     return ZKGPU_EINVAL;
   if (op == 3) b = a;  // unused operand
   if (n == 0) return ZKGPU_OK;
@@ -393,10 +411,16 @@ extern "C" int zkgpu_field_op(int device, int op, int fid, const uint64_t* a, co
   zk::h2d_copy(da, a, bytes, s);
   zk::h2d_copy(db, b, bytes, s);
   const unsigned grid = (unsigned)((n + 255) / 256);
+  TableScales sc{};
+  if (op > 3) {  // w^(k) = w 2^(256 k / forms + ...), see field.cuh
+    static const int forms[3] = {2, 4, 8}, first[3] = {160, 96, 64};
+    for (int k = 0; k < forms[op - 4]; k++)
+      std::memcpy(sc.v[k].w, hf::pow2(256 / forms[op - 4] * k + first[op - 4]).v, 32);
+  }
   if (fid == 0)
-    field_op_kernel<zk::FrP><<<grid, 256, 0, s>>>(op, da, db, dout, n);
+    field_op_kernel<zk::FrP><<<grid, 256, 0, s>>>(op, da, db, dout, n, sc);
   else
-    field_op_kernel<zk::FqP><<<grid, 256, 0, s>>>(op, da, db, dout, n);
+    field_op_kernel<zk::FqP><<<grid, 256, 0, s>>>(op, da, db, dout, n, sc);
   zk::count_launches(1);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = zk::d2h_copy(out, dout, bytes, s);
