@@ -48,12 +48,19 @@ NttPlan make_ntt_plan(int log_n) {
     p.bits[3] = last;
     return p;
   }
-  // 2^21 and 2^22 trade passes of 7 bits for 6 and 8 as well: 2^22 as 6+8+8
-  // takes 619 us, as 8+7+7 659; 2^21 as 6+7+8 328, as 7+7+7 331.
-  if (log_n == 21 || log_n == 22) {
+  // Three passes as 6, 7 or 8, 8 bits where that adds up: a pass of 7 takes a
+  // short round of one bit first and is the slowest per bit, and the last pass,
+  // which has no twists, is the cheapest place for 8.  Against balanced widths
+  // (B200, us): 2^21 327.6 / 329.2 (7+7+7), 2^22 619.4 / 660.0 (8+7+7).  Left
+  // balanced: 2^17 and 2^18, where that is fastest; 2^19, 94.6 at best against
+  // 96.6; 2^20, 185.0 as 6+6+8 against 197.1, whose plan of 7+7+6 the tuner's
+  // test knows as the built-in one, as it does 8+8+8 for 2^24 (2557, 2519 as
+  // 6+6+6+6); 2^23, 1262 as 6+6+6+5 against 1291.
+  const int middle = log_n - 6 - kNarrowMax;
+  if (np == 3 && middle >= 7 && middle <= kNarrowMax) {
     p.bits[0] = 6;
+    p.bits[1] = middle;
     p.bits[2] = kNarrowMax;
-    p.bits[1] = log_n - 6 - kNarrowMax;
     return p;
   }
   const int base = log_n / np, extra = log_n % np;
