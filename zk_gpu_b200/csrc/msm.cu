@@ -1,9 +1,6 @@
 // msm.cu — Pippenger MSM kernels and orchestration (see msm.cuh).
 #include <algorithm>
 
-#include <mutex>
-#include <vector>
-
 #include "curve.cuh"
 #include "msm.cuh"
 #include "msm_field.cuh"
@@ -843,21 +840,11 @@ uint64_t ba_tasks_bound(uint64_t jb, uint64_t fill_k) {
 }
 constexpr uint32_t kFillK = 148 * 64;  // task threads that fill a B200 (148 SMs) at 64 per SM
 
-// dynamic shared memory of the round kernels at 256 threads (two stages)
-constexpr int kPrefixSmem = 2 * BA_CP * 16 * 256;  // 32 KiB
-constexpr int kApplySmem = 2 * BA_CA * 16 * BA_APPLY;   // 80 KiB: above the 48 KiB default, opted in per device
-
-cudaError_t ba_kernel_attrs(int device) {
-  static std::mutex mu;
-  static uint64_t done = 0;  // one bit per device
-  std::lock_guard<std::mutex> lk(mu);
-  if (device < 64 && (done >> device) & 1) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(ba_apply_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kApplySmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(ba_apply_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kApplySmem);
-  if (e == cudaSuccess && device < 64) done |= 1ull << device;
-  return e;
-}
+// dynamic shared memory of the round kernels (two stages): 32 and 40 KiB, below
+// the 48 KiB a kernel gets without asking
+constexpr int kPrefixSmem = 2 * BA_CP * 16 * 256;
+constexpr int kApplySmem = 2 * BA_CA * 16 * BA_APPLY;
+static_assert(kPrefixSmem <= 48 << 10 && kApplySmem <= 48 << 10, "needs cudaFuncSetAttribute");
 
 int sm_count(int dev = -1) {
   int sms = 148;
@@ -1013,11 +1000,6 @@ cudaError_t msm_run_impl(const fe* d_scalars, const fe* d_bases, uint64_t n, uin
     winsum = wout->d_winsum;  // caller's buffer, left for the host's Horner step
   else
     alloc((void**)&winsum, W * 128ull);
-  if (e == cudaSuccess) {
-    int dev = 0;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = ba_kernel_attrs(dev);
-  }
   if (e == cudaSuccess) {
     const double nd = (double)n;
     const int sms = sm_count();

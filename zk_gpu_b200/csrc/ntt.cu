@@ -294,30 +294,6 @@ __global__ void scale_copy_kernel(fe* dst, const fe* src, uint64_t n, uint64_t d
 // host side
 // ---------------------------------------------------------------------------
 
-static cudaError_t pow_two_level(fe** lo, fe** hi, uint32_t* shift, const host::Fr& base, int log_count,
-                                 cudaStream_t s, bool pooled) {
-  const uint32_t sh = (uint32_t)((log_count + 1) / 2);
-  const uint64_t nlo = 1ull << sh, nhi = 1ull << (log_count > (int)sh ? log_count - sh : 0);
-  cudaError_t e;
-  *lo = *hi = nullptr;
-  if (pooled) {
-    e = zk::dmalloc((void**)lo, nlo * sizeof(fe), s);
-    if (e != cudaSuccess) return e;
-    e = zk::dmalloc((void**)hi, nhi * sizeof(fe), s);
-    if (e != cudaSuccess) return e;
-  } else {
-    e = cudaMalloc((void**)lo, nlo * sizeof(fe));
-    if (e != cudaSuccess) return e;
-    e = cudaMalloc((void**)hi, nhi * sizeof(fe));
-    if (e != cudaSuccess) return e;
-  }
-  const host::Fr bstep = host::pow_2k(base, sh);
-  pow_seq_kernel<<<(unsigned)((nlo + 255) / 256), 256, 0, s>>>(*lo, to_fe(base), nlo, 1);
-  pow_seq_kernel<<<(unsigned)((nhi + 255) / 256), 256, 0, s>>>(*hi, to_fe(bstep), nhi, 1);
-  *shift = sh;
-  return cudaGetLastError();
-}
-
 // Both power tables in one launch: entry e of lo is scale base^e, of hi
 // base^(e 2^shift), as products of the host's base^(2^k) by the bits of e
 // (without squarings, which would double the chain of dependent products).
@@ -414,14 +390,12 @@ static cudaError_t build_tables(NttTables* t, cudaStream_t s) {
       e = cudaMalloc((void**)&t->twist[k], 2 * total * sizeof(fe));
       if (e != cudaSuccess) return e;
       t->bytes += 2 * total * sizeof(fe);
-      fe *lo = nullptr, *hi = nullptr;
-      uint32_t sh = 0;
-      e = pow_two_level(&lo, &hi, &sh, wMJ, b + log_J, s, true);
+      PowTables pw;
+      e = pow_tables_make(&pw, wMJ, b + log_J, s);
       if (e != cudaSuccess) return e;
-      twist_table_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(t->twist[k], lo, hi, sh, (uint32_t)log_J, total,
-                                                                          table_scale());
-      cudaFreeAsync(lo, s);
-      cudaFreeAsync(hi, s);
+      twist_table_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(t->twist[k], pw.lo, pw.hi, pw.shift,
+                                                                          (uint32_t)log_J, total, table_scale());
+      pow_tables_free(&pw, s);
     }
     done_bits += b;
   }
