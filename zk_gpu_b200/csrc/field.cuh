@@ -43,7 +43,10 @@ struct FqP {
 #define ZK_A_OPS(a) "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7])
 
 // ---- Montgomery product ----------------------------------------------------
-// r = a b 2^-256 mod p on 32-bit words.  The running sum T is kept as two
+// r = a b 2^-256 mod p on 32-bit words: Montgomery's product with the reduction
+// interleaved row by row, the sums of even and odd columns in carry chains of
+// their own, a published arrangement of wide products on multiply-add pairs
+// that other GPU libraries use too.  The running sum T is kept as two
 // column chains: E holds word pairs at even positions, O at odd ones, so each
 // 32 x 32-bit product lands in one aligned pair and a row of four products is
 // one lo/hi multiply-add chain whose carries run from pair to pair.  A row
@@ -188,7 +191,7 @@ __device__ __forceinline__ void mul_out(uint32_t r[8], const uint32_t a[8], cons
 // in the form (Montgomery or not) a has; the last reduced word is there for
 // that bound, which lets a radix-8 butterfly add eight such values without
 // conditional subtractions in between.  Cycles per warp on one scheduler
-// (B200): 555 mul_lazy, about 460 mul_w2, about 390 mul_w4.
+// (B200): 555 mul_lazy, 440 mul_w2, 390 mul_w4.
 
 // A += x b over the four pairs of A[0..7], the carry into the two words above
 __device__ __forceinline__ void row_mad_cc(uint32_t A[10], uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3,

@@ -2,7 +2,7 @@
 // branch-free steps, for the MSM's batch-affine rounds.
 //
 // A Fermat inversion a^(q-2) is ~330 dependent Montgomery products (about
-// 0.18 ms of latency on the FP64 product); Stein's binary algorithm needs
+// 0.14 ms of latency); Stein's binary algorithm needs
 // ~500 steps of 256-bit subtractions, selects and shifts (~10^5
 // instructions).  The divstep recurrence of D. J. Bernstein and B.-Y. Yang,
 // "Fast constant-time gcd computation and modular inversion" (TCHES 2019),

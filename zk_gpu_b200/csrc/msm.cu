@@ -25,11 +25,14 @@ MsmPlan make_msm_plan(uint64_t n, int c_override, int device) {
   p.c = c;
   p.windows = (254 + c - 1) / c;
   p.buckets = 1u << (c - 1);
-  // buckets per reduction segment: a segment thread's latency is its
-  // running sum (2L additions); the window kernel then walks B / L segment
-  // sums per window, M = B / (256 L) per thread.  Few buckets per window:
-  // L = 4 for parallelism; many (2^12 and up): L = 16, which keeps the
-  // per-window pass (one block per window) short
+  // Buckets per reduction segment: a segment's quad of lanes adds 2 L times one
+  // after the other, and its sums then go through the group levels, about three
+  // additions per segment.  Few buckets leave the GPU idle, so short chains win;
+  // from 2^12 per window on it is full, and longer segments save work.  MSM of
+  // n points on B200 with L = 4 / 8 / 16 / 32 (us): 2^14 (2^9 buckets) 396 / 418
+  // / 460 / 526, 2^16 (2^11) 763 / 741 / 767 / 857, 2^18 (2^13) 1659 / 1652 /
+  // 1670 / 1653, 300007 (2^14) 1812 / 1755 / 1724 / 1724, 2^20 (2^15) 4013 /
+  // 3862 / 3789 / 3823.
   p.seg_len = std::min<uint32_t>(p.buckets >= 4096 ? 16u : 4u, p.buckets);
   return p;
 }
@@ -757,10 +760,9 @@ __global__ void __launch_bounds__(256) ba_heavy_kernel(const uint32_t* coff, con
 }
 
 // Bucket reduction.  A window's sum is W = sum_j (j + 1) B_j over its B
-// buckets.  Level 1, one thread per segment of L buckets: running sums from
-// the top give T_s = sum_i (i + 1) B_{sL+i} and S_s = sum_i B_{sL+i}, so
-// W = sum_s T_s + L sum_s s S_s.
-// A quad of lanes per segment (quad.cuh).
+// buckets.  Level 1, a quad of lanes (quad.cuh) per segment of L buckets:
+// running sums from the top give T_s = sum_i (i + 1) B_{sL+i} and
+// S_s = sum_i B_{sL+i}, so W = sum_s T_s + L sum_s s S_s.
 __global__ void __launch_bounds__(128) msm_segment_kernel(const fe* buckets, fe* seg_t, fe* seg_s, uint32_t B,
                                                           uint32_t L, uint32_t total_segs) {
   const Quad z;

@@ -10,9 +10,11 @@
 //   2. sort     : counting sort of the entries by bucket (histogram, scan,
 //                 scatter), so each bucket's points are contiguous.
 //   3. buckets  : pairwise affine additions in rounds, the inverses of each
-//                 round from Montgomery's trick (batch-affine accumulation).
-//   4. reduce   : per window, sum_b b * B_b by segmented running sums
-//                 (segment results T_s + lo_s * S_s), then a block tree sum.
+//                 round from Montgomery's trick (batch-affine accumulation);
+//                 with few entries direct XYZZ folds.
+//   4. reduce   : per window, sum_b b * B_b: running sums over segments of
+//                 buckets, then levels of suffix scans over up to 16 segments,
+//                 point additions by quads of lanes (quad.cuh).
 //   5. combine  : Horner over windows, sum_w 2^(c w) W_w, on the host (the
 //                 ~250 dependent doublings are serial), normalised Jacobian.
 #pragma once

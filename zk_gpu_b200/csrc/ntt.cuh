@@ -4,7 +4,7 @@
 // Algorithm: a natural-order-in / natural-order-out DFT
 //     A[k] = sum_i a[i] * w^(i k)           (w of order exactly n = 2^log_n)
 // computed as a mixed-radix four-step over p passes with bit widths
-// b_1 .. b_p (sum = log_n, each <= 12).  Pass t views the data as
+// b_1 .. b_p (sum = log_n, each <= 11).  Pass t views the data as
 // [O_t][m_t][J_t] (m_t = 2^b_t, O_t = 2^(b_1+..+b_(t-1)), J_t = 2^(b_(t+1)+..))
 // and runs one m_t-point DIF DFT per (o, j) column, then multiplies output
 // k of column j by the twist w_(m_t J_t)^(k j) and writes it back in place.
@@ -46,15 +46,17 @@ struct DftConsts {
   uint32_t w[3][64];
 };
 // As the parameter of a pass of B bits.  Where they start decides how wide
-// the compiler's constant loads are, and with that the pass's registers: on a
-// 16-byte boundary passes of 6 bits are fastest (2^24 as 6+6+6+6: 2520 us,
-// 2590 eight bytes past it), eight bytes past it those of 7 (2^21 as 7+7+7: 331
-// against 337) and of 8 (2^24 as 8+8+8: 2556 against 2580).
+// the compiler's constant loads are (nvcc 12.9; only speed depends on it), and
+// with that the pass's registers: on a 16-byte boundary passes of 6 bits are
+// fastest (2^24 as 6+6+6+6: 2520 us, 2590 eight bytes past it), eight bytes past
+// it those of 7 (2^21 as 7+7+7: 331 against 337) and of 8 (2^24 as 8+8+8: 2556
+// against 2580).
 template <int B>
 struct alignas(16) DftParam {
   uint32_t lead[B >= 7 ? 2 : 4];
   DftConsts c;
 };
+static_assert(offsetof(DftParam<6>, c) % 16 == 0 && offsetof(DftParam<7>, c) % 16 == 8, "see above");
 
 // Device tables for one (omega, log_n): per pass the roots its rounds use and,
 // for non-final passes, the twist table [k * J + j] (two entries of mul_w2).
