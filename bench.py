@@ -1020,7 +1020,7 @@ def msm_roofline(prof: dict, imad_ps: float, n: int, total_ms: float):
     return out
 
 
-HBM_GBS = 6543.1
+HBM_GBS = 6547.8
 # DRAM bytes (read + write) per launch over algorithmic bytes, from one ncu
 # capture of the same kernel on a smaller case (traffic grows with the
 # elements processed): ntt_pass_kernel<6> on a 2^24 transform, plan 6+6+6+6,
