@@ -82,7 +82,7 @@ struct VanishInv {
 };
 
 // The grid's stride is a multiple of the number of distinct values, so a
-// thread's elements all take the same one, tabulated once (mul_w2: 441 cycles
+// thread's elements all take the same one, tabulated once (mul_w2: 440 cycles
 // per warp and scheduler against 555).
 __global__ void __launch_bounds__(256) vanish_kernel(fe* d, const __grid_constant__ VanishInv tinv, uint32_t mask,
                                                      uint64_t n) {
